@@ -40,10 +40,6 @@ struct GemmArgs {
   // kernel of the same step.  Tile i covers rows [g_row0[i], g_row0[i] + g_rows[i]) of A and C and
   // multiplies them by expert g_expert[i]'s [N, K] block of the weight stack.
   const int* g_count; const int* g_row0; const int* g_rows; const int* g_expert;
-  // split-K for products with few rows (batched decode): `splits` CTAs share one output tile, each
-  // multiplies a K slice and leaves an fp32 partial tile in `ws`; the last one to arrive (ticket)
-  // adds the partials in slice order and writes the result, so the sum does not depend on timing.
-  int splits; float* ws; unsigned* tickets;
   int c_f32 = 0;                   // C is fp32 instead of bf16 (gate pre-activations, logits)
   float* C2 = nullptr; int64_t ldc2 = 0; int n_main = 0;   // columns from n_main on leave as fp32 in C2 (null: none)
   int act = 0; float act_a = 0.f, act_b = 0.f;   // epilogue activation (epi_act), 0: none
@@ -96,7 +92,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   __shared__ uint64_t full_bar[STAGES], empty_bar[STAGES], acc_full[2], acc_empty[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_s;
-  __shared__ bool split_last_s;
   volatile int* abort_flag = &abort_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -121,17 +116,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
   int m_tiles = a.m_tiles;
   if (a.g_count) { m_tiles = *a.g_count; if (m_tiles > a.m_tiles) m_tiles = a.m_tiles; }   // a.m_tiles: list capacity
-  const int splits = a.splits > 1 ? a.splits : 1;
-  const int kper = (a.k_blocks + splits - 1) / splits;            // k-blocks per slice
-  const int total = m_tiles * a.n_tiles * splits;                  // work item = (tile, K slice), slice fastest
+  const int total = m_tiles * a.n_tiles;
   if (warp == 0) {
     // ------------------------------- TMA producer -----------------------------------------
     if (lane == 0) {
       uint32_t it = 0;
       for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x) {
-        const TileCoord tc = tile_coord<BN>(a, tile / splits, m_tiles);
-        const int kb0 = (tile % splits) * kper, kb1 = min(a.k_blocks, kb0 + kper);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        const TileCoord tc = tile_coord<BN>(a, tile, m_tiles);
+        for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!wait_bar(&empty_bar[s], ph ^ 1, abort_flag)) { atomicExch(a.status, 1); abort_s = 1; break; }
@@ -152,8 +144,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         bool ok = true;
-        const int kb0 = (tile % splits) * kper, kb1 = min(a.k_blocks, kb0 + kper);
-        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+        for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!wait_bar(&full_bar[s], ph, abort_flag)) { atomicExch(a.status, 3); abort_s = 1; ok = false; break; }
@@ -163,8 +154,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
           for (int k = 0; k < BK / UK; ++k) {
             // advance 32 bytes along K inside the 128-byte swizzle atom: +2 in 16-byte units
-            if (I8) umma_i8(d_tmem, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
-            else umma_f16(d_tmem, ad + 2 * k, bd + 2 * k, IDESC, ((kb - kb0) | k) != 0);
+            if (I8) umma_i8(d_tmem, ad + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
+            else umma_f16(d_tmem, ad + 2 * k, bd + 2 * k, IDESC, (kb | k) != 0);
           }
           umma_commit(&empty_bar[s]);
         }
@@ -177,8 +168,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int q = warp & 3;  // TMEM lane quadrant this warp may read
     uint32_t tcount = 0;
     for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x, ++tcount) {
-      const int otile = tile / splits, ksl = tile % splits;
-      const TileCoord tc = tile_coord<BN>(a, otile, m_tiles);
+      const TileCoord tc = tile_coord<BN>(a, tile, m_tiles);
       const int m0 = tc.m0, n0 = tc.n0, row_end = tc.row_end;
       const uint32_t acc = tcount & 1, aph = (tcount >> 1) & 1;
       if (!wait_bar(&acc_full[acc], aph, abort_flag)) { if (lane == 0) { atomicExch(a.status, 4); abort_s = 1; } break; }
@@ -187,83 +177,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
       const float rs = (I8 && row < row_end) ? a.row_scale[row] : 1.f;
       // weight scales of this tile's columns: the grouped form keeps one [N] vector per expert, back to back
       const float* cscale = I8 ? a.col_scale + (tc.brow - n0) : nullptr;
-      if (splits > 1) {
-        // ---- K slice: park the fp32 partial tile, the last slice to arrive reduces all of them ----
-        float* mine = a.ws + ((size_t)tile * BM + q * 32 + lane) * BN;
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
-          uint32_t r[32];
-          tmem_ld32(tmem_base + acc * BN + ((uint32_t)(q * 32) << 16) + c0, r);
-          tmem_ld_wait();
-          if (row < row_end && n0 + c0 < a.N) {
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-              float4 f;
-              if (I8) f = make_float4((float)(int)r[4 * v], (float)(int)r[4 * v + 1], (float)(int)r[4 * v + 2], (float)(int)r[4 * v + 3]);
-              else f = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
-              __stcg(reinterpret_cast<float4*>(mine + c0) + v, f);
-            }
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[acc]);
-        __threadfence();
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (warp == 2 && lane == 0) {
-          const unsigned prev = atomicAdd(a.tickets + otile, 1u);
-          split_last_s = prev == (unsigned)splits - 1;
-          if (split_last_s) a.tickets[otile] = 0;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (split_last_s) {
-          __threadfence();
-          // all 128 epilogue threads walk the tile's valid rows as float4 columns (coalesced), adding
-          // the slices in slice order
-          const int et = (warp - 2) * 32 + lane;
-          const int nrow = min(BM, row_end - m0), ncol4 = min(BN, a.N - n0) >> 2;
-          const float* base = a.ws + (size_t)otile * splits * BM * BN;
-#pragma unroll 2
-          for (int e = et; e < nrow * ncol4; e += 128) {
-            const int r = e / ncol4, c = (e % ncol4) * 4;
-            float4 f = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int sidx = 0; sidx < splits; ++sidx) {
-              const float4 x = __ldcg(reinterpret_cast<const float4*>(base + ((size_t)sidx * BM + r) * BN + c));
-              f.x += x.x; f.y += x.y; f.z += x.z; f.w += x.w;
-            }
-            const int grow = m0 + r, gcol = n0 + c;
-            if (I8) {
-              const float rsr = a.row_scale[grow];
-              f.x *= rsr * a.col_scale[gcol]; f.y *= rsr * a.col_scale[gcol + 1];
-              f.z *= rsr * a.col_scale[gcol + 2]; f.w *= rsr * a.col_scale[gcol + 3];
-            }
-            if (a.act) {
-              f.x = epi_act(a.act, f.x, a.act_a, a.act_b); f.y = epi_act(a.act, f.y, a.act_a, a.act_b);
-              f.z = epi_act(a.act, f.z, a.act_a, a.act_b); f.w = epi_act(a.act, f.w, a.act_a, a.act_b);
-            }
-            if (a.residual) {
-              const uint2 rr = *reinterpret_cast<const uint2*>(a.residual + (int64_t)grow * a.ldr + gcol);
-              f.x += __uint_as_float(rr.x << 16); f.y += __uint_as_float(rr.x & 0xffff0000u);
-              f.z += __uint_as_float(rr.y << 16); f.w += __uint_as_float(rr.y & 0xffff0000u);
-            }
-            if (a.c_f32) {
-              *reinterpret_cast<float4*>(reinterpret_cast<float*>(a.C) + (int64_t)grow * a.ldc + gcol) = f;
-              continue;
-            }
-            if (a.C2 && gcol >= a.n_main) {
-              *reinterpret_cast<float4*>(a.C2 + (int64_t)grow * a.ldc2 + gcol - a.n_main) = f;
-              continue;
-            }
-            const __nv_bfloat162 lo = __floats2bfloat162_rn(f.x, f.y), hi = __floats2bfloat162_rn(f.z, f.w);
-            uint2 o;
-            o.x = *reinterpret_cast<const uint32_t*>(&lo);
-            o.y = *reinterpret_cast<const uint32_t*>(&hi);
-            *reinterpret_cast<uint2*>(reinterpret_cast<bf16*>(a.C) + (int64_t)grow * a.ldc + gcol) = o;
-          }
-        }
-        (void)ksl;
-        continue;
-      }
 #pragma unroll 1
       for (int c0 = 0; c0 < BN; c0 += 32) {
         uint32_t r[32];
@@ -336,7 +249,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, GemmArgs a, int 
   auto kern = gemm_tc_kernel<BN, STAGES, I8>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  const int total = a.m_tiles * a.n_tiles * (a.splits > 1 ? a.splits : 1);
+  const int total = a.m_tiles * a.n_tiles;
   const int grid = total < sms ? total : sms;
   return (int)cb_launch(kern, dim3((unsigned)grid), dim3(kThreadsGemm), smem, st, tmA, tmB, a);
 }
@@ -375,37 +288,13 @@ int pick_bn(int M, int N, int sms, bool allow64) {
 
 }  // namespace
 
-namespace {
-// Tile width and slice count for a product of at most 128 rows.  Every (tile, slice) gets its own CTA
-// in a single wave; the estimate is the bytes one CTA moves into shared memory (its slice of W and of
-// the valid rows of A) plus what the last slice re-reads to add the partial tiles.
-// K is counted in bytes of a row (a k-block is 128 bytes); n_cand = 2 leaves out the 64-wide tile.
-void plan_split(int64_t M, int64_t N, int64_t Kbytes, int* bn_out, int* s_out, int n_cand = 3) {
-  const int sms = sm_count();
-  const int64_t kb = (Kbytes + 127) / 128, K = Kbytes / 2;
-  const int cand[3] = {256, 128, 64};
-  double best = 1e300;
-  *bn_out = 256; *s_out = 1;
-  for (int i = 0; i < n_cand; ++i) {
-    const int bn = cand[i];
-    const int64_t tiles = (N + bn - 1) / bn;
-    int64_t s = sms / tiles;
-    if (s > kb / 4) s = kb / 4;          // at least four k-blocks per slice
-    if (s > 32) s = 32;
-    if (s < 1) s = 1;
-    for (;;) {                           // no slice may be empty: s = ceil(kb / ceil(kb / s))
-      const int64_t kper = (kb + s - 1) / s, s2 = (kb + kper - 1) / kper;
-      if (s2 == s) break;
-      s = s2;
-    }
-    const int64_t waves = (tiles * s + sms - 1) / sms;
-    const double stream = (double)waves * (bn + M) * ((double)K / s) * 2.0 / 130e3;        // us at ~130 GB/s per SM
-    const double reduce = s > 1 ? (double)s * M * bn * 4.0 / 100e3 + 2.0 : 0.0;
-    const double cost = stream + reduce;
-    if (cost < best) { best = cost; *bn_out = bn; *s_out = (int)s; }
-  }
-}
-}  // namespace
+// Products of at most 128 rows (gemm_rows.cu).
+int cb_gemm_rows_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N, int64_t K,
+                       float act_a, float act_b, void* status, void* stream);
+CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
+                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, void* status, void* stream);
+int cb_gemm_rows_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2, int64_t n_main,
+                       int64_t M, int64_t N, int64_t K, void* status, void* stream);
 
 // CTA-pair kernel (gemm_tc2.cu): tile width it would use for [M, N], or 0 for "not this product".
 int cb_gemm_pair_plan(int64_t M, int64_t N);
@@ -443,7 +332,6 @@ CB_EXPORT int cb_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ld
   a.k_blocks = (int)((K + 63) / 64); a.status = (int*)status;
   a.pf = (const TpPfDev*)pf; a.pf_seq = (unsigned)pf_seq;
   a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = 1; a.ws = nullptr; a.tickets = nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, false>(tmA, tmB, a, sms, st);
   if (bn == 160) return launch_gemm<160, 5, false>(tmA, tmB, a, sms, st);
@@ -453,21 +341,15 @@ CB_EXPORT int cb_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ld
 }
 
 // C[M,N] = xIELU(A[M,K] x W[N,K]^T), bf16, with the coefficients (act_a, act_b) of its two branches: the activation is taken
-// in the epilogue (CTA pairs above 256 rows, split K up to 128 rows when scratch is given).
+// in the epilogue.
 CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N,
-                                 int64_t K, float act_a, float act_b, void* ws, int64_t ws_bytes, void* tickets, int64_t n_tickets,
-                                 void* status, void* stream) {
+                                 int64_t K, float act_a, float act_b, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 8 || !status) return CB_ERR_SHAPE;
+  if (M <= BM) return cb_gemm_rows_xielu(A, lda, W, ldw, C, ldc, M, N, K, act_a, act_b, status, stream);
   const int tile = cb_gemm_pair_plan(M, N);
   if (tile) return cb_gemm_pair_xielu(A, lda, W, ldw, C, ldc, M, N, K, tile, act_a, act_b, status, stream);
   const int sms = sm_count();
-  int bn = pick_bn((int)M, (int)N, sms, true), splits = 1;
-  if (ws && tickets && M <= BM) {
-    int b2, s2;
-    plan_split(M, N, K * 2, &b2, &s2);
-    const int64_t tiles = (N + b2 - 1) / b2;
-    if (s2 > 1 && ws_bytes >= tiles * s2 * BM * b2 * (int64_t)sizeof(float) && n_tickets >= tiles) { bn = b2; splits = s2; }
-  }
+  const int bn = pick_bn((int)M, (int)N, sms, true);
   CUtensorMap tmA, tmB;
   int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, 64);
   if (rc) return rc;
@@ -479,7 +361,6 @@ CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int6
   a.k_blocks = (int)((K + 63) / 64); a.status = (int*)status;
   a.pf = nullptr; a.pf_seq = 0;
   a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = splits; a.ws = (float*)ws; a.tickets = (unsigned*)tickets;
   a.act = 1; a.act_a = act_a; a.act_b = act_b;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, false>(tmA, tmB, a, sms, st);
@@ -489,21 +370,15 @@ CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int6
 }
 
 // One product, two results: columns [0, n_main) of A[M,K] x W[N,K]^T as bf16 in C, the others (gate pre-activations) as
-// fp32 in C2.  n_main % 8 == 0; ws / tickets as above.
+// fp32 in C2.  n_main % 8 == 0.
 CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2,
-                                 int64_t n_main, int64_t M, int64_t N, int64_t K, void* ws, int64_t ws_bytes, void* tickets, int64_t n_tickets,
-                                 void* status, void* stream) {
+                                 int64_t n_main, int64_t M, int64_t N, int64_t K, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 8 || ldc2 % 4 || n_main % 8 || n_main < 0 || n_main > N || !C2 || !status) return CB_ERR_SHAPE;
+  if (M <= BM) return cb_gemm_rows_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, status, stream);
   const int tile = cb_gemm_pair_plan(M, N);
   if (tile) return cb_gemm_pair_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, tile, status, stream);
   const int sms = sm_count();
-  int bn = pick_bn((int)M, (int)N, sms, true), splits = 1;
-  if (ws && tickets && M <= BM) {
-    int b2, s2;
-    plan_split(M, N, K * 2, &b2, &s2);
-    const int64_t tiles = (N + b2 - 1) / b2;
-    if (s2 > 1 && ws_bytes >= tiles * s2 * BM * b2 * (int64_t)sizeof(float) && n_tickets >= tiles) { bn = b2; splits = s2; }
-  }
+  const int bn = pick_bn((int)M, (int)N, sms, true);
   CUtensorMap tmA, tmB;
   int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, 64);
   if (rc) return rc;
@@ -515,7 +390,6 @@ CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int6
   a.k_blocks = (int)((K + 63) / 64); a.status = (int*)status;
   a.pf = nullptr; a.pf_seq = 0;
   a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = splits; a.ws = (float*)ws; a.tickets = (unsigned*)tickets;
   a.C2 = (float*)C2; a.ldc2 = ldc2; a.n_main = (int)n_main;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, false>(tmA, tmB, a, sms, st);
@@ -525,20 +399,13 @@ CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int6
 }
 
 // C[M,N] (fp32) = A[M,K] (bf16) x W[N,K]^T (bf16): the accumulator leaves unrounded (gate pre-activations of the
-// recurrent mixers, logits of many rows).  K % 8 == 0, N % 8 == 0, ldc % 4 == 0.  ws / tickets: split-K scratch
-// for products of at most 128 rows (see cb_gemm_bf16_splitk); null = never split.
+// recurrent mixers, logits of many rows).  K % 8 == 0, N % 8 == 0, ldc % 4 == 0.
 CB_EXPORT int cb_gemm_bf16_f32out(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M,
-                                  int64_t N, int64_t K, void* ws, int64_t ws_bytes, void* tickets, int64_t n_tickets,
-                                  void* status, void* stream) {
+                                  int64_t N, int64_t K, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 4 || !status) return CB_ERR_SHAPE;
+  if (M <= BM) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, status, stream);
   const int sms = sm_count();
-  int bn = pick_bn((int)M, (int)N, sms, true), splits = 1;
-  if (ws && tickets && M <= BM) {
-    int b2, s2;
-    plan_split(M, N, K * 2, &b2, &s2);
-    const int64_t tiles = (N + b2 - 1) / b2;
-    if (s2 > 1 && ws_bytes >= tiles * s2 * BM * b2 * (int64_t)sizeof(float) && n_tickets >= tiles) { bn = b2; splits = s2; }
-  }
+  const int bn = pick_bn((int)M, (int)N, sms, true);
   CUtensorMap tmA, tmB;
   int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, 64);
   if (rc) return rc;
@@ -550,7 +417,6 @@ CB_EXPORT int cb_gemm_bf16_f32out(const void* A, int64_t lda, const void* W, int
   a.k_blocks = (int)((K + 63) / 64); a.status = (int*)status;
   a.pf = nullptr; a.pf_seq = 0;
   a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = splits; a.ws = (float*)ws; a.tickets = (unsigned*)tickets;
   a.c_f32 = 1;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, false>(tmA, tmB, a, sms, st);
@@ -587,7 +453,6 @@ CB_EXPORT int cb_gemm_i8(const void* A, int64_t lda, const void* W, int64_t ldw,
   a.k_blocks = (int)((K + 127) / 128); a.status = (int*)status;
   a.pf = (const TpPfDev*)pf; a.pf_seq = (unsigned)pf_seq;
   a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = 1; a.ws = nullptr; a.tickets = nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, true>(tmA, tmB, a, sms, st);
   if (bn == 160) return launch_gemm<160, 5, true>(tmA, tmB, a, sms, st);
@@ -620,7 +485,6 @@ CB_EXPORT int cb_gemm_bf16_grouped(const void* A, int64_t lda, const void* W, in
   a.k_blocks = (int)((K + 63) / 64); a.status = (int*)status;
   a.pf = nullptr; a.pf_seq = 0;
   a.g_count = (const int*)g_count; a.g_row0 = (const int*)g_row0; a.g_rows = (const int*)g_rows; a.g_expert = (const int*)g_expert;
-  a.splits = 1; a.ws = nullptr; a.tickets = nullptr;
   a.act = (int)act;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, false>(tmA, tmB, a, sms, st);
@@ -652,90 +516,8 @@ CB_EXPORT int cb_gemm_i8_grouped(const void* A, int64_t lda, const void* W, int6
   a.k_blocks = (int)((K + 127) / 128); a.status = (int*)status;
   a.pf = nullptr; a.pf_seq = 0;
   a.g_count = (const int*)g_count; a.g_row0 = (const int*)g_row0; a.g_rows = (const int*)g_rows; a.g_expert = (const int*)g_expert;
-  a.splits = 1; a.ws = nullptr; a.tickets = nullptr;
   cudaStream_t st = (cudaStream_t)stream;
   if (bn == 256) return launch_gemm<256, 4, true>(tmA, tmB, a, sms, st);
   if (bn == 160) return launch_gemm<160, 5, true>(tmA, tmB, a, sms, st);
-  return launch_gemm<128, 6, true>(tmA, tmB, a, sms, st);
-}
-
-// Skinny product for batched decode (M <= 128 rows: one m-tile): C = A x W^T (+ residual) with the K
-// dimension split over CTAs so that the whole machine streams the weights even when N gives only a
-// few 256-wide tiles (N = 2560: 10 tiles x 14 slices).  ws holds the fp32 partial tiles
-// (cb_gemm_splitk_ws_bytes), tickets one zero-initialised counter per output tile; both may be
-// shared by all calls of a stream.  Falls back to the plain kernel when splitting does not pay.
-// (slices, or 1 when the plain kernel is used) and the workspace a call needs
-CB_EXPORT int64_t cb_gemm_splitk_plan(int64_t M, int64_t N, int64_t K) {
-  if (M > BM) return 1;
-  int bn, s;
-  plan_split(M, N, K * 2, &bn, &s);
-  return s;
-}
-CB_EXPORT int64_t cb_gemm_splitk_ws_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M > BM) return 0;
-  int bn, s;
-  plan_split(M, N, K * 2, &bn, &s);
-  return s < 2 ? 0 : ((N + bn - 1) / bn) * s * BM * bn * (int64_t)sizeof(float);
-}
-CB_EXPORT int cb_gemm_bf16_splitk(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc,
-                                  const void* residual, int64_t ldr, int64_t M, int64_t N, int64_t K, void* ws,
-                                  int64_t ws_bytes, void* tickets, int64_t n_tickets, void* status, void* stream) {
-  if (M < 1 || M > BM || N < 1 || K < 1) return CB_ERR_SHAPE;
-  if (K % 8 || N % 8 || ldc % 8 || (residual && ldr % 8) || !status) return CB_ERR_SHAPE;
-  int bn, splits;
-  plan_split(M, N, K * 2, &bn, &splits);
-  if (splits < 2) return cb_gemm_bf16(A, lda, W, ldw, C, ldc, residual, ldr, M, N, K, bn, nullptr, 0, status, stream);
-  const int64_t tiles = (N + bn - 1) / bn;
-  if (!ws || !tickets || ws_bytes < cb_gemm_splitk_ws_bytes(M, N, K) || n_tickets < tiles) return CB_ERR_ARG;
-  const int sms = sm_count();
-  CUtensorMap tmA, tmB;
-  int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, 64);
-  if (rc) return rc;
-  rc = cb_make_tmap_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)bn, 64);
-  if (rc) return rc;
-  GemmArgs a;
-  a.C = C; a.ldc = ldc; a.residual = (const bf16*)residual; a.ldr = ldr; a.row_scale = nullptr; a.col_scale = nullptr;
-  a.M = (int)M; a.N = (int)N; a.K = (int)K; a.m_tiles = 1; a.n_tiles = 0;
-  a.k_blocks = (int)((K + 63) / 64); a.status = (int*)status;
-  a.pf = nullptr; a.pf_seq = 0;
-  a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = splits; a.ws = (float*)ws; a.tickets = (unsigned*)tickets;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (bn == 256) return launch_gemm<256, 4, false>(tmA, tmB, a, sms, st);
-  if (bn == 128) return launch_gemm<128, 6, false>(tmA, tmB, a, sms, st);
-  return launch_gemm<64, 8, false>(tmA, tmB, a, sms, st);
-}
-
-// int8 (W8A8) form of the split-K product: int32 partial sums are parked as fp32 (exact up to 2^24 per
-// slice, then rounded like any fp32 sum) and the row x column scales are applied by the reducing slice.
-CB_EXPORT int cb_gemm_i8_splitk(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc,
-                                const void* residual, int64_t ldr, const void* row_scale, const void* col_scale,
-                                int64_t M, int64_t N, int64_t K, void* ws, int64_t ws_bytes, void* tickets,
-                                int64_t n_tickets, void* status, void* stream) {
-  if (M < 1 || M > BM || N < 1 || K < 1) return CB_ERR_SHAPE;
-  if (K % 16 || N % 8 || ldc % 8 || lda % 16 || ldw % 16 || (residual && ldr % 8) || !status || !row_scale || !col_scale)
-    return CB_ERR_SHAPE;
-  int bn, splits;
-  plan_split(M, N, K, &bn, &splits, 2);
-  if (splits < 2)
-    return cb_gemm_i8(A, lda, W, ldw, C, ldc, residual, ldr, row_scale, col_scale, M, N, K, bn, nullptr, 0, status, stream);
-  const int64_t tiles = (N + bn - 1) / bn;
-  if (!ws || !tickets || ws_bytes < tiles * splits * BM * bn * (int64_t)sizeof(float) || n_tickets < tiles) return CB_ERR_ARG;
-  const int sms = sm_count();
-  CUtensorMap tmA, tmB;
-  int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, BM, 128);
-  if (rc) return rc;
-  rc = cb_make_tmap_2d(&tmB, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, (uint32_t)bn, 128);
-  if (rc) return rc;
-  GemmArgs a;
-  a.C = C; a.ldc = ldc; a.residual = (const bf16*)residual; a.ldr = ldr;
-  a.row_scale = (const float*)row_scale; a.col_scale = (const float*)col_scale;
-  a.M = (int)M; a.N = (int)N; a.K = (int)K; a.m_tiles = 1; a.n_tiles = 0;
-  a.k_blocks = (int)((K + 127) / 128); a.status = (int*)status;
-  a.pf = nullptr; a.pf_seq = 0;
-  a.g_count = a.g_row0 = a.g_rows = a.g_expert = nullptr;
-  a.splits = splits; a.ws = (float*)ws; a.tickets = (unsigned*)tickets;
-  cudaStream_t st = (cudaStream_t)stream;
-  if (bn == 256) return launch_gemm<256, 4, true>(tmA, tmB, a, sms, st);
   return launch_gemm<128, 6, true>(tmA, tmB, a, sms, st);
 }

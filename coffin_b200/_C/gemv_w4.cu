@@ -283,7 +283,9 @@ int launch_w4(W4Args a, cudaStream_t st, int n_slots) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  return (int)cb_launch(kern, dim3((unsigned)grid, (unsigned)n_slots), dim3(kT), smem, st, a);
+  // loads in flight live in L1: shared memory for two CTAs and no more, whatever split the kernel before this one left
+  const int64_t carve = std::min<int64_t>(100, (2 * (int64_t)(smem + 2048) * 100 + 228 * 1024 - 1) / (228 * 1024));
+  return (int)cb_launch_carve((int)carve, kern, dim3((unsigned)grid, (unsigned)n_slots), dim3(kT), smem, st, a);
 }
 
 template <bool NORM>
@@ -333,7 +335,8 @@ CB_EXPORT int cb_moe_gemv_w4(const void* Wq, const void* wscale, const void* x, 
 namespace {
 __global__ void __launch_bounds__(256) w4_dequant_kernel(const uint8_t* __restrict__ Wq, const float* __restrict__ scale,
                                                          bf16* __restrict__ out, int64_t N, int64_t K) {
-  griddep_launch();
+  // dependents are not launched early: the products that follow request the weights written here ahead of their own wait
+  cbtrace::stamp(0);
   griddep_wait();
   const int64_t half = K >> 1, G = K / kGroup;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < N * (half >> 2); i += (int64_t)gridDim.x * 256) {

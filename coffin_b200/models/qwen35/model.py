@@ -375,13 +375,14 @@ class Qwen35Model:
             A = K.swiglu(A)
         return K.gemm(A, W, out=out, residual=residual, push=push)
 
-    def _gemm_gu(self, A, W, gu: torch.Tensor, aq=None):
-        """Gate|up projection of a prefill chunk into ``gu [T, 2I]``.  bf16 weights and more rows than one
-        CTA-pair tile: the SwiGLU product comes out of the GEMM epilogue and the ``[T, I]`` view holding it
-        is returned; otherwise ``gu`` is filled with both halves and None is returned."""
+    def _gemm_gu(self, A, W, gu: torch.Tensor, aq=None, decode: bool = False):
+        """Gate|up projection of a prefill chunk or a wide decode bucket (``decode``) into ``gu [T, 2I]``.  The SwiGLU product
+        comes out of the GEMM epilogue (decode buckets; chunks of more rows than one CTA-pair tile) and the ``[T, I]`` view
+        holding it is returned; otherwise ``gu`` is filled with both halves, rounded, and None is returned."""
         if isinstance(W, QW4):
             W = W.expanded()
-        if K.PAIR_GEMM and gu.shape[0] >= K.PAIR_MIN_ROWS and W.shape[0] >= 256:
+        T = gu.shape[0]
+        if (decode and T <= K.ROWS and W.shape[0] % 16 == 0) or (K.PAIR_GEMM and T >= K.PAIR_MIN_ROWS and W.shape[0] >= 256):
             if isinstance(W, QW):
                 q, sc = aq if aq is not None else K.quant_rows(A)
                 return K.gemm_i8_swiglu(q, sc, W.wq, W.scale, out=gu[:, :W.shape[0] // 2])
@@ -397,7 +398,7 @@ class Qwen35Model:
         not fill) writes the partial rows and a small kernel copies them there.  A reduce/gather kernel
         on every rank then pulls the rows it owns from all ranks, adds them and stores the sums to every rank.  Without the region the partial result is all-reduced by NCCL."""
         if self.tp is not None and self.tp.pf_rows:
-            if A.shape[0] <= 128 and K.SPLITK_GEMM:
+            if A.shape[0] <= K.ROWS:
                 self._gemm(A, W, out=scratch, swiglu_in=swiglu_in)
                 self.tp.scatter(scratch)
             else:
@@ -678,7 +679,6 @@ class Qwen35Model:
                 b["normed"] = torch.zeros(M, H, dtype=bf, device=dev)
                 if not c.is_moe:
                     b["gu"] = torch.zeros(M, 2 * c.intermediate_size, dtype=bf, device=dev)
-                b["logits_bf"] = torch.zeros(M, self.vocab_local, dtype=bf, device=dev)
                 if self.tp is not None:
                     b["part"] = torch.zeros(M, H, dtype=bf, device=dev)
             self._rows[key] = b
@@ -866,15 +866,17 @@ class Qwen35Model:
                 res.add_(lw.moe.apply(normed, self))
                 K._count()
             else:
-                self._gemm(normed, lw.w_gu, out=b["gu"], aq=gq)
+                gu = self._gemm_gu(normed, lw.w_gu, b["gu"], aq=gq, decode=True)
+                halves = gu is None
+                gu = b["gu"] if halves else gu
                 if tpw and self.tp.pf_rows:
-                    self._gemm(b["gu"], lw.w_down, out=b["part"], swiglu_in=True)
+                    self._gemm(gu, lw.w_down, out=b["part"], swiglu_in=halves)
                     self.tp.oneshot(b["part"], residual=res, res_out=res)
                 elif tpw:
-                    res.add_(self._row_parallel(b["gu"], lw.w_down, b["part"], swiglu_in=True))
+                    res.add_(self._row_parallel(gu, lw.w_down, b["part"], swiglu_in=halves))
                     K._count()
                 else:
-                    self._gemm(b["gu"], lw.w_down, out=res, residual=res, swiglu_in=True)
+                    self._gemm(gu, lw.w_down, out=res, residual=res, swiglu_in=halves)
         if not self.pp_last:
             b["hidden"].copy_(res)
             K._count()
@@ -884,11 +886,9 @@ class Qwen35Model:
             K.rmsnorm(res, self.final_gain, self.eps, quant=hq)
         else:
             K.rmsnorm(res, self.final_gain, self.eps, out=normed)
-        self._gemm(normed, self.lm_head, out=b["logits_bf"], aq=hq)
+        self._gemm(normed, self.lm_head, out=b["logits_local"], aq=hq)          # fp32, straight from the accumulators
         if tpw:
             # vocabulary-parallel head: every rank needs the arg-max over the whole vocabulary
-            b["logits_local"].copy_(b["logits_bf"])
-            K._count()
             if not self.full_logits and self.tp.n_sites > 2 * len(self.layers):
                 # greedy rows: each rank's best {value, index} per row through the inbox, no logits gather
                 self.tp.epoch_bump()
@@ -900,8 +900,6 @@ class Qwen35Model:
                 b["logits"].copy_(self._gather_logits(b["logits_local"], M))
                 K.argmax(b["logits"], b["next"])
         else:
-            b["logits"].copy_(b["logits_bf"])
-            K._count()
             K.argmax(b["logits"], b["next"])
         b["final_res"] = res
         if self._advance:
@@ -1052,7 +1050,6 @@ class Qwen35Model:
                 "inter": torch.zeros(N, max(1, c.intermediate_size), dtype=bf, device=dev),
                 "gu": torch.zeros(N, max(1, 2 * c.intermediate_size), dtype=bf, device=dev) if N > WIDE else None,
                 "logits": torch.zeros(N, c.vocab_size, dtype=torch.float32, device=dev),
-                "logits_bf": torch.zeros(N, self.vocab_local, dtype=bf, device=dev) if N > WIDE else None,
                 "slot": torch.full((R,), -1, dtype=torch.int32, device=dev),
                 "pos": torch.zeros(R, dtype=torch.int32, device=dev),
                 "kv_slots": torch.full((N,), -1, dtype=torch.int32, device=dev),
@@ -1148,8 +1145,8 @@ class Qwen35Model:
                     cur.add_(lw.moe.apply(b["normed"], self))
                     K._count()
                 else:
-                    self._gemm(b["normed"], lw.w_gu, out=b["gu"])
-                    self._gemm(b["gu"], lw.w_down, out=cur, residual=cur, swiglu_in=True)
+                    gu = self._gemm_gu(b["normed"], lw.w_gu, b["gu"], decode=True)
+                    self._gemm(b["gu"] if gu is None else gu, lw.w_down, out=cur, residual=cur, swiglu_in=gu is None)
                 continue
             self._gemv(lw.w_out, act, b["h"])
             if lw.moe is not None:
@@ -1162,9 +1159,7 @@ class Qwen35Model:
             carry = b["h2"]
         if wide:
             K.rmsnorm(cur, self.final_gain, self.eps, out=b["normed"])
-            self._gemm(b["normed"], self.lm_head, out=b["logits_bf"])
-            b["logits"].copy_(b["logits_bf"])
-            K._count()
+            self._gemm(b["normed"], self.lm_head, out=b["logits"])
             b["final_res"] = cur
         else:
             self._gemv(self.lm_head, None, b["logits"], norm=(cur, carry, self.final_gain, nxt, self.eps))

@@ -212,13 +212,7 @@ class MoEWeights:
         # (eight 8-row GEMV launches per layer were a fifth of a 64-row step)
         wide = T > 8
         if wide:
-            if "logits_bf" not in b:
-                b["logits_bf"] = torch.zeros(T, self.router.shape[0], dtype=torch.bfloat16, device=normed.device)
-                if self.sh_gu is not None:
-                    b["sh_gu_out"] = torch.zeros(T, self.sh_gu.shape[0], dtype=torch.bfloat16, device=normed.device)
-            K.gemm(normed, self.router, out=b["logits_bf"])
-            b["logits"][:T].copy_(b["logits_bf"])
-            K._count()
+            K.gemm(normed, self.router, out=b["logits"][:T])
         else:
             K.gemv(self.router, normed, b["logits"][:T])
         K.call("moe_router", b["logits"], b["logits"].stride(0), T, E, k, int(c.norm_topk_prob), b["idx"], b["w"],
@@ -238,8 +232,7 @@ class MoEWeights:
         shared = gate = None
         if self.sh_gu is not None:
             if wide:
-                K.gemm(normed, self.sh_gu, out=b["sh_gu_out"])
-                K.swiglu(b["sh_gu_out"], out=b["sh_inter"][:T])
+                K.gemm_swiglu(normed, self.sh_gu, out=b["sh_inter"][:T])
                 K.gemm(b["sh_inter"][:T], self.sh_down, out=b["sh_out"][:T])
             else:
                 K.gemv(self.sh_gu, normed, b["sh_inter"][:T], swiglu=True)

@@ -241,6 +241,12 @@ def _norm_rows(res_in: torch.Tensor, add, gain: torch.Tensor, res_out, eps: floa
     return buf
 
 
+def _rows_gemv_ok(W, x, out, M: int, N: int, K: int) -> bool:
+    """Whether a decode projection of several rows takes the tcgen05 kernel."""
+    return (GEMV_IMPL == "mma" and M >= 2 and N % 8 == 0 and K % 8 == 0 and out.stride(0) % 8 == 0 and out.stride(1) == 1 and W.is_contiguous()
+            and (W.data_ptr() | x.data_ptr() | out.data_ptr()) % 16 == 0)
+
+
 def gemv(W: torch.Tensor, x: torch.Tensor | None, out: torch.Tensor | None, *, swiglu: bool = False,
          norm: tuple | None = None, tp=None, pull_site: int = -1, push_site: int = -1, rows: int | None = None,
          tail: tuple | None = None) -> torch.Tensor | None:
@@ -291,6 +297,8 @@ def gemv(W: torch.Tensor, x: torch.Tensor | None, out: torch.Tensor | None, *, s
         tpp = tp.cstruct_ref() if push_site >= 0 else None
     elif norm is not None and M >= NORM_SPLIT_ROWS and pull_site < 0:
         x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
+    if x is not None and tpp is None and _rows_gemv_ok(W, x, out, M, N, K):
+        return _gemm_rows(x, W, out, form=2 if swiglu else int(f32))
     if GEMV_IMPL == "mma" and M * K * 2 <= 160 * 1024:
         call("gemv_mma_bf16", W, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
              pull_site, push_site)
@@ -327,8 +335,18 @@ def gemv_i8(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
             x, res_in, add, gain, res_out = _pull_norm_rows(tp, pull_site, res_in, gain, res_out, eps), None, None, None, None
             pull_site = -1
             tpp = tp.cstruct_ref() if push_site >= 0 else None
-        elif M >= NORM_SPLIT_ROWS and pull_site < 0:
-            x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
+    if tpp is None and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K // 2):
+        # several rows: quantised once by a small kernel (the norm's own, where there is one), then the tcgen05 product
+        if x is None:
+            if add is None and res_out is not None and res_out.data_ptr() != res_in.data_ptr():
+                res_out.copy_(res_in)
+            q = rmsnorm(res_in, gain, eps, add=add, res_out=res_out,
+                        quant=(torch.empty(M, K, dtype=torch.int8, device=Wq.device), torch.empty(M, dtype=torch.float32, device=Wq.device)))
+        else:
+            q = quant_rows(x)
+        return _gemm_rows_i8(*q, Wq, wscale, out, form=2 if swiglu else mode >> 1)
+    if x is None and M >= NORM_SPLIT_ROWS and pull_site < 0:
+        x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
     call("gemv_i8", Wq, wscale, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
          pull_site, push_site)
     _count()
@@ -501,13 +519,8 @@ def gemm(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor | None = None,
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=A.device)
     assert out.stride(1) == 1
-    if M <= 128 and bn == 0 and SPLITK_GEMM:
-        ws, tickets = _splitk_scratch(A.device)
-        call("gemm_bf16_splitk", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual,
-             residual.stride(0) if residual is not None else 0, M, N, K, ws, ws.numel() * 4, tickets, tickets.numel(),
-             status_word(A.device))
-        _count()
-        return out
+    if M <= ROWS and bn == 0:
+        return _gemm_rows(A, W, out, residual, 1 if out.dtype == torch.float32 else 0)
     call("gemm_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual,
          residual.stride(0) if residual is not None else 0, M, N, K, bn, None, 0, status_word(A.device))
     _count()
@@ -532,6 +545,8 @@ def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = N
     if out is None:
         out = torch.empty(M, I, dtype=torch.bfloat16, device=A.device)
     assert out.stride(1) == 1
+    if M <= ROWS and I % 8 == 0:
+        return _gemm_rows(A, Wgu, out, form=2)
     if not (PAIR_GEMM and M >= PAIR_MIN_ROWS and I >= 128):
         return swiglu(gemm(A, Wgu), out=out)
     call("gemm_bf16_swiglu", A, A.stride(0), Wgu, Wgu.stride(0), out, out.stride(0), M, I, I, K, status_word(A.device))
@@ -542,32 +557,37 @@ def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = N
 def gemm_i8_swiglu(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: torch.Tensor,
                    out: torch.Tensor | None = None) -> torch.Tensor:
     """W8A8 form of :func:`gemm_swiglu`: ``out[M, I] = silu(gate) * up`` of the int8 gate|up projection, scales
-    applied before the activation.  More than 256 rows only (callers fall back to projection + ``quant_rows(swiglu)``)."""
+    applied before the activation.  At most 128 or more than 256 rows (callers fall back to projection + ``quant_rows(swiglu)``)."""
     M, K = Aq.shape
     I = Wq.shape[0] // 2
-    assert PAIR_GEMM and M >= PAIR_MIN_ROWS and I >= 128
+    assert M <= ROWS or (PAIR_GEMM and M >= PAIR_MIN_ROWS and I >= 128)
     if out is None:
         out = torch.empty(M, I, dtype=torch.bfloat16, device=Aq.device)
+    if M <= ROWS:
+        return _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, form=2)
     call("gemm_i8_swiglu", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), a_scale, w_scale, M, I, I, K,
          status_word(Aq.device))
     _count()
     return out
 
 
-# Products with at most 128 rows (batched decode buckets of 16..64 rows, small prefill chunks) split K
-# over CTAs: fp32 partial tiles in a per-device workspace, reduced by the last slice to arrive.
-SPLITK_GEMM = os.environ.get("COFFIN_SPLITK_GEMM", "1") != "0"
-_splitk: dict[int, tuple[torch.Tensor, torch.Tensor]] = {}
+# Products with at most this many rows (decode buckets, small prefill chunks): weights as the M operand, K split over a cluster.
+ROWS = 128
 
 
-def _splitk_scratch(device) -> tuple[torch.Tensor, torch.Tensor]:
-    idx = torch.device(device).index or 0      # one compute stream per device: its launches are ordered
-    s = _splitk.get(idx)
-    if s is None:
-        # 148 slice-tiles of 128 x 256 fp32 is the most one launch parks (tiles * slices <= SMs)
-        s = _splitk[idx] = (torch.empty(160 * 128 * 256, dtype=torch.float32, device=device),
-                            torch.zeros(4096, dtype=torch.int32, device=device))
-    return s
+def _gemm_rows(A, W, out, residual=None, form: int = 0):
+    """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows."""
+    call("gemm_rows_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
+         A.shape[0], out.shape[1], A.shape[1], form, status_word(A.device))
+    _count()
+    return out
+
+
+def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0):
+    call("gemm_rows_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
+         a_scale, w_scale, Aq.shape[0], out.shape[1], Aq.shape[1], form, status_word(Aq.device))
+    _count()
+    return out
 
 
 def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: torch.Tensor,
@@ -583,13 +603,8 @@ def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: 
         return None
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=Aq.device)
-    if M <= 128 and bn == 0 and SPLITK_GEMM:
-        ws, tickets = _splitk_scratch(Aq.device)
-        call("gemm_i8_splitk", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual,
-             residual.stride(0) if residual is not None else 0, a_scale, w_scale, M, N, K, ws, ws.numel() * 4, tickets,
-             tickets.numel(), status_word(Aq.device))
-        _count()
-        return out
+    if M <= ROWS and bn == 0:
+        return _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual, 1 if out.dtype == torch.float32 else 0)
     call("gemm_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual,
          residual.stride(0) if residual is not None else 0, a_scale, w_scale, M, N, K, bn, None, 0,
          status_word(Aq.device))

@@ -47,11 +47,8 @@ def gemm_f32out(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor) -> torch.Te
     M, Kd = A.shape
     N = W.shape[0]
     assert out.dtype == torch.float32 and out.stride(1) == 1 and A.stride(1) == 1 and W.stride(1) == 1
-    ws = tickets = None
-    if M <= 128 and K.SPLITK_GEMM:
-        ws, tickets = K._splitk_scratch(A.device)
-    call("gemm_bf16_f32out", A, A.stride(0), W, W.stride(0), out, out.stride(0), M, N, Kd, ws,
-         ws.numel() * 4 if ws is not None else 0, tickets, tickets.numel() if tickets is not None else 0, K.status_word(A.device))
+    call("gemm_bf16_f32out", A, A.stride(0), W, W.stride(0), out, out.stride(0), M, N, Kd,
+         K.status_word(A.device))
     K._count()
     return out
 
@@ -61,11 +58,8 @@ def gemm_mixed(A: torch.Tensor, W: torch.Tensor, main: torch.Tensor, gates: torc
     M, Kd = A.shape
     N, n_main = W.shape[0], main.shape[1]
     assert gates.dtype == torch.float32 and gates.shape[1] == N - n_main and main.stride(1) == gates.stride(1) == A.stride(1) == 1
-    ws = tickets = None
-    if M <= 128 and K.SPLITK_GEMM:
-        ws, tickets = K._splitk_scratch(A.device)
-    call("gemm_bf16_mixed", A, A.stride(0), W, W.stride(0), main, main.stride(0), gates, gates.stride(0), n_main, M, N, Kd, ws,
-         ws.numel() * 4 if ws is not None else 0, tickets, tickets.numel() if tickets is not None else 0, K.status_word(A.device))
+    call("gemm_bf16_mixed", A, A.stride(0), W, W.stride(0), main, main.stride(0), gates, gates.stride(0), n_main, M, N, Kd,
+         K.status_word(A.device))
     K._count()
 
 
@@ -95,11 +89,8 @@ def linear_xielu(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor, a: float, 
     elif T <= 8 and T * Kd * 2 <= 160 * 1024:
         call("gemv_mma_bf16_xielu", W, x.contiguous(), out, T, W.shape[0], Kd, out.stride(0), float(a), float(b))
     else:
-        ws = tickets = None
-        if T <= 128 and K.SPLITK_GEMM:
-            ws, tickets = K._splitk_scratch(x.device)
-        call("gemm_bf16_xielu", x, x.stride(0), W, W.stride(0), out, out.stride(0), T, W.shape[0], Kd, float(a), float(b), ws,
-             ws.numel() * 4 if ws is not None else 0, tickets, tickets.numel() if tickets is not None else 0, K.status_word(x.device))
+        call("gemm_bf16_xielu", x, x.stride(0), W, W.stride(0), out, out.stride(0), T, W.shape[0], Kd, float(a), float(b),
+             K.status_word(x.device))
     K._count(2 if out.dtype == torch.float32 else 1)
     return out
 

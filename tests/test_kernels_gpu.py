@@ -786,3 +786,46 @@ def test_argmax_and_attention_tickets_repeat_bit_exact():
         assert _intact(buf, 1, nh * hd) and int(tickets.abs().sum()) == 0
         outs.append(out.clone())
     assert torch.equal(outs[0], outs[1])
+
+
+@pytest.mark.parametrize("M,N,Kd", [(2, 8, 8), (7, 136, 72), (16, 2560, 4096), (17, 12352, 2560), (33, 6176, 512), (64, 1000, 200),
+                                    (65, 2048, 2048), (128, 40000, 264)])
+def test_few_row_products(M, N, Kd):
+    """Tile edges in rows (16 / 32 / 64 / 128) and columns, K tails, one slice and clusters of 2 to 8, one tile per CTA and several.
+    Sums of bf16 products in fp32: 1e-5; one rounding to bf16 more: 2^-8 of the value.  int8: sums exact, scales in fp32."""
+    k = K()
+    from coffin_b200.ops import mixers as X
+    A, W, res = bf(M, Kd, seed=1), bf(2 * N, Kd, s=Kd ** -0.5, seed=2), bf(M, N, seed=3)
+    Ad, Wd = A.to(DEV), W.to(DEV)
+    ref = A.to(DEV).double() @ Wd.double().t()
+    g, u = ref[:, :N], ref[:, N:]
+
+    def off(got, want):
+        return ((got.double() - want).norm() / want.norm()).item()
+
+    room = torch.full((M + 1, N + 8), 3.0, dtype=torch.bfloat16, device=DEV)
+    assert off(k.gemm(Ad, Wd[:N], out=room[:M, :N], residual=res.to(DEV)), g + res.to(DEV).double()) < 4e-3
+    assert bool((room[M] == 3.0).all()) and bool((room[:, N:] == 3.0).all())
+    f = torch.full((M, N), float("nan"), device=DEV)
+    assert off(k.gemm(Ad, Wd[:N], out=f), g) < 1e-5
+    assert off(X.gemm_f32out(Ad, Wd[:N], f.fill_(float("nan"))), g) < 1e-5
+    prod = torch.nn.functional.silu(g) * u
+    assert off(k.gemm_swiglu(Ad, Wd), prod) < 4e-3
+    main, gates = torch.empty(M, N, dtype=torch.bfloat16, device=DEV), torch.empty(M, N, device=DEV)
+    X.gemm_mixed(Ad, Wd, main, gates)
+    assert off(main, g) < 4e-3 and off(gates, u) < 1e-5
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    if M <= 8:                                       # decode projections of several rows end here too
+        assert off(k.gemv(Wd, Ad, out, swiglu=True), prod) < 4e-3
+        gain = torch.ones(Kd, device=DEV)
+        h = k.rmsnorm(Ad, gain, 1e-6)
+        assert off(k.gemv(Wd[:N], None, f, norm=(Ad, None, gain, None, 1e-6)), h.double() @ Wd[:N].double().t()) < 1e-5
+    if Kd % 16 == 0:
+        q, qs = k.quant_rows(Ad)
+        w8, ws = k.quant_rows(Wd)
+        r8 = (q.double() @ w8.double().t()) * qs.double()[:, None] * ws.double()
+        assert off(k.gemm_i8(q, qs, w8[:N], ws[:N], out=f), r8[:, :N]) < 1e-6
+        assert off(k.gemm_i8(q, qs, w8[:N], ws[:N], residual=res.to(DEV)), r8[:, :N] + res.to(DEV).double()) < 4e-3
+        assert off(k.gemm_i8_swiglu(q, qs, w8, ws), torch.nn.functional.silu(r8[:, :N]) * r8[:, N:]) < 4e-3
+        if M <= 8:
+            assert off(k.gemv_i8(w8[:N], ws[:N], Ad, f), r8[:, :N]) < 1e-6
