@@ -34,12 +34,17 @@ using namespace sm100;
 
 constexpr int kBQ = 128, kBKV = 64, kThreads = 352, kStages = 3;
 
+// One sequence of the call: its rows [row0, row0 + T) of q / gate / out, the position of the first, its first query tile of the grid
+// and its pool pages.
+struct AttnSeg { int row0, T, q_pos0, tile0; const int* block_table; };
+constexpr int kMaxSegs = 16;
+
 struct AttnTcArgs {
-  const bf16* q;                   // [T, nh, hd] normed and rotated queries
+  const bf16* q;                   // [rows, nh, hd] normed and rotated queries
   const bf16* gate; int64_t ldg;   // gate of head h at gate[t*ldg + h*2*hd + hd + d] (null: no gate)
-  const int* block_table;          // [pages] pool page ids of the sequence
-  bf16* out; int64_t ldo;          // [T, nh*hd]
-  int T, q_pos0, nh, nkv;
+  bf16* out; int64_t ldo;          // [rows, nh*hd]
+  int nh, nkv, nseg;
+  AttnSeg seg[kMaxSegs];
   float scale_log2;                // hd^-0.5 * log2(e)
   int* status;
   unsigned long long* trace;       // debugging: [tiles][8] %globaltimer stamps of CTA (0, 0), or null
@@ -90,14 +95,18 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // heavy (late) query tiles first: they walk the most pages
-  const int qt = (int)gridDim.x - 1 - (int)blockIdx.x, h = blockIdx.y, kvh = h / (a.nh / a.nkv);
+  const int gt = (int)gridDim.x - 1 - (int)blockIdx.x, h = blockIdx.y, kvh = h / (a.nh / a.nkv);
+  int si = 0;
+  while (si + 1 < a.nseg && gt >= a.seg[si + 1].tile0) ++si;
+  const AttnSeg sg = a.seg[si];
+  const int qt = gt - sg.tile0;
   const int row0 = qt * kBQ;
   const bool traced = a.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0;
   // stamp slots per tile: 0 K landed (seen by the MMA thread), 1 S issued, 2 S complete (seen by softmax),
   // 3 P published, 4 P and V seen by the MMA thread, 5 PV issued, 6 K requested, 7 V requested
   auto stamp = [&](int j, int slot) { if (traced) a.trace[j * 8 + slot] = now_ns(); };
-  const int last_row = min(a.T, row0 + kBQ) - 1;
-  const int n_tiles = (a.q_pos0 + last_row) / kBKV + 1;
+  const int last_row = min(sg.T, row0 + kBQ) - 1;
+  const int n_tiles = (sg.q_pos0 + last_row) / kBKV + 1;
 
   if (threadIdx.x == 0) {
     mbar_init(&q_full, 8);
@@ -133,7 +142,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       for (int j = 0; j < n_tiles && !*abort_flag; ++j) {
         const int s = j % kStages;
         const uint32_t ph = (j / kStages) & 1;
-        const int slot0 = a.block_table[j] * kBKV;
+        const int slot0 = sg.block_table[j] * kBKV;
         if (!wait_bar(&k_free[s], ph ^ 1, abort_flag)) { atomicCAS(a.status, 0, 65); abort_s = 1; break; }
         mbar_expect_tx(&k_full[s], KV_BYTES);
         stamp(j, 6);
@@ -198,11 +207,11 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     // 64 scores and of its O row, warp w + 4 the right half; row maxima and sums meet in shared memory.
     const int q = warp & 3, hf = (warp - 2) >> 2;
     const int r = q * 32 + lane;                       // query row of this thread inside the tile
-    const int t = row0 + r, pos = a.q_pos0 + t;
+    const int t = row0 + r, pos = sg.q_pos0 + t;
     const uint32_t lane_base = (uint32_t)(q * 32) << 16;
     // ---- Q row -> tensor memory (64 elements per store; the two warps of a quadrant alternate)
     {
-      const bf16* qrow = a.q + ((int64_t)min(t, a.T - 1) * a.nh + h) * HD;
+      const bf16* qrow = a.q + ((int64_t)(sg.row0 + min(t, sg.T - 1)) * a.nh + h) * HD;
 #pragma unroll 1
       for (int i = hf; i < HD / 64; i += 2) {
         uint32_t w[32];
@@ -235,7 +244,7 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
       if (lane == 0) mbar_arrive(&s_free[sb]);         // the accumulator may take S_{j+2}
       const int key0 = j * kBKV + hf * 32;
       float mx0 = -INFINITY, mx1 = -INFINITY;
-      if (j * kBKV + kBKV - 1 > a.q_pos0 + row0) {     // the tile touches the diagonal
+      if (j * kBKV + kBKV - 1 > sg.q_pos0 + row0) {     // the tile touches the diagonal
 #pragma unroll
         for (int c = 0; c < 32; c += 2) {
           const float x0 = key0 + c <= pos ? __uint_as_float(sv[c]) * a.scale_log2 : -INFINITY;
@@ -322,14 +331,14 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
     if (ok) {
       tc_fence_after();
       const float inv = 1.f / l;
-      const bf16* gp = a.gate ? a.gate + (int64_t)t * a.ldg + (int64_t)h * 2 * HD + HD : nullptr;
-      bf16* op = a.out + (int64_t)t * a.ldo + (int64_t)h * HD;
+      const bf16* gp = a.gate ? a.gate + (int64_t)(sg.row0 + t) * a.ldg + (int64_t)h * 2 * HD + HD : nullptr;
+      bf16* op = a.out + (int64_t)(sg.row0 + t) * a.ldo + (int64_t)h * HD;
 #pragma unroll 1
       for (int c0 = hf * (HD / 2); c0 < (hf + 1) * (HD / 2); c0 += 32) {
         uint32_t o[32];
         tmem_ld32(tmem_o + lane_base + c0, o);         // warp-collective: rows beyond T load too
         tmem_ld_wait();
-        if (t < a.T) {
+        if (t < sg.T) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             float f[8];
@@ -361,30 +370,40 @@ attn_tc_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ 
 }
 
 template <int HD>
-int launch_attn_tc(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnTcArgs& a, cudaStream_t st) {
+int launch_attn_tc(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnTcArgs& a, int tiles, cudaStream_t st) {
   const size_t smem = 2 * (size_t)kStages * kBKV * HD * 2 + 2 * (size_t)kBQ * kBKV * 2 + 1024;
   auto kern = attn_tc_kernel<HD>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
-  dim3 grid((unsigned)((a.T + kBQ - 1) / kBQ), (unsigned)a.nh);
+  dim3 grid((unsigned)tiles, (unsigned)a.nh);
   return (int)cb_launch(kern, grid, dim3(kThreads), smem, st, tmK, tmV, a);
 }
 }  // namespace
 
-// q [T, nh, hd] bf16 (normed, rotated); pools [slots, nkv, hd] bf16; causal; hd 64 or 256.
+// q [rows, nh, hd] bf16 (normed, rotated); pools [slots, nkv, hd] bf16; causal; hd 64 or 256.  seg (host memory): (first row, rows,
+// position of the first row, device pointer of the int32 block table) of each of the nseg sequences.
 CB_EXPORT int cb_attn_prefill_tc(const void* q, const void* gate, int64_t ldg, const void* kpool, const void* vpool,
-                                 int64_t slots, const void* block_table, void* out, int64_t ldo, int64_t T,
-                                 int64_t q_pos0, int64_t nh, int64_t nkv, int64_t hd, void* status, void* trace, void* stream) {
-  if (T == 0) return 0;
-  if (!q || !kpool || !vpool || !block_table || !out || !status || nh % nkv || (hd != 64 && hd != 256)) return CB_ERR_SHAPE;
+                                 int64_t slots, void* out, int64_t ldo, const void* seg, int64_t nseg, int64_t nh, int64_t nkv,
+                                 int64_t hd, void* status, void* trace, void* stream) {
+  if (!q || !kpool || !vpool || !seg || nseg < 1 || nseg > kMaxSegs || !out || !status || nh % nkv || (hd != 64 && hd != 256)) return CB_ERR_SHAPE;
   if ((uintptr_t)q & 15) return CB_ERR_ARG;
   CUtensorMap tmK, tmV;
   int rc = cb_make_tmap_2d(&tmK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kpool, (uint64_t)slots, (uint64_t)(nkv * hd), (uint64_t)(nkv * hd), kBKV, 64);
   if (rc) return rc;
   rc = cb_make_tmap_2d(&tmV, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vpool, (uint64_t)slots, (uint64_t)(nkv * hd), (uint64_t)(nkv * hd), kBKV, 64);
   if (rc) return rc;
-  AttnTcArgs a{(const bf16*)q, (const bf16*)gate, ldg, (const int*)block_table, (bf16*)out, ldo, (int)T, (int)q_pos0, (int)nh, (int)nkv,
-               1.4426950408889634f / sqrtf((float)hd), (int*)status, (unsigned long long*)trace};
-  if (hd == 256) return launch_attn_tc<256>(tmK, tmV, a, (cudaStream_t)stream);
-  return launch_attn_tc<64>(tmK, tmV, a, (cudaStream_t)stream);
+  AttnTcArgs a = {};
+  a.q = (const bf16*)q; a.gate = (const bf16*)gate; a.ldg = ldg; a.out = (bf16*)out; a.ldo = ldo;
+  a.nh = (int)nh; a.nkv = (int)nkv; a.nseg = (int)nseg;
+  int tiles = 0;
+  for (int i = 0; i < (int)nseg; ++i) {
+    const int64_t* s = (const int64_t*)seg + 4 * i;
+    if (s[0] < 0 || s[1] < 1 || s[2] < 0 || !s[3]) return CB_ERR_SHAPE;
+    a.seg[i] = AttnSeg{(int)s[0], (int)s[1], (int)s[2], tiles, (const int*)s[3]};
+    tiles += (int)((s[1] + kBQ - 1) / kBQ);
+  }
+  a.scale_log2 = 1.4426950408889634f / sqrtf((float)hd);
+  a.status = (int*)status; a.trace = (unsigned long long*)trace;
+  if (hd == 256) return launch_attn_tc<256>(tmK, tmV, a, tiles, (cudaStream_t)stream);
+  return launch_attn_tc<64>(tmK, tmV, a, tiles, (cudaStream_t)stream);
 }

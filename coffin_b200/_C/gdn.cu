@@ -14,7 +14,7 @@
 // position & 15: a step writes only slot pos&15 and reads the three before it, so the CTAs of
 // value heads that share a key head never race, and a speculative verify of up to 12 tokens
 // can be rolled back without restoring the window.
-#include "common.cuh"
+#include "sm100.cuh"
 
 namespace {
 
@@ -281,16 +281,22 @@ __global__ void __launch_bounds__(256) gdn_prep_kernel(const GdnPrepArgs a) {
   }
 }
 
-// ring[(pos0 + t) & 15] = proj[t] for the last min(T, 16) tokens of the chunk
-__global__ void gdn_ring_update_kernel(const bf16* proj, int64_t ldp, bf16* ring, int T, int pos0, int conv_dim) {
+// The sequences of one prefill forward: rows [row0, row0 + T) of the stacked projections, first position pos0, chunks
+// [c0, c0 + nc) of the forward's, state slot.
+struct GdnSeg { int row0, T, pos0, c0, nc, slot; };
+constexpr int kMaxSegs = 16;
+struct GdnSegs { int n; GdnSeg s[kMaxSegs]; };
+
+// ring[(pos0 + t) & 15] = proj[t] for the last min(T, 16) tokens of every sequence (blockIdx.y)
+__global__ void gdn_ring_update_kernel(const bf16* proj, int64_t ldp, bf16* ring, int conv_dim, const GdnSegs segs) {
   griddep_launch();
   griddep_wait();
-  const int first = max(0, T - kRing);
-  const int t = first + blockIdx.x;
-  if (t >= T) return;
-  const uint4* src = reinterpret_cast<const uint4*>(proj + (int64_t)t * ldp);
-  uint4* dst = reinterpret_cast<uint4*>(ring + (int64_t)((pos0 + t) & (kRing - 1)) * conv_dim);
-  for (int c = threadIdx.x; c < (conv_dim >> 3); c += blockDim.x) dst[c] = src[c];
+  const GdnSeg sg = segs.s[blockIdx.y];
+  const int t = sg.T - 1 - blockIdx.x;
+  if (t < 0) return;
+  uint4* dst = reinterpret_cast<uint4*>(ring + ((int64_t)sg.slot * kRing + ((sg.pos0 + t) & (kRing - 1))) * conv_dim);
+  const uint4* src = reinterpret_cast<const uint4*>(proj + (int64_t)(sg.row0 + t) * ldp);
+  for (int c = threadIdx.x; c < conv_dim / 8; c += blockDim.x) dst[c] = src[c];
 }
 
 // ---------------------------------------------------------------------------------------
@@ -310,7 +316,9 @@ struct GdnChunkArgs {
   // fused form (the prepare kernel takes conv + SiLU, the q/k normalisation, beta and g from the raw
   // projection rows itself; qn / kn / v / beta / g above are then unused)
   const bf16* proj; int64_t ldp; const float* conv_w; const float* A_log; const float* dt_bias; const bf16* ring;
-  int T, pos0, nk, nv;
+  int nk, nv;
+  GdnSegs segs;     // fused form; the others take one sequence
+  int heads;        // value heads of one key head that a CTA of the tensor-core forms takes, one after the other (1..4)
 };
 
 template <int DK, int DV>
@@ -454,6 +462,8 @@ struct GdnScanArgs {
   float* state;   // this sequence's state [nv, DK, DV] (read as S0, written as S_final)
   float* out;     // [T, nv*DV] fp32
   int T, nc, nv;
+  GdnSegs segs;   // bf16 scan: state is then the pool of all slots; the other forms take one sequence
+  int* status;    // set when a bounded wait ran out
 };
 
 template <int DK, int DV, int DVS>
@@ -591,21 +601,22 @@ __device__ __forceinline__ void frag_b(const float* M, int ld, int k0, int c0, i
   b[0] = __float_as_uint(p[0]);
   b[1] = __float_as_uint(p[4 * ld]);
 }
-// B fragment of the transpose: element (k, column) = M[column][k]
-__device__ __forceinline__ void frag_bt(const float* M, int ld, int k0, int c0, int g, int t, uint32_t* b) {
-  const float* p = M + (c0 + g) * ld + k0 + t;
-  b[0] = __float_as_uint(p[0]);
-  b[1] = __float_as_uint(p[4]);
-}
-
 template <int DK, int DV>
 struct PrepTcLayout {
-  static constexpr int L = kChunk, LDA = DK + 4, LDB = DK + 8, LDV = DV + 8, LDL = L + 4;
-  // R1 [L][max(LDA, LDV)]: K as a row operand, later V (k-major operand of the last product)
-  // R2 [L][LDB]: Q as a row operand (leading dimension LDA), later e^c K as a k-major operand
-  // Tm, Wi [L][LDL]; cs, bs [L].  105 KB for 128-wide heads: two CTAs per SM.
-  static constexpr int LD1 = LDA > LDV ? LDA : LDV;
-  static constexpr size_t floats = (size_t)L * LD1 + (size_t)L * LDB + (size_t)2 * L * LDL + 2 * L;
+  static constexpr int L = kChunk, LDA = DK + 4, LDV = DV + 8, LDL = L + 4;
+  // R1 [L][LDA]: K, a row operand of the first products and the k-major operand of the last
+  // R2 [L][LDV]: Q as a row operand (leading dimension LDA), then the block sums of the inversion, then V (k-major)
+  // Tm, Wi [L][LDL]; cs, bs [L] of up to four heads.  106 KB for 128-wide heads: two CTAs per SM.
+  static constexpr size_t floats = (size_t)L * LDA + (size_t)L * (LDA > LDV ? LDA : LDV) + (size_t)2 * L * LDL + 4 * 2 * L;
+};
+// Operands of the bf16 scan as the prepare kernel leaves them, per (head, chunk) one run of bytes that a bulk copy brings into
+// shared memory as it is: kcd, qe, ke [L][DK], ica [L][L].  16-byte piece c of row i lies at piece c ^ (i % 8), so that the eight
+// rows of a fragment load lie in different banks without padding.
+template <int DK>
+struct ScanOps {
+  static constexpr int L = kChunk, MAT = L * DK, TOTAL = 3 * L * DK + L * L;      // elements
+  static __device__ __forceinline__ int at(int i, int c) { return i * DK + ((((c >> 3) ^ (i & 7)) << 3) | (c & 7)); }
+  static __device__ __forceinline__ int at_ica(int i, int c) { return i * L + ((((c >> 3) ^ (i & 7)) << 3) | (c & 7)); }
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -615,246 +626,310 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Causal 4-tap conv + SiLU of NT consecutive tokens (first token t_first of the chunk whose rows are proj,
-// earlier rows come from the ring) for the four channels c..c+3 of this lane.  All NT + 3 rows are
-// requested before anything is computed.  val[k][j]: token t_first + k, channel c + j; rows past T give 0.
-template <int NT>
-__device__ __forceinline__ void conv_tokens(const bf16* proj, int64_t ldp, const bf16* ring, int conv_dim, const float* conv_w,
-                                            int c, bool act, int t_first, int T, int pos0, float (*val)[4]) {
-  float w[4][4];
+// Causal 4-tap conv + SiLU of eight consecutive tokens (first token t_first of the sequence whose rows are proj, earlier rows come
+// from the ring) for the four channels c..c+3 of this lane, in two steps: the raw rows are requested long before they are used.
+struct ConvRows {
+  uint2 raw[11];
+  float4 w[4];
+};
+__device__ __forceinline__ void conv_request(ConvRows& r, const bf16* proj, int64_t ldp, const bf16* ring, int conv_dim, const float* conv_w,
+                                             int c, bool act, int t_first, int T, int pos0) {
+#pragma unroll
+  for (int i = 0; i < 11; ++i) {
+    const int tt = t_first - 3 + i, pp = pos0 + tt;
+    const bf16* src = tt >= 0 ? proj + (int64_t)tt * ldp + c : ring + (int64_t)(pp & (kRing - 1)) * conv_dim + c;
+    r.raw[i] = act && tt < T && pp >= 0 ? *reinterpret_cast<const uint2*>(src) : make_uint2(0u, 0u);
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    r.w[j] = act ? *reinterpret_cast<const float4*>(conv_w + (int64_t)(c + j) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+// token t_first + k, its four channels; rows past T give 0
+__device__ __forceinline__ float4 conv_apply(const ConvRows& r, int k, bool live) {
+  float v[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    const float4 wj = act ? *reinterpret_cast<const float4*>(conv_w + (int64_t)(c + j) * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    w[j][0] = wj.x; w[j][1] = wj.y; w[j][2] = wj.z; w[j][3] = wj.w;
-  }
-  uint2 raw[NT + 3];
+    float x[4];
 #pragma unroll
-  for (int r = 0; r < NT + 3; ++r) {
-    const int tt = t_first - 3 + r, pp = pos0 + tt;
-    raw[r] = make_uint2(0u, 0u);
-    if (act) {
-      if (tt >= 0) { if (tt < T) raw[r] = *reinterpret_cast<const uint2*>(proj + (int64_t)tt * ldp + c); }
-      else if (pp >= 0) raw[r] = *reinterpret_cast<const uint2*>(ring + (int64_t)(pp & (kRing - 1)) * conv_dim + c);
+    for (int tap = 0; tap < 4; ++tap) {
+      const uint32_t word = (j < 2) ? r.raw[k + tap].x : r.raw[k + tap].y;
+      x[tap] = (j & 1) ? __uint_as_float(word & 0xffff0000u) : __uint_as_float(word << 16);
     }
+    v[j] = live ? silu_f(r.w[j].x * x[0] + r.w[j].y * x[1] + r.w[j].z * x[2] + r.w[j].w * x[3]) : 0.f;
   }
+  return make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ uint32_t smem_u32addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// Inclusive sums of the log decay over the 64 rows of a chunk, and beta: one warp, rows lane and lane + 32.
+__device__ __forceinline__ void chunk_decay(float g0, float g1, float be0, float be1, int lane, float* cs, float* bs) {
+  float x0 = g0, x1 = g1;
 #pragma unroll
-  for (int k = 0; k < NT; ++k) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float x[4];
-#pragma unroll
-      for (int tap = 0; tap < 4; ++tap) {
-        const uint32_t word = (j < 2) ? raw[k + tap].x : raw[k + tap].y;
-        x[tap] = (j & 1) ? __uint_as_float(word & 0xffff0000u) : __uint_as_float(word << 16);
-      }
-      val[k][j] = (act && t_first + k < T) ? silu_f(w[j][0] * x[0] + w[j][1] * x[1] + w[j][2] * x[2] + w[j][3] * x[3]) : 0.f;
-    }
+  for (int o = 1; o < 32; o <<= 1) {
+    const float y0 = __shfl_up_sync(0xffffffffu, x0, o), y1 = __shfl_up_sync(0xffffffffu, x1, o);
+    if (lane >= o) { x0 += y0; x1 += y1; }
   }
+  const float tot0 = __shfl_sync(0xffffffffu, x0, 31);
+  cs[lane] = x0;
+  cs[32 + lane] = x1 + tot0;
+  bs[lane] = be0;
+  bs[32 + lane] = be1;
 }
 
 // FUSE: the q / k / v rows, beta and g are computed here from the raw projection rows (what gdn_prep_kernel
 // does as a launch of its own, with an fp32 round trip through memory).
-// BF: kcd, qe, ke and ica leave as bf16 (same element offsets in the same regions) for the bf16 scan below;
+// BF: kcd, qe, ke and ica leave as bf16 in the layout of ScanOps (in kcd's region and those behind it) for the bf16 scan below;
 // the triangular system itself is still solved from TF32 products in fp32.
+// Bound by latencies, not by memory (two CTAs of 16 dependent phases an SM): at 2048 tokens, 16 key and 32 value heads 141 us with
+// the value rows fetched where they are used, the inverse column by column through shared memory and one value head a CTA; 95 us
+// with the rows requested ahead, the diagonal blocks inverted in registers and ldmatrix fragments; 87 us with the value heads of a
+// key head in one CTA.
 template <int DK, int DV, bool BF = false, bool FUSE = false>
 __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnChunkArgs a) {
   using Lay = PrepTcLayout<DK, DV>;
-  constexpr int L = kChunk, LDA = Lay::LDA, LDB = Lay::LDB, LDV = Lay::LDV, LDL = Lay::LDL;
+  using Ops = ScanOps<DK>;
+  constexpr int L = kChunk, LDA = Lay::LDA, LDV = Lay::LDV, LDL = Lay::LDL;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* R1 = reinterpret_cast<float*>(smem_raw);
-  float* R2 = R1 + L * Lay::LD1;
-  float* Tm = R2 + L * LDB;
+  float* R2 = R1 + L * LDA;
+  float* Tm = R2 + L * (LDA > LDV ? LDA : LDV);
   float* Wi = Tm + L * LDL;
-  float* cs = Wi + L * LDL;
-  float* bs = cs + L;
-  float* Ks = R1;          // phase 1-3
-  float* Qs = R2;          // phase 1-2
-  float* Kb = R2;          // phase 4-5
-  float* Vs = R1;          // phase 5
+  float* cs0 = Wi + L * LDL;                           // [heads][2][L]
+  float* Ks = R1;
+  float* Qs = R2;          // until the inversion
+  float* Vs = R2;          // after it
   griddep_launch();
   griddep_wait();
-  const int n = blockIdx.x, h = blockIdx.y, kh = h / a.rep, tid = threadIdx.x;
+  const int n = blockIdx.x, h0 = blockIdx.y * a.heads, kh = h0 / a.rep, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const int64_t t0 = (int64_t)n * L;
-  const float* kp = a.kn + ((int64_t)kh * a.Tp + t0) * DK;
-  const float* qp = a.qn + ((int64_t)kh * a.Tp + t0) * DK;
-  const float* vp = a.v + ((int64_t)h * a.Tp + t0) * DV;
+  int si = 0;
+  if (FUSE)
+    while (si + 1 < a.segs.n && n >= a.segs.s[si + 1].c0) ++si;
+  const GdnSeg sg = a.segs.s[si];
+  const int64_t t0 = (int64_t)(n - sg.c0) * L;         // first token of the chunk in its sequence
+  const bf16* proj = a.proj + (int64_t)sg.row0 * a.ldp;
   const int kdim = a.nk * DK, conv_dim = 2 * kdim + a.nv * DV;
+  const bf16* ring = a.ring + (int64_t)sg.slot * kRing * conv_dim;
+  const int i0 = lane * 4, tf = (int)t0 + warp * 8;    // fused: warp w takes tokens 8w .. 8w+7, a lane four adjacent channels of the head
+  auto ops_of = [&](int h) { return reinterpret_cast<bf16*>(a.kcd) + ((int64_t)h * a.nc + n) * Ops::TOTAL; };     // BF: kcd | qe | ke | ica
   if (FUSE) {
-    // warp w: tokens 8w .. 8w+7 of the chunk, a lane owns four adjacent channels of the key head
-    const int i0 = lane * 4;
+    ConvRows rq, rk;
     const bool act = i0 < DK;
-    const int tf = (int)t0 + warp * 8;
+    conv_request(rq, proj, a.ldp, ring, conv_dim, a.conv_w, kh * DK + i0, act, tf, sg.T, sg.pos0);
+    conv_request(rk, proj, a.ldp, ring, conv_dim, a.conv_w, kdim + kh * DK + i0, act, tf, sg.T, sg.pos0);
+    if (warp < a.heads) {
+      const int h = h0 + warp;
+      float g0 = 0.f, g1 = 0.f, be0 = 0.f, be1 = 0.f;
+      const float al = -__expf(a.A_log[h]), db = a.dt_bias[h];
+      const int64_t ta = t0 + lane, tb = ta + 32;
+      const bf16* pa = proj + ta * a.ldp + conv_dim + a.nv * DV;
+      const bf16* pb = proj + tb * a.ldp + conv_dim + a.nv * DV;
+      if (ta < sg.T) { be0 = sigmoid_f(__bfloat162float(pa[h])); g0 = al * softplus_f(__bfloat162float(pa[a.nv + h]) + db); }
+      if (tb < sg.T) { be1 = sigmoid_f(__bfloat162float(pb[h])); g1 = al * softplus_f(__bfloat162float(pb[a.nv + h]) + db); }
+      chunk_decay(g0, g1, be0, be1, lane, cs0 + warp * 2 * L, cs0 + warp * 2 * L + L);
+    }
 #pragma unroll
-    for (int kind = 0; kind < 2; ++kind) {              // 0: q, 1: k
-      float val[8][4];
-      conv_tokens<8>(a.proj, a.ldp, a.ring, conv_dim, a.conv_w, kind * kdim + kh * DK + i0, act, tf, a.T, a.pos0, val);
-      float* dstm = kind ? Ks : Qs;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const float ss = warp_sum(val[k][0] * val[k][0] + val[k][1] * val[k][1] + val[k][2] * val[k][2] + val[k][3] * val[k][3]);
-        const float sc = rsqrtf(ss + 1e-6f) * (kind == 0 ? rsqrtf((float)DK) : 1.f);
-        if (act) *reinterpret_cast<float4*>(dstm + (warp * 8 + k) * LDA + i0) = make_float4(val[k][0] * sc, val[k][1] * sc, val[k][2] * sc, val[k][3] * sc);
+    for (int k = 0; k < 8; ++k) {
+      const bool live = act && tf + k < sg.T;
+      const float4 q = conv_apply(rq, k, live), kk = conv_apply(rk, k, live);
+      const float sq = warp_sum(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
+      const float sk = warp_sum(kk.x * kk.x + kk.y * kk.y + kk.z * kk.z + kk.w * kk.w);
+      const float cq = rsqrtf(sq + 1e-6f) * rsqrtf((float)DK), ck = rsqrtf(sk + 1e-6f);
+      if (act) {
+        *reinterpret_cast<float4*>(Qs + (warp * 8 + k) * LDA + i0) = make_float4(q.x * cq, q.y * cq, q.z * cq, q.w * cq);
+        *reinterpret_cast<float4*>(Ks + (warp * 8 + k) * LDA + i0) = make_float4(kk.x * ck, kk.y * ck, kk.z * ck, kk.w * ck);
       }
     }
   } else {
+    const float* kp = a.kn + ((int64_t)kh * a.Tp + t0) * DK;
+    const float* qp = a.qn + ((int64_t)kh * a.Tp + t0) * DK;
     for (int idx = tid; idx < L * DK / 4; idx += 256) {
       const int i = idx / (DK / 4), c = (idx % (DK / 4)) * 4;
       *reinterpret_cast<float4*>(Ks + i * LDA + c) = *reinterpret_cast<const float4*>(kp + (int64_t)i * DK + c);
       *reinterpret_cast<float4*>(Qs + i * LDA + c) = *reinterpret_cast<const float4*>(qp + (int64_t)i * DK + c);
     }
-  }
-  if (tid < 32) {  // inclusive scan of g over the 64 rows
-    float g0, g1, be0, be1;
-    if (FUSE) {
-      const float al = -__expf(a.A_log[h]), db = a.dt_bias[h];
-      const int64_t ta = t0 + tid, tb = ta + 32;
-      const bf16* pa = a.proj + ta * a.ldp + conv_dim + a.nv * DV;
-      const bf16* pb = a.proj + tb * a.ldp + conv_dim + a.nv * DV;
-      g0 = g1 = be0 = be1 = 0.f;
-      if (ta < a.T) { be0 = sigmoid_f(__bfloat162float(pa[h])); g0 = al * softplus_f(__bfloat162float(pa[a.nv + h]) + db); }
-      if (tb < a.T) { be1 = sigmoid_f(__bfloat162float(pb[h])); g1 = al * softplus_f(__bfloat162float(pb[a.nv + h]) + db); }
-    } else {
-      g0 = a.g[(int64_t)h * a.Tp + t0 + tid]; g1 = a.g[(int64_t)h * a.Tp + t0 + 32 + tid];
-      be0 = a.beta[(int64_t)h * a.Tp + t0 + tid]; be1 = a.beta[(int64_t)h * a.Tp + t0 + 32 + tid];
+    if (warp == 0) {
+      const int64_t at = (int64_t)h0 * a.Tp + t0 + lane;
+      chunk_decay(a.g[at], a.g[at + 32], a.beta[at], a.beta[at + 32], lane, cs0, cs0 + L);
     }
-    float x0 = g0, x1 = g1;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const float y0 = __shfl_up_sync(0xffffffffu, x0, o), y1 = __shfl_up_sync(0xffffffffu, x1, o);
-      if (tid >= o) { x0 += y0; x1 += y1; }
-    }
-    const float tot0 = __shfl_sync(0xffffffffu, x0, 31);
-    cs[tid] = x0;
-    cs[32 + tid] = x1 + tot0;
-    bs[tid] = be0;
-    bs[32 + tid] = be1;
   }
   __syncthreads();
-  // ---- K K^T and Q K^T: warp (row tile of 16) x (column half of 32) ----------------------------
+  // ---- K K^T and Q K^T: warp (row tile of 16) x (column half of 32); fragments by ldmatrix (an 8 x 8 matrix of 16-bit values is
+  // 8 rows of four 32-bit ones) -----------------------------------------------------------------
+  const int r0 = (warp & 3) * 16, c0 = (warp >> 2) * 32;
+  float kk[4][4] = {};
   {
-    const int r0 = (warp & 3) * 16, c0 = (warp >> 2) * 32;
-    float kk[4][4] = {}, qk[4][4] = {};
+    const uint32_t a_off = 4u * ((r0 + (lane & 15)) * LDA + (lane >> 4) * 4);
+    const uint32_t b_off = 4u * ((c0 + (lane & 7) + (lane >> 4) * 8) * LDA + ((lane >> 3) & 1) * 4);
+    const uint32_t ka = smem_u32addr(Ks) + a_off, qa = smem_u32addr(Qs) + a_off, kb = smem_u32addr(Ks) + b_off;
+    float qk[4][4] = {};
+#pragma unroll 4
     for (int k0 = 0; k0 < DK; k0 += 8) {
-      uint32_t ak[4], aq[4];
-      frag_a(Ks, LDA, r0, k0, g, t, ak);
-      frag_a(Qs, LDA, r0, k0, g, t, aq);
+      uint32_t ak[4], aq[4], b[8];
+      ldsm_x4(ka + 4 * k0, ak);
+      ldsm_x4(qa + 4 * k0, aq);
+      ldsm_x4(kb + 4 * k0, b);
+      ldsm_x4(kb + 4 * (16 * LDA + k0), b + 4);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        uint32_t b[2];
-        frag_bt(Ks, LDA, k0, c0 + j * 8, g, t, b);
-        mma_tf32(kk[j], ak[0], ak[1], ak[2], ak[3], b[0], b[1]);
-        mma_tf32(qk[j], aq[0], aq[1], aq[2], aq[3], b[0], b[1]);
+        mma_tf32(kk[j], ak[0], ak[1], ak[2], ak[3], b[2 * j], b[2 * j + 1]);
+        mma_tf32(qk[j], aq[0], aq[1], aq[2], aq[3], b[2 * j], b[2 * j + 1]);
       }
     }
-    float* icap = a.ica + ((int64_t)h * a.nc + n) * L * L;
-    bf16* icab = reinterpret_cast<bf16*>(a.ica) + ((int64_t)h * a.nc + n) * L * L;
+    for (int hh = 0; hh < a.heads; ++hh) {
+      const float* cs = cs0 + hh * 2 * L;
+      float* icap = a.ica + ((int64_t)(h0 + hh) * a.nc + n) * L * L;
+      bf16* icab = ops_of(h0 + hh) + 3 * Ops::MAT;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int i = r0 + g + ((e & 2) ? 8 : 0), jj = c0 + j * 8 + 2 * t + (e & 1);
-        const float dec = (jj <= i) ? __expf(cs[i] - cs[jj]) : 0.f;
-        Tm[i * LDL + jj] = (jj < i) ? bs[i] * dec * kk[j][e] : 0.f;
-        if (BF) icab[i * L + jj] = __float2bfloat16(dec * qk[j][e]);
-        else icap[i * L + jj] = dec * qk[j][e];
-      }
-  }
-  // ---- qe = e^c Q for the scan (Q's last use), zero the inverse ---------------------------------
-  {
-    float* qep = a.qe + ((int64_t)h * a.nc + n) * L * DK;
-    bf16* qeb = reinterpret_cast<bf16*>(a.qe) + ((int64_t)h * a.nc + n) * L * DK;
-    for (int idx = tid; idx < L * DK / 4; idx += 256) {
-      const int i = idx / (DK / 4), c = (idx % (DK / 4)) * 4;
-      const float ec = __expf(cs[i]);
-      const float4 q = *reinterpret_cast<const float4*>(Qs + i * LDA + c);
-      if (BF) *reinterpret_cast<uint2*>(qeb + (int64_t)i * DK + c) = make_uint2(pack_bf162(q.x * ec, q.y * ec), pack_bf162(q.z * ec, q.w * ec));
-      else *reinterpret_cast<float4*>(qep + (int64_t)i * DK + c) = make_float4(q.x * ec, q.y * ec, q.z * ec, q.w * ec);
+        for (int e = 0; e < 4; e += 2) {
+          const int i = r0 + g + ((e & 2) ? 8 : 0), jj = c0 + j * 8 + 2 * t;
+          const float q0 = jj <= i ? __expf(cs[i] - cs[jj]) * qk[j][e] : 0.f, q1 = jj + 1 <= i ? __expf(cs[i] - cs[jj + 1]) * qk[j][e + 1] : 0.f;
+          if (BF) *reinterpret_cast<uint32_t*>(icab + Ops::at_ica(i, jj)) = pack_bf162(q0, q1);
+          else *reinterpret_cast<float2*>(icap + i * L + jj) = make_float2(q0, q1);
+        }
     }
-    for (int idx = tid; idx < L * L; idx += 256) Wi[(idx / L) * LDL + idx % L] = 0.f;
   }
-  __syncthreads();                                   // Tm complete, Q no longer needed
-  // ---- W = (I + Tm)^-1, blocked: the four 16x16 diagonal blocks are inverted by forward
-  // substitution (one warp each, one column per lane, 16 dependent rows instead of 64), then the
-  // blocks below the diagonal follow level by level from  W_ij = -W_ii (sum_{k=j..i-1} T_ik W_kj).
-  if (warp < 4 && lane < 16) {
-    const int b0 = warp * 16, c = lane;
+#pragma unroll 1
+  for (int hh = 0; hh < a.heads; ++hh) {
+  const int h = h0 + hh;
+  const float* cs = cs0 + hh * 2 * L;
+  const float* bs = cs + L;
+  bf16* ops = ops_of(h);
+  if (hh) __syncthreads();                           // the head before has read its W and V
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; e += 2) {
+      const int i = r0 + g + ((e & 2) ? 8 : 0), jj = c0 + j * 8 + 2 * t;
+      *reinterpret_cast<float2*>(Tm + i * LDL + jj) = make_float2(jj < i ? bs[i] * __expf(cs[i] - cs[jj]) * kk[j][e] : 0.f,
+                                                                  jj + 1 < i ? bs[i] * __expf(cs[i] - cs[jj + 1]) * kk[j][e + 1] : 0.f);
+    }
+  // the value rows are used last: requested now, they arrive during the inversion
+  ConvRows rv;
+  if (FUSE) conv_request(rv, proj, a.ldp, ring, conv_dim, a.conv_w, 2 * kdim + h * DV + i0, i0 < DV, tf, sg.T, sg.pos0);
+  __syncthreads();                                   // Tm complete
+  // ---- W = (I + Tm)^-1, blocked: the four 16x16 diagonal blocks are inverted by forward substitution (one warp each, a column
+  // per lane held in registers), then the blocks below the diagonal follow level by level from
+  // W_ij = -W_ii (sum_{k=j..i-1} T_ik W_kj).  The other four warps write qe = e^c Q of all heads (Q's last use) meanwhile.
+  if (warp < 4) {
+    const int b0 = warp * 16, c = lane & 15;
+    float w[16];
+#pragma unroll
     for (int i = 0; i < 16; ++i) {
       float acc = (i == c) ? 1.f : 0.f;
-      for (int jj = c; jj < i; ++jj) acc -= Tm[(b0 + i) * LDL + b0 + jj] * Wi[(b0 + jj) * LDL + b0 + c];
-      if (i >= c) Wi[(b0 + i) * LDL + b0 + c] = acc;
+      const float4* row = reinterpret_cast<const float4*>(Tm + (b0 + i) * LDL + b0);
+#pragma unroll
+      for (int q = 0; q < (i + 3) / 4; ++q) {
+        const float4 x = row[q];
+        const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (q * 4 + u < i) acc -= xs[u] * w[q * 4 + u];
+      }
+      w[i] = acc;
+    }
+    if (lane < 16) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) Wi[(b0 + i) * LDL + b0 + c] = w[i];
+    }
+  } else if (hh == 0) {
+    for (int qh = 0; qh < a.heads; ++qh) {
+      const float* cq = cs0 + qh * 2 * L;
+      float* qep = a.qe + ((int64_t)(h0 + qh) * a.nc + n) * L * DK;
+      bf16* qeb = ops_of(h0 + qh) + Ops::MAT;
+      for (int idx = tid - 128; idx < L * DK / 4; idx += 128) {
+        const int i = idx / (DK / 4), c = (idx % (DK / 4)) * 4;
+        const float ec = __expf(cq[i]);
+        const float4 q = *reinterpret_cast<const float4*>(Qs + i * LDA + c);
+        if (BF) *reinterpret_cast<uint2*>(qeb + Ops::at(i, c)) = make_uint2(pack_bf162(q.x * ec, q.y * ec), pack_bf162(q.z * ec, q.w * ec));
+        else *reinterpret_cast<float4*>(qep + (int64_t)i * DK + c) = make_float4(q.x * ec, q.y * ec, q.z * ec, q.w * ec);
+      }
     }
   }
   __syncthreads();
   {
-    float* P = R2;                                    // scratch for the block sums (Q is gone, e^c K not yet there)
+    float* P = R2;                                    // scratch for the block sums (Q is gone, V not yet there)
+    const int pr = tid >> 6, r = (tid >> 2) & 15, c = (tid & 3) * 4;   // a row of four columns of pair `pr` per thread
+#pragma unroll
     for (int d = 1; d < 4; ++d) {
-      const int npairs = 4 - d;
-      // P_p = sum_{k=j}^{i-1} T_ik W_kj for the pairs (i = j + d, j)
-      for (int idx = tid; idx < npairs * 256; idx += 256) {
-        const int pr = idx >> 8, r = (idx >> 4) & 15, c = idx & 15;
-        const int j = pr, i = pr + d;
-        float acc = 0.f;
-        for (int kk = j * 16; kk < i * 16; ++kk) acc += Tm[(i * 16 + r) * LDL + kk] * Wi[kk * LDL + j * 16 + c];
-        P[idx] = acc;
+      const int i = pr + d, j = pr;                   // P = sum_{k=j}^{i-1} T_ik W_kj
+      const bool on = i < 4;
+      if (on) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* tr = Tm + (i * 16 + r) * LDL + j * 16;
+        const float* wr = Wi + j * 16 * LDL + j * 16 + c;
+#pragma unroll
+        for (int kk2 = 0; kk2 < d * 16; kk2 += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(tr + kk2);
+          const float xs[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float4 y = *reinterpret_cast<const float4*>(wr + (kk2 + u) * LDL);
+            acc.x += xs[u] * y.x; acc.y += xs[u] * y.y; acc.z += xs[u] * y.z; acc.w += xs[u] * y.w;
+          }
+        }
+        *reinterpret_cast<float4*>(P + pr * 256 + r * 16 + c) = acc;
       }
       __syncthreads();
-      for (int idx = tid; idx < npairs * 256; idx += 256) {
-        const int pr = idx >> 8, r = (idx >> 4) & 15, c = idx & 15;
-        const int j = pr, i = pr + d;
-        float acc = 0.f;
-        for (int kk = 0; kk <= r; ++kk) acc += Wi[(i * 16 + r) * LDL + i * 16 + kk] * P[(pr << 8) + kk * 16 + c];
-        Wi[(i * 16 + r) * LDL + j * 16 + c] = -acc;
+      if (on) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float* dr = Wi + (i * 16 + r) * LDL + i * 16;
+#pragma unroll
+        for (int kk2 = 0; kk2 < 16; ++kk2)
+          if (kk2 <= r) {
+            const float x = dr[kk2];
+            const float4 y = *reinterpret_cast<const float4*>(P + pr * 256 + kk2 * 16 + c);
+            acc.x += x * y.x; acc.y += x * y.y; acc.z += x * y.z; acc.w += x * y.w;
+          }
+        *reinterpret_cast<float4*>(Wi + (i * 16 + r) * LDL + j * 16 + c) = make_float4(-acc.x, -acc.y, -acc.z, -acc.w);
       }
       __syncthreads();
     }
   }
-  // ---- W <- W diag(beta) (both products below carry beta); ke and e^c K from K -------------------
+  // ---- ke = e^{c_L - c} K for the scan ------------------------------------------------------------
   {
-    for (int idx = tid; idx < L * L; idx += 256) Wi[(idx / L) * LDL + idx % L] *= bs[idx % L];
     float* kep = a.ke + ((int64_t)h * a.nc + n) * L * DK;
-    bf16* keb = reinterpret_cast<bf16*>(a.ke) + ((int64_t)h * a.nc + n) * L * DK;
     const float cl = cs[L - 1];
     for (int idx = tid; idx < L * DK / 4; idx += 256) {
       const int i = idx / (DK / 4), c = (idx % (DK / 4)) * 4;
-      const float ec = __expf(cs[i]), el = __expf(cl - cs[i]);
+      const float el = __expf(cl - cs[i]);
       const float4 k = *reinterpret_cast<const float4*>(Ks + i * LDA + c);
-      if (BF) *reinterpret_cast<uint2*>(keb + (int64_t)i * DK + c) = make_uint2(pack_bf162(k.x * el, k.y * el), pack_bf162(k.z * el, k.w * el));
+      if (BF) *reinterpret_cast<uint2*>(ops + 2 * Ops::MAT + Ops::at(i, c)) = make_uint2(pack_bf162(k.x * el, k.y * el), pack_bf162(k.z * el, k.w * el));
       else *reinterpret_cast<float4*>(kep + (int64_t)i * DK + c) = make_float4(k.x * el, k.y * el, k.z * el, k.w * el);
-      *reinterpret_cast<float4*>(Kb + i * LDB + c) = make_float4(k.x * ec, k.y * ec, k.z * ec, k.w * ec);
     }
     if (tid == 0) a.ecl[(int64_t)h * a.nc + n] = __expf(cl);
   }
-  __syncthreads();                                   // K is no longer needed: V takes its place
-  // ---- nvv = W' V, kcd = W' (e^c K): warp (row tile) x (V or K half); W' is lower triangular ------
-  {
-    const int r0 = (warp & 3) * 16;
-    const bool isv = (warp >> 2) == 0;
-    if (isv) {                                       // the four V warps fetch V while the K warps multiply
-      if (FUSE) {                                    // conv + SiLU of the value channels: 16 tokens per warp, 8 at a time
-        const int i0 = lane * 4;
-        const bool act = i0 < DV;
-#pragma unroll 1
-        for (int half = 0; half < 2; ++half) {
-          const int tl = warp * 16 + half * 8;
-          float val[8][4];
-          conv_tokens<8>(a.proj, a.ldp, a.ring, conv_dim, a.conv_w, 2 * kdim + h * DV + i0, act, (int)t0 + tl, a.T, a.pos0, val);
+  if (FUSE) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (act) *reinterpret_cast<float4*>(Vs + (tl + k) * LDV + i0) = make_float4(val[k][0], val[k][1], val[k][2], val[k][3]);
-        }
-      } else {
-        for (int idx = tid; idx < L * DV / 4; idx += 128) {
-          const int i = idx / (DV / 4), c = (idx % (DV / 4)) * 4;
-          cp_async16(Vs + i * LDV + c, vp + (int64_t)i * DV + c);
-        }
-        cp_async_commit();
-        cp_async_wait_all();
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+    for (int k = 0; k < 8; ++k) {
+      const float4 v = conv_apply(rv, k, i0 < DV && tf + k < sg.T);
+      if (i0 < DV) *reinterpret_cast<float4*>(Vs + (warp * 8 + k) * LDV + i0) = v;
     }
-    const float* B = isv ? Vs : Kb;
-    const int ldb = isv ? LDV : LDB;
+  } else {
+    const float* vp = a.v + ((int64_t)h * a.Tp + t0) * DV;
+    for (int idx = tid; idx < L * DV / 4; idx += 256) {
+      const int i = idx / (DV / 4), c = (idx % (DV / 4)) * 4;
+      cp_async16(Vs + i * LDV + c, vp + (int64_t)i * DV + c);
+    }
+    cp_async_commit();
+    cp_async_wait_all();
+  }
+  __syncthreads();
+  // ---- nvv = W (beta V), kcd = W (beta e^c K): warp (row tile) x (V or K half); W is lower triangular, its columns take the
+  // factors of the rows they meet ------
+  {
+    const bool isv = (warp >> 2) == 0;
+    const float* B = isv ? Vs : Ks;
+    const int ldb = isv ? LDV : LDA;
     constexpr int NT = (DV > DK ? DV : DK) / 8;
     const int nt = (isv ? DV : DK) / 8;
     float acc[NT][4];
@@ -863,6 +938,10 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnC
     for (int k0 = 0; k0 < r0 + 16; k0 += 8) {
       uint32_t aw[4];
       frag_a(Wi, LDL, r0, k0, g, t, aw);
+      float f0 = bs[k0 + t], f1 = bs[k0 + t + 4];
+      if (!isv) { f0 *= __expf(cs[k0 + t]); f1 *= __expf(cs[k0 + t + 4]); }
+      aw[0] = __float_as_uint(__uint_as_float(aw[0]) * f0); aw[1] = __float_as_uint(__uint_as_float(aw[1]) * f0);
+      aw[2] = __float_as_uint(__uint_as_float(aw[2]) * f1); aw[3] = __float_as_uint(__uint_as_float(aw[3]) * f1);
 #pragma unroll
       for (int j = 0; j < NT; ++j) {
         if (j < nt) {
@@ -873,20 +952,20 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnC
       }
     }
     float* dst = isv ? a.nvv + ((int64_t)h * a.nc + n) * L * DV : a.kcd + ((int64_t)h * a.nc + n) * L * DK;
-    bf16* dstb = reinterpret_cast<bf16*>(a.kcd) + ((int64_t)h * a.nc + n) * L * DK;
     const int ldd = isv ? DV : DK;
 #pragma unroll
     for (int j = 0; j < NT; ++j) {
       if (j < nt) {
         if (BF && !isv) {
-          *reinterpret_cast<uint32_t*>(dstb + (r0 + g) * ldd + j * 8 + 2 * t) = pack_bf162(acc[j][0], acc[j][1]);
-          *reinterpret_cast<uint32_t*>(dstb + (r0 + g + 8) * ldd + j * 8 + 2 * t) = pack_bf162(acc[j][2], acc[j][3]);
+          *reinterpret_cast<uint32_t*>(ops + Ops::at(r0 + g, j * 8 + 2 * t)) = pack_bf162(acc[j][0], acc[j][1]);
+          *reinterpret_cast<uint32_t*>(ops + Ops::at(r0 + g + 8, j * 8 + 2 * t)) = pack_bf162(acc[j][2], acc[j][3]);
         } else {
           *reinterpret_cast<float2*>(dst + (r0 + g) * ldd + j * 8 + 2 * t) = make_float2(acc[j][0], acc[j][1]);
           *reinterpret_cast<float2*>(dst + (r0 + g + 8) * ldd + j * 8 + 2 * t) = make_float2(acc[j][2], acc[j][3]);
         }
       }
     }
+  }
   }
 }
 
@@ -1038,35 +1117,28 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_tc_kernel(const GdnScanArg
 // last.  Half-size operands make room for a three-stage ring of whole-chunk operand sets, so the loads
 // of chunk n+2 are in flight while chunk n is multiplied: the TF32 scan could only look half a chunk
 // ahead and spent most of a chunk waiting for L2.  Fragments come from ldmatrix (.trans where the
-// stored layout has the reduction index in rows); row strides of 16 B (mod 128) keep them conflict free.
+// stored layout has the reduction index in rows).
+// The copies of a chunk (56 KB a CTA) as 16-byte cp.async of all threads took 1430 of a chunk's 3640 cycles; as one bulk copy of an
+// operand set that the prepare kernel already laid out for the fragment loads they take none (2048 tokens, 32 heads: 72 -> 52 us).
 __device__ __forceinline__ void mma_bf16(float* c, const uint32_t* a, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t* r) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t addr, uint32_t* r) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ uint32_t smem_u32addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 template <int DK, int DVS>
 struct ScanBfLayout {
-  static constexpr int L = kChunk, LDA = DK + 8, LDL = L + 8, LDS = DVS + 8, STAGES = 3;
-  // stage: kcd [L][LDA], qe [L][LDA], ke [L][LDA], ica [L][LDL] (bf16); then S copy [DK][LDS], U [L][LDS] (bf16)
-  static constexpr size_t stage_bytes = 2 * ((size_t)3 * L * LDA + (size_t)L * LDL);
+  static constexpr int L = kChunk, LDS = DVS + 8, STAGES = 3;
+  // stages (ScanOps), then S copy [DK][LDS], U [L][LDS] (bf16)
+  static constexpr size_t stage_bytes = 2 * (size_t)ScanOps<DK>::TOTAL;
   static constexpr size_t bytes = STAGES * stage_bytes + 2 * ((size_t)DK * LDS + (size_t)L * LDS);
 };
 
 template <int DK, int DV, int DVS>
 __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArgs a) {
   using Lay = ScanBfLayout<DK, DVS>;
-  constexpr int L = kChunk, LDA = Lay::LDA, LDL = Lay::LDL, LDS = Lay::LDS, ST = Lay::STAGES;
+  using Ops = ScanOps<DK>;
+  constexpr int L = kChunk, LDS = Lay::LDS, ST = Lay::STAGES;
   constexpr int NRT = DK / 16;                 // row tiles of the state
   constexpr int CG = 8 / NRT;                  // column groups the 8 warps split the state into
   constexpr int NTS = (DVS / 8) / CG;          // n-tiles of a warp's state tile (2 or 4)
@@ -1074,39 +1146,33 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* Sb = reinterpret_cast<bf16*>(smem_raw + ST * Lay::stage_bytes);
   bf16* Ub = Sb + DK * LDS;
+  __shared__ uint64_t full[ST];
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < ST; ++i) sm100::mbar_init(&full[i], 1);
+    sm100::mbar_fence_init();
+  }
   griddep_launch();
   griddep_wait();
+  __syncthreads();
   const int h = blockIdx.x, sl = blockIdx.y, tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   const int col0 = sl * DVS;
-  const bf16* kcd = reinterpret_cast<const bf16*>(a.kcd);
-  const bf16* qe = reinterpret_cast<const bf16*>(a.qe);
-  const bf16* ke = reinterpret_cast<const bf16*>(a.ke);
-  const bf16* ica = reinterpret_cast<const bf16*>(a.ica);
+  const GdnSeg sg = a.segs.s[blockIdx.z];
+  const int nc = sg.nc;
+  // one thread requests a chunk's operand set as one copy; the threads that multiply spend no issue slots on it
   auto load_chunk = [&](int n) {
-    if (n < a.nc) {
-      bf16* st = reinterpret_cast<bf16*>(smem_raw + (size_t)(n % ST) * Lay::stage_bytes);
-      const int64_t base = (int64_t)h * a.nc + n;
-      for (int idx = tid; idx < L * DK / 8; idx += 256) {
-        const int i = idx / (DK / 8), c = (idx % (DK / 8)) * 8;
-        const int64_t off = base * L * DK + (int64_t)i * DK + c;
-        cp_async16(st + i * LDA + c, kcd + off);
-        cp_async16(st + L * LDA + i * LDA + c, qe + off);
-        cp_async16(st + 2 * L * LDA + i * LDA + c, ke + off);
-      }
-      for (int idx = tid; idx < L * L / 8; idx += 256) {
-        const int i = idx / (L / 8), c = (idx % (L / 8)) * 8;
-        cp_async16(st + 3 * L * LDA + i * LDL + c, ica + base * L * L + (int64_t)i * L + c);
-      }
+    if (n < nc && tid == 0) {
+      sm100::mbar_expect_tx(&full[n % ST], (uint32_t)Lay::stage_bytes);
+      sm100::bulk_load(smem_raw + (size_t)(n % ST) * Lay::stage_bytes,
+                       reinterpret_cast<const bf16*>(a.kcd) + ((int64_t)h * a.nc + sg.c0 + n) * Ops::TOTAL, (uint32_t)Lay::stage_bytes, &full[n % ST]);
     }
-    cp_async_commit();            // one group per chunk, empty past the end: the wait below counts groups
   };
   load_chunk(0);
   load_chunk(1);
   const int r0 = (warp & 3) * 16, ch = (warp >> 2) * 16;                // U / O tile of this warp: 16 rows x 16 columns
   const int s0 = (warp % NRT) * 16, sc0 = (warp / NRT) * (NTS * 8);    // state tile: 16 rows x NTS*8 columns
   // the warp's tile of the state: fp32 in registers for the whole scan, bf16 copy in shared memory
-  float* sp = a.state + (int64_t)h * DK * DV + col0;
+  float* sp = a.state + ((int64_t)sg.slot * a.nv + h) * DK * DV + col0;
   float accS[NTS][4];
 #pragma unroll
   for (int j = 0; j < NTS; ++j) {
@@ -1125,8 +1191,8 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
   float2 nv0[2], nv1[2];
   float el = 0.f;
   auto load_nv = [&](int n) {
-    if (n < a.nc) {
-      const int64_t base = (int64_t)h * a.nc + n;
+    if (n < nc) {
+      const int64_t base = (int64_t)h * a.nc + sg.c0 + n;
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const float* nvp = a.nvv + base * L * DV + col0 + ch + j * 8 + 2 * t;
@@ -1137,12 +1203,17 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
     }
   };
   load_nv(0);
-  for (int n = 0; n < a.nc; ++n) {
-    cp_async_wait_1();
-    __syncthreads();          // chunk n's operands and the S copy are visible; every warp has left chunk n-1
+  bool gave_up = false;
+  for (int n = 0; n < nc; ++n) {
+    if (!sm100::mbar_wait(&full[n % ST], (n / ST) & 1)) {      // bounded; leave time for the copies still in flight
+      if (lane == 0) atomicExch(a.status, 85);
+      for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+      gave_up = true;
+    }
+    if (__syncthreads_or(gave_up)) break;      // the S copy is visible; every warp has left chunk n-1, whose stage takes chunk n+2
     load_chunk(n + 2);
     const uint32_t st_u = smem_u32addr(smem_raw + (size_t)(n % ST) * Lay::stage_bytes);
-    const uint32_t a1_u = st_u, a2_u = st_u + 2 * L * LDA, a3_u = st_u + 4 * L * LDA, ic_u = st_u + 6 * L * LDA;
+    const uint32_t a1_u = st_u, a2_u = st_u + 2 * Ops::MAT, a3_u = st_u + 4 * Ops::MAT, ic_u = st_u + 6 * Ops::MAT;
     const float2 cnv0[2] = {nv0[0], nv0[1]}, cnv1[2] = {nv1[0], nv1[1]};
     const float cel = el;
     load_nv(n + 1);
@@ -1151,8 +1222,8 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
 #pragma unroll
     for (int k0 = 0; k0 < DK; k0 += 16) {
       uint32_t ak[4], aq[4], b[4];
-      ldsm_x4(a1_u + 2 * ((r0 + a_row) * LDA + k0 + a_col), ak);
-      ldsm_x4(a2_u + 2 * ((r0 + a_row) * LDA + k0 + a_col), aq);
+      ldsm_x4(a1_u + 2 * Ops::at(r0 + a_row, k0 + a_col), ak);
+      ldsm_x4(a2_u + 2 * Ops::at(r0 + a_row, k0 + a_col), aq);
       ldsm_x4_t(sb_u + 2 * ((k0 + b_row) * LDS + ch + b_col), b);
       mma_bf16(accU[0], ak, b[0], b[1]);
       mma_bf16(accU[1], ak, b[2], b[3]);
@@ -1169,7 +1240,7 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
     // ---- O += ica U (ica is lower triangular: k <= row) -----------------------------------------
     for (int k0 = 0; k0 < r0 + 16; k0 += 16) {
       uint32_t ai[4], b[4];
-      ldsm_x4(ic_u + 2 * ((r0 + a_row) * LDL + k0 + a_col), ai);
+      ldsm_x4(ic_u + 2 * Ops::at_ica(r0 + a_row, k0 + a_col), ai);
       ldsm_x4_t(ub_u + 2 * ((k0 + b_row) * LDS + ch + b_col), b);
       mma_bf16(accO[0], ai, b[0], b[1]);
       mma_bf16(accO[1], ai, b[2], b[3]);
@@ -1177,9 +1248,9 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       const int64_t ta = (int64_t)n * L + r0 + g, tb = ta + 8;
-      float* op = a.out + (int64_t)h * DV + col0 + ch + j * 8 + 2 * t;
-      if (ta < a.T) *reinterpret_cast<float2*>(op + ta * a.nv * DV) = make_float2(accO[j][0], accO[j][1]);
-      if (tb < a.T) *reinterpret_cast<float2*>(op + tb * a.nv * DV) = make_float2(accO[j][2], accO[j][3]);
+      float* op = a.out + ((int64_t)sg.row0 * a.nv + h) * DV + col0 + ch + j * 8 + 2 * t;
+      if (ta < sg.T) *reinterpret_cast<float2*>(op + ta * a.nv * DV) = make_float2(accO[j][0], accO[j][1]);
+      if (tb < sg.T) *reinterpret_cast<float2*>(op + tb * a.nv * DV) = make_float2(accO[j][2], accO[j][3]);
     }
     // ---- S <- ecl S + ke^T U on the warp's own tile; refresh the bf16 copy -----------------------
 #pragma unroll
@@ -1187,7 +1258,7 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
 #pragma unroll
     for (int k0 = 0; k0 < L; k0 += 16) {
       uint32_t at[4];
-      ldsm_x4_t(a3_u + 2 * ((k0 + t_row) * LDA + s0 + t_col), at);
+      ldsm_x4_t(a3_u + 2 * Ops::at(k0 + t_row, s0 + t_col), at);
 #pragma unroll
       for (int jj = 0; jj < NTS; jj += 2) {
         uint32_t b[4];
@@ -1202,7 +1273,6 @@ __global__ void __launch_bounds__(256) gdn_chunk_scan_bf_kernel(const GdnScanArg
       *reinterpret_cast<uint32_t*>(Sb + (s0 + g + 8) * LDS + sc0 + j * 8 + 2 * t) = pack_bf162(accS[j][2], accS[j][3]);
     }
   }
-  asm volatile("cp.async.wait_all;" ::: "memory");
 #pragma unroll
   for (int j = 0; j < NTS; ++j) {
     *reinterpret_cast<float2*>(sp + (int64_t)(s0 + g) * DV + sc0 + j * 8 + 2 * t) = make_float2(accS[j][0], accS[j][1]);
@@ -1307,25 +1377,87 @@ CB_EXPORT int cb_gdn_commit(void* state, const void* record, const void* slots, 
   return CB_ERR_SHAPE;
 }
 
-// Whole prefill chain for one sequence chunk of T tokens starting at pos0.
-// scratch (fp32) must hold cb_gdn_prefill_scratch(T, ...) floats.
-CB_EXPORT int64_t cb_gdn_prefill_scratch(int64_t T, int64_t nk, int64_t nv, int64_t dk, int64_t dv) {
-  const int64_t nc = (T + kChunk - 1) / kChunk, Tp = nc * kChunk;
+// Scratch (fp32 elements) of a prefill chain over T rows of `segs` sequences.
+namespace {
+int64_t prefill_scratch(int64_t T, int64_t segs, int64_t nk, int64_t nv, int64_t dk, int64_t dv) {
+  const int64_t nc = (T + kChunk - 1) / kChunk + segs - 1, Tp = nc * kChunk;
   return 2 * nk * Tp * dk + nv * Tp * dv + 2 * nv * Tp       // qn kn v beta g
          + nv * nc * kChunk * (dv + 3 * dk + kChunk) + ((nv * nc + 3) & ~(int64_t)3)  // nvv kcd qe ke ica ecl
          + T * nv * dv;                                        // scan output
 }
 
+template <int DK, int DV, int DVS>
+int run_prefill(const GdnPrepArgs& pa, const GdnChunkArgs& ca, const GdnScanArgs& sa, int nc, int conv_dim, const float* norm_w, bf16* out,
+                int64_t ldo, int64_t T, float eps, int gate_sigmoid, cudaStream_t st) {
+  const int nv = sa.nv, nseg = sa.segs.n;
+  int rc;
+  auto ring_update = [&]() {       // the fused prepare kernel reads the rows before the chunk there, so the ring moves on after it
+    return (int)cb_launch(gdn_ring_update_kernel, dim3(kRing, (unsigned)nseg), dim3(256), 0, st, ca.proj, ca.ldp, const_cast<bf16*>(ca.ring),
+                          conv_dim, sa.segs);
+  };
+  auto prepare = [&](auto kern, size_t smem) {
+    const int e = set_smem(kern, smem);
+    return e ? e : (int)cb_launch(kern, dim3((unsigned)nc, (unsigned)(nv / ca.heads)), dim3(256), smem, st, ca);
+  };
+  auto scan = [&](auto kern, size_t smem) {
+    const int e = set_smem(kern, smem);
+    return e ? e : (int)cb_launch(kern, dim3((unsigned)nv, (unsigned)(DV / DVS), (unsigned)nseg), dim3(256), smem, st, sa);
+  };
+  if (g_gdn_tc != 3)
+    if ((rc = (int)cb_launch(gdn_prep_kernel<DK, DV>, dim3((unsigned)((pa.Tp + kPrepTok - 1) / kPrepTok)), dim3(256), 0, st, pa))) return rc;
+  const size_t s_tc = sizeof(float) * PrepTcLayout<DK, DV>::floats;
+  if (g_gdn_tc >= 2) {
+    rc = g_gdn_tc == 3 ? prepare(gdn_chunk_prepare_tc_kernel<DK, DV, true, true>, s_tc) : prepare(gdn_chunk_prepare_tc_kernel<DK, DV, true>, s_tc);
+    if (rc || (rc = ring_update()) || (rc = scan(gdn_chunk_scan_bf_kernel<DK, DV, DVS>, ScanBfLayout<DK, DVS>::bytes))) return rc;
+  } else if (g_gdn_tc) {
+    if ((rc = ring_update()) || (rc = prepare(gdn_chunk_prepare_tc_kernel<DK, DV>, s_tc)) ||
+        (rc = scan(gdn_chunk_scan_tc_kernel<DK, DV, DVS>, sizeof(float) * ScanTcLayout<DK, DVS>::floats)))
+      return rc;
+  } else {
+    if ((rc = ring_update()) || (rc = prepare(gdn_chunk_prepare_kernel<DK, DV>, chunk_prepare_smem<DK, DV>())) ||
+        (rc = scan(gdn_chunk_scan_kernel<DK, DV, DVS>, chunk_scan_smem<DK, DVS>())))
+      return rc;
+  }
+  return (int)cb_launch(gdn_gated_norm_kernel<DV>, dim3((unsigned)((T * nv + 7) / 8)), dim3(256), 0, st, (const float*)sa.out, ca.proj + conv_dim,
+                        ca.ldp, norm_w, out, ldo, (int)T, nv, eps, gate_sigmoid);
+}
+}  // namespace
+
+CB_EXPORT int64_t cb_gdn_prefill_scratch(int64_t T, int64_t segs, int64_t nk, int64_t nv, int64_t dk, int64_t dv) {
+  return prefill_scratch(T, segs, nk, nv, dk, dv);
+}
+
+// Whole prefill chain over the rows of `nseg` sequences stacked in proj: seg (host memory) holds (rows, first position, state
+// slot) of each, in the order of the rows.  ring [slots, 16, conv_dim], state [slots, nv, dk, dv]; no slot twice.  scratch (fp32)
+// must hold cb_gdn_prefill_scratch floats.
 CB_EXPORT int cb_gdn_prefill(const void* proj, int64_t ldp, const void* conv_w, const void* A_log,
-                             const void* dt_bias, const void* norm_w, void* ring_seq, void* state_seq,
-                             void* scratch, void* out, int64_t ldo, int64_t T, int64_t pos0, int64_t nk,
-                             int64_t nv, int64_t dk, int64_t dv, float eps, int64_t gate_sigmoid, void* stream) {
-  if (T < 1 || nv % nk) return CB_ERR_SHAPE;
+                             const void* dt_bias, const void* norm_w, void* ring, void* state,
+                             void* scratch, void* out, int64_t ldo, const void* seg, int64_t nseg, int64_t nk,
+                             int64_t nv, int64_t dk, int64_t dv, float eps, int64_t gate_sigmoid, void* status, void* stream) {
+  if (!seg || !status || nseg < 1 || nseg > kMaxSegs || nv % nk) return CB_ERR_SHAPE;
   // the ring update moves whole 16-byte vectors of a projection row
-  if (ldp % 8 || (2 * nk * dk + nv * dv) % 8 || ((uintptr_t)proj & 15) || ((uintptr_t)ring_seq & 15)) return CB_ERR_SHAPE;
-  cudaStream_t st = (cudaStream_t)stream;
-  const int64_t nc = (T + kChunk - 1) / kChunk, Tp = nc * kChunk;
   const int conv_dim = (int)(2 * nk * dk + nv * dv);
+  if (ldp % 8 || conv_dim % 8 || ((uintptr_t)proj & 15) || ((uintptr_t)ring & 15)) return CB_ERR_SHAPE;
+  if (g_gdn_tc != 3 && nseg > 1) {                    // one sequence at a time
+    for (int64_t i = 0, row = 0; i < nseg; row += ((const int64_t*)seg)[3 * i], ++i) {
+      const int rc = cb_gdn_prefill((const bf16*)proj + row * ldp, ldp, conv_w, A_log, dt_bias, norm_w, ring, state, scratch,
+                                    (bf16*)out + row * ldo, ldo, (const int64_t*)seg + 3 * i, 1, nk, nv, dk, dv, eps, gate_sigmoid, status, stream);
+      if (rc) return rc;
+    }
+    return CB_OK;
+  }
+  GdnSegs segs = {};
+  segs.n = (int)nseg;
+  int64_t T = 0, nc = 0;
+  for (int i = 0; i < (int)nseg; ++i) {
+    const int64_t* q = (const int64_t*)seg + 3 * i;
+    if (q[0] < 1 || q[1] < 0 || q[2] < 0) return CB_ERR_SHAPE;
+    const int64_t c = (q[0] + kChunk - 1) / kChunk;
+    segs.s[i] = GdnSeg{(int)T, (int)q[0], (int)q[1], (int)nc, (int)c, (int)q[2]};
+    T += q[0];
+    nc += c;
+  }
+  const int64_t Tp = nc * kChunk, rep = nv / nk;
   float* p = (float*)scratch;
   float* qn = p; p += nk * Tp * dk;
   float* kn = p; p += nk * Tp * dk;
@@ -1339,74 +1471,27 @@ CB_EXPORT int cb_gdn_prefill(const void* proj, int64_t ldp, const void* conv_w, 
   float* ica = p; p += nv * nc * kChunk * kChunk;
   float* ecl = p; p += (nv * nc + 3) & ~(int64_t)3;
   float* o = p;
+  // the forms with a prep kernel of their own take one sequence: its ring and state rows
+  bf16* ring0 = (bf16*)ring;
+  float* state0 = (float*)state;
+  if (g_gdn_tc != 3) {
+    ring0 += (int64_t)segs.s[0].slot * kRing * conv_dim;
+    state0 += (int64_t)segs.s[0].slot * nv * dk * dv;
+    segs.s[0].slot = 0;
+  }
   GdnPrepArgs pa{(const bf16*)proj, ldp, (const float*)conv_w, (const float*)A_log, (const float*)dt_bias,
-                 (const bf16*)ring_seq, qn, kn, v, beta, g, (int)T, (int)Tp, (int)pos0, (int)nk, (int)nv};
-  GdnChunkArgs ca{qn, kn, v, beta, g, nvv, kcd, ica, qe, ke, ecl, (int)Tp, (int)nc, (int)(nv / nk),
+                 ring0, qn, kn, v, beta, g, (int)T, (int)Tp, segs.s[0].pos0, (int)nk, (int)nv};
+  GdnChunkArgs ca{qn, kn, v, beta, g, nvv, kcd, ica, qe, ke, ecl, (int)Tp, (int)nc, (int)rep,
                   (const bf16*)proj, ldp, (const float*)conv_w, (const float*)A_log, (const float*)dt_bias,
-                  (const bf16*)ring_seq, (int)T, (int)pos0, (int)nk, (int)nv};
-  GdnScanArgs sa{nvv, kcd, ica, qe, ke, ecl, (float*)state_seq, o, (int)T, (int)nc, (int)nv};
-  cudaError_t e;
-  int rc;
-#define GDN_PREFILL(DK_, DV_, DVS_)                                                                      \
-  do {                                                                                                   \
-    if (g_gdn_tc != 3) {                                                                                 \
-      e = cb_launch(gdn_prep_kernel<DK_, DV_>, dim3((unsigned)((Tp + kPrepTok - 1) / kPrepTok)), dim3(256), 0, st, pa);                \
-      if (e != cudaSuccess) return (int)e;                                                               \
-    }                                                                                                    \
-    if (g_gdn_tc >= 2) {                                                                                 \
-      /* the fused prepare kernel reads the ring (rows before the chunk), so the ring moves on after it */ \
-      size_t s1 = sizeof(float) * PrepTcLayout<DK_, DV_>::floats;                                        \
-      if (g_gdn_tc == 3) {                                                                               \
-        if ((rc = set_smem(gdn_chunk_prepare_tc_kernel<DK_, DV_, true, true>, s1))) return rc;           \
-        e = cb_launch(gdn_chunk_prepare_tc_kernel<DK_, DV_, true, true>, dim3((unsigned)nc, (unsigned)nv), dim3(256), s1, st, ca); \
-      } else {                                                                                           \
-        if ((rc = set_smem(gdn_chunk_prepare_tc_kernel<DK_, DV_, true>, s1))) return rc;                 \
-        e = cb_launch(gdn_chunk_prepare_tc_kernel<DK_, DV_, true>, dim3((unsigned)nc, (unsigned)nv), dim3(256), s1, st, ca); \
-      }                                                                                                  \
-      if (e != cudaSuccess) return (int)e;                                                               \
-      e = cb_launch(gdn_ring_update_kernel, dim3((unsigned)(T < kRing ? T : kRing)), dim3(256), 0, st,   \
-                    (const bf16*)proj, ldp, (bf16*)ring_seq, (int)T, (int)pos0, conv_dim);               \
-      if (e != cudaSuccess) return (int)e;                                                               \
-      size_t s2 = ScanBfLayout<DK_, DVS_>::bytes;                                                        \
-      if ((rc = set_smem(gdn_chunk_scan_bf_kernel<DK_, DV_, DVS_>, s2))) return rc;                      \
-      e = cb_launch(gdn_chunk_scan_bf_kernel<DK_, DV_, DVS_>, dim3((unsigned)nv, (unsigned)(DV_ / DVS_)), \
-                    dim3(256), s2, st, sa);                                                              \
-      if (e != cudaSuccess) return (int)e;                                                               \
-    } else if (g_gdn_tc) {                                                                               \
-      e = cb_launch(gdn_ring_update_kernel, dim3((unsigned)(T < kRing ? T : kRing)), dim3(256), 0, st,   \
-                    (const bf16*)proj, ldp, (bf16*)ring_seq, (int)T, (int)pos0, conv_dim);               \
-      if (e != cudaSuccess) return (int)e;                                                               \
-      size_t s1 = sizeof(float) * PrepTcLayout<DK_, DV_>::floats;                                        \
-      if ((rc = set_smem(gdn_chunk_prepare_tc_kernel<DK_, DV_>, s1))) return rc;                         \
-      e = cb_launch(gdn_chunk_prepare_tc_kernel<DK_, DV_>, dim3((unsigned)nc, (unsigned)nv), dim3(256), s1, st, ca); \
-      if (e != cudaSuccess) return (int)e;                                                               \
-      size_t s2 = sizeof(float) * ScanTcLayout<DK_, DVS_>::floats;                                       \
-      if ((rc = set_smem(gdn_chunk_scan_tc_kernel<DK_, DV_, DVS_>, s2))) return rc;                      \
-      e = cb_launch(gdn_chunk_scan_tc_kernel<DK_, DV_, DVS_>, dim3((unsigned)nv, (unsigned)(DV_ / DVS_)), \
-                    dim3(256), s2, st, sa);                                                              \
-      if (e != cudaSuccess) return (int)e;                                                               \
-    } else {                                                                                             \
-      e = cb_launch(gdn_ring_update_kernel, dim3((unsigned)(T < kRing ? T : kRing)), dim3(256), 0, st,   \
-                    (const bf16*)proj, ldp, (bf16*)ring_seq, (int)T, (int)pos0, conv_dim);               \
-      if (e != cudaSuccess) return (int)e;                                                               \
-      size_t s1 = chunk_prepare_smem<DK_, DV_>();                                                        \
-      if ((rc = set_smem(gdn_chunk_prepare_kernel<DK_, DV_>, s1))) return rc;                            \
-      e = cb_launch(gdn_chunk_prepare_kernel<DK_, DV_>, dim3((unsigned)nc, (unsigned)nv), dim3(256), s1, st, ca); \
-      if (e != cudaSuccess) return (int)e;                                                               \
-      size_t s2 = chunk_scan_smem<DK_, DVS_>();                                                          \
-      if ((rc = set_smem(gdn_chunk_scan_kernel<DK_, DV_, DVS_>, s2))) return rc;                         \
-      e = cb_launch(gdn_chunk_scan_kernel<DK_, DV_, DVS_>, dim3((unsigned)nv, (unsigned)(DV_ / DVS_)),    \
-                    dim3(256), s2, st, sa);                                                              \
-      if (e != cudaSuccess) return (int)e;                                                               \
-    }                                                                                                    \
-    const int64_t tasks = T * nv;                                                                        \
-    e = cb_launch(gdn_gated_norm_kernel<DV_>, dim3((unsigned)((tasks + 7) / 8)), dim3(256), 0, st,       \
-                  (const float*)o, (const bf16*)proj + conv_dim, ldp, (const float*)norm_w, (bf16*)out,  \
-                  ldo, (int)T, (int)nv, eps, (int)gate_sigmoid);                                         \
-    return (int)e;                                                                                       \
-  } while (0)
-  if (dk == 128 && dv == 128) GDN_PREFILL(128, 128, 32);
-  if (dk == 64 && dv == 64) GDN_PREFILL(64, 64, 32);
-#undef GDN_PREFILL
+                  ring0, (int)nk, (int)nv, segs, 1};
+  // The value heads of a key head share its conv rows, norms and products.  One CTA for all of them pays once every SM has a
+  // CTA to work on; below that the longer CTA would only add latency.
+  if (g_gdn_tc == 3 && rep <= 4 && nk * nc >= 148) ca.heads = (int)rep;
+  GdnScanArgs sa{nvv, kcd, ica, qe, ke, ecl, state0, o, (int)T, (int)nc, (int)nv, segs, (int*)status};
+  cudaStream_t st = (cudaStream_t)stream;
+  if (dk == 128 && dv == 128)
+    return run_prefill<128, 128, 32>(pa, ca, sa, (int)nc, conv_dim, (const float*)norm_w, (bf16*)out, ldo, T, eps, (int)gate_sigmoid, st);
+  if (dk == 64 && dv == 64)
+    return run_prefill<64, 64, 32>(pa, ca, sa, (int)nc, conv_dim, (const float*)norm_w, (bf16*)out, ldo, T, eps, (int)gate_sigmoid, st);
   return CB_ERR_SHAPE;
 }

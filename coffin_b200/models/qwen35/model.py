@@ -505,8 +505,8 @@ class Qwen35Model:
                       want_hidden: bool = False) -> list:
         """Chunks of several sequences in ONE forward: ``items[i] = (tokens [T_i], pos0, slot,
         block_table)``.  The rows of all chunks are stacked, so every projection is one GEMM over
-        ``sum(T_i)`` rows (short prompts share weight tiles instead of each streaming the weights); the
-        delta-net scan and the attention, which are per sequence, run per chunk on its row range.
+        ``sum(T_i)`` rows (short prompts share weight tiles instead of each streaming the weights), and the
+        delta-net chain, the attention and the head take all sequences in a launch.
         ``embeds`` / ``cos_sin`` cover the stacked rows (only used with a single item by the engine).
         Returns, per item, the fp32 logits ``[vocab]`` of its last token or ``None``
         (reference: ``models/qwen35/model.py:861`` ``prefill_group``)."""
@@ -529,8 +529,10 @@ class Qwen35Model:
             offs.append(offs[-1] + n)
         slots = ws["slots"][:T]
         ridx = ws["ridx"][:T] if cos_sin is None else None
+        tables = []
         for i, (it, n) in enumerate(zip(items, lens)):          # pool slots (and 1-D rotary rows): one small kernel per chunk
             bt = it[3] if it[3].dtype == torch.int32 and it[3].is_contiguous() else it[3].to(torch.int32).contiguous()
+            tables.append(bt)
             K.call("prefill_index", bt, it[1], n, K.BLOCK, slots[offs[i]:offs[i + 1]],
                    ridx[offs[i]:offs[i + 1]] if ridx is not None else None)
             K._count()
@@ -540,6 +542,19 @@ class Qwen35Model:
             cos, sin = cos_sin[0].float().contiguous(), cos_sin[1].float().contiguous()
             ridx = None
         q8 = (ws["q8"][:T], ws["s8"][:T]) if "q8" in ws else None
+        # the delta-net layers take runs of sequences with distinct slots, the attention layers all of them
+        runs: list[list[int]] = []
+        for i, it in enumerate(items):
+            if not runs or len(runs[-1]) == K.GDN_SEGS or any(items[k][2] == it[2] for k in runs[-1]):
+                runs.append([])
+            runs[-1].append(i)
+        lin_segs = [(slice(offs[r[0]], offs[r[-1] + 1]), [(lens[i], items[i][1], items[i][2]) for i in r]) for r in runs]
+        if self.lin_ids:
+            need = max(K.gdn_prefill_scratch_floats(sl.stop - sl.start, c.linear_num_key_heads, c.linear_num_value_heads,
+                                                    c.linear_key_head_dim, c.linear_value_head_dim, len(segs)) for sl, segs in lin_segs)
+            if ws["gdn"].numel() < need:
+                ws["gdn"] = torch.empty(need, dtype=torch.float32, device=self.device)
+        att_segs = [(offs[i], n, it[1], bt) for i, (it, n, bt) in enumerate(zip(items, lens, tables))]
         for li, lw in enumerate(self.layers):
             # an int8 projection takes its int8 rows straight from the norm kernel (no bf16 copy, no quantise launch)
             aq = q8 if isinstance(lw.w_in, QW) else None
@@ -550,12 +565,10 @@ class Qwen35Model:
             if lw.kind == LINEAR:
                 j = self.lin_ids[li]
                 act = ws["act"][:T, :c.lin_vdim]
-                for i, (it, n) in enumerate(zip(items, lens)):
-                    sl = slice(offs[i], offs[i + 1])
-                    K.gdn_prefill(proj[sl], lw.conv_w, lw.A_log, lw.dt_bias, lw.norm_w, self.ring[j, it[2]],
-                                  self.state[j, it[2]], ws["gdn"], act[sl], pos0=it[1], nk=c.linear_num_key_heads,
-                                  nv=c.linear_num_value_heads, dk=c.linear_key_head_dim, dv=c.linear_value_head_dim,
-                                  eps=self.eps)
+                for sl, segs in lin_segs:
+                    K.gdn_prefill_group(proj[sl], lw.conv_w, lw.A_log, lw.dt_bias, lw.norm_w, self.ring[j], self.state[j], ws["gdn"],
+                                        act[sl], segs, nk=c.linear_num_key_heads, nv=c.linear_num_value_heads,
+                                        dk=c.linear_key_head_dim, dv=c.linear_value_head_dim, eps=self.eps)
             else:
                 j = self.full_ids[li]
                 act = ws["act"][:T, :c.num_attention_heads * c.head_dim]
@@ -563,10 +576,8 @@ class Qwen35Model:
                 K.attn_prep(proj, lw.qg, lw.kg, cos, sin, ridx, slots, q, self.kpool[j], self.vpool[j],
                             nh=c.num_attention_heads, nkv=c.num_key_value_heads, hd=c.head_dim,
                             rot=c.rotary_dim, eps=self.eps, **self._kvs(j))
-                for i, (it, n) in enumerate(zip(items, lens)):
-                    sl = slice(offs[i], offs[i + 1])
-                    K.attn_prefill(q[sl], proj[sl], self.kpool[j], self.vpool[j], it[3], act[sl], q_pos0=it[1],
-                                   nh=c.num_attention_heads, nkv=c.num_key_value_heads, hd=c.head_dim, **self._kvs(j))
+                K.attn_prefill_group(q, proj, self.kpool[j], self.vpool[j], act, att_segs, nh=c.num_attention_heads,
+                                     nkv=c.num_key_value_heads, hd=c.head_dim, **self._kvs(j))
             aq = q8 if lw.moe is None and isinstance(lw.w_gu, QW) else None
             if self.tp_world > 1 or (self.tp_force and not c.is_moe):
                 part = self._row_parallel(act, lw.w_out, ws["part"][:T])
@@ -592,12 +603,14 @@ class Qwen35Model:
             return out
         if want_hidden:
             self.last_hidden = K.rmsnorm(res, self.final_gain, self.eps)
-        for i in range(len(items)):
-            if want_logits[i]:
-                last = offs[i + 1] - 1
-                local = torch.empty(1, self.vocab_local, dtype=torch.float32, device=self.device)
-                self._gemv(self.lm_head, None, local, norm=(res[last:last + 1].contiguous(), None, self.final_gain, None, self.eps))
-                out[i] = self._gather_logits(local, 1)[0]
+        wanted = [i for i in range(len(items)) if want_logits[i]]
+        for k in range(0, len(wanted), WIDE):           # the head streams its weights once for the last rows of all sequences
+            some = wanted[k:k + WIDE]
+            rows = res[offs[some[0] + 1] - 1:offs[some[0] + 1]] if len(some) == 1 else torch.cat([res[offs[i + 1] - 1:offs[i + 1]] for i in some])
+            local = torch.empty(len(some), self.vocab_local, dtype=torch.float32, device=self.device)
+            self._gemv(self.lm_head, None, local, norm=(rows.contiguous(), None, self.final_gain, None, self.eps))
+            for i, row in zip(some, self._gather_logits(local, len(some))):
+                out[i] = row
         return out
 
     # ------------------------------------------------------------------ tensor-parallel helpers

@@ -630,20 +630,35 @@ def gdn_commit(state, record, slots, steps, *, nv, dk, dv) -> None:
     _count()
 
 
-def gdn_prefill_scratch_floats(T: int, nk: int, nv: int, dk: int, dv: int) -> int:
+GDN_SEGS = 16        # sequences of one delta-net prefill call
+
+
+def gdn_prefill_scratch_floats(T: int, nk: int, nv: int, dk: int, dv: int, segs: int = 1) -> int:
     fn = _lib.lib().cb_gdn_prefill_scratch
     import ctypes
     fn.restype = ctypes.c_int64
-    return int(fn(*[ctypes.c_int64(v) for v in (T, nk, nv, dk, dv)]))
+    return int(fn(*[ctypes.c_int64(v) for v in (T, segs, nk, nv, dk, dv)]))
 
 
 def gdn_prefill(proj, conv_w, A_log, dt_bias, norm_w, ring_seq, state_seq, scratch, out, *, pos0, nk, nv, dk, dv,
                 eps, gate_sigmoid: bool = False) -> torch.Tensor:
-    T = proj.shape[0]
-    assert scratch.dtype == torch.float32 and scratch.numel() >= gdn_prefill_scratch_floats(T, nk, nv, dk, dv)
-    call("gdn_prefill", proj, proj.stride(0), conv_w, A_log, dt_bias, norm_w, ring_seq, state_seq, scratch,
-         out, out.stride(0), T, pos0, nk, nv, dk, dv, float(eps), int(gate_sigmoid))
-    _count(5)
+    """One sequence: its rows ``proj``, conv ring ``[16, channels]`` and state ``[nv, dk, dv]``."""
+    return gdn_prefill_group(proj, conv_w, A_log, dt_bias, norm_w, ring_seq, state_seq, scratch, out, [(proj.shape[0], pos0, 0)],
+                             nk=nk, nv=nv, dk=dk, dv=dv, eps=eps, gate_sigmoid=gate_sigmoid)
+
+
+def gdn_prefill_group(proj, conv_w, A_log, dt_bias, norm_w, ring, state, scratch, out, segs, *, nk, nv, dk, dv, eps,
+                      gate_sigmoid: bool = False) -> torch.Tensor:
+    """Rows of at most ``GDN_SEGS`` sequences stacked in ``proj``: ``segs = [(rows, first position, slot)]`` with distinct slots of
+    ``ring [slots, 16, channels]`` and ``state [slots, nv, dk, dv]``."""
+    import ctypes
+    assert sum(s[0] for s in segs) == proj.shape[0] and len({s[2] for s in segs}) == len(segs)
+    assert scratch.dtype == torch.float32 and scratch.numel() >= gdn_prefill_scratch_floats(proj.shape[0], nk, nv, dk, dv, len(segs))
+    table = (ctypes.c_int64 * (3 * len(segs)))(*[v for s in segs for v in s])
+    call("gdn_prefill", proj, proj.stride(0), conv_w, A_log, dt_bias, norm_w, ring, state, scratch, out, out.stride(0),
+         ctypes.c_void_p(ctypes.addressof(table)), len(segs), nk, nv, dk, dv, float(eps), int(gate_sigmoid),
+         status_word(proj.device))
+    _count(4)
     return out
 
 
@@ -659,6 +674,37 @@ def attn_prep(proj, qg, kg, cos, sin, rope_idx, kv_slot, q_out, kpool, vpool, *,
     _count()
 
 
+ATTN_SEGS = 16       # sequences of one tcgen05 attention launch
+
+
+def _attn_tc_ok(q, kpool, vpool, hd: int) -> bool:
+    """Dense causal attention over bf16 pages runs on the tcgen05 kernel (TMA pages, TMEM accumulators)."""
+    return (ATTN_TC and hd in (64, 256) and kpool.dtype == torch.bfloat16 and q.is_contiguous() and kpool.is_contiguous()
+            and vpool.is_contiguous())
+
+
+def _attn_tc(q, proj, kpool, vpool, out, segs, nh, nkv, hd):
+    import ctypes
+    table = (ctypes.c_int64 * (4 * len(segs)))(*[v for row0, n, pos0, bt in segs for v in (row0, n, pos0, bt.data_ptr())])
+    call("attn_prefill_tc", q, proj, proj.stride(0) if proj is not None else 0, kpool, vpool, kpool.shape[0], out, out.stride(0),
+         ctypes.c_void_p(ctypes.addressof(table)), len(segs), nh, nkv, hd, status_word(q.device), ATTN_TC_TRACE)
+    _count()
+    return out
+
+
+def attn_prefill_group(q, proj, kpool, vpool, out, segs, *, nh, nkv, hd, kscale=None, vscale=None) -> torch.Tensor:
+    """Causal attention of several sequences whose rows are stacked: ``segs = [(first row, rows, position of the first row,
+    block_table)]``.  One launch for those with enough rows for the tcgen05 kernel, one each for the others."""
+    wide = [s for s in segs if s[1] >= ATTN_TC_MIN_T] if kscale is None and _attn_tc_ok(q, kpool, vpool, hd) else []
+    for i in range(0, len(wide), ATTN_SEGS):
+        _attn_tc(q, proj, kpool, vpool, out, wide[i:i + ATTN_SEGS], nh, nkv, hd)
+    for row0, n, pos0, bt in segs:
+        if not wide or n < ATTN_TC_MIN_T:
+            sl = slice(row0, row0 + n)
+            attn_prefill(q[sl], proj[sl], kpool, vpool, bt, out[sl], q_pos0=pos0, nh=nh, nkv=nkv, hd=hd, kscale=kscale, vscale=vscale)
+    return out
+
+
 def attn_prefill(q, proj, kpool, vpool, block_table, out, *, q_pos0, nh, nkv, hd, causal: bool = True,
                  kv_len: int = 0, keep: torch.Tensor | None = None, ratio: int = 0, kscale=None, vscale=None) -> torch.Tensor:
     """``proj`` supplies the per-head output gate (``None``: no gate). ``causal=False`` attends to the
@@ -666,13 +712,8 @@ def attn_prefill(q, proj, kpool, vpool, block_table, out, *, q_pos0, nh, nkv, hd
     (int32 ``[T, words]`` bit mask over blocks of ``ratio`` tokens) restricts query ``t`` to the kept
     blocks plus the tokens after its last complete block."""
     T = q.shape[0]
-    if (ATTN_TC and causal and keep is None and kscale is None and T >= ATTN_TC_MIN_T and hd in (64, 256)
-            and kpool.dtype == torch.bfloat16 and q.is_contiguous() and kpool.is_contiguous() and vpool.is_contiguous()):
-        # dense causal attention over bf16 pages: the tcgen05 kernel (TMA pages, TMEM accumulators)
-        call("attn_prefill_tc", q, proj, proj.stride(0) if proj is not None else 0, kpool, vpool, kpool.shape[0],
-             block_table, out, out.stride(0), T, q_pos0, nh, nkv, hd, status_word(q.device), ATTN_TC_TRACE)
-        _count()
-        return out
+    if causal and keep is None and kscale is None and T >= ATTN_TC_MIN_T and _attn_tc_ok(q, kpool, vpool, hd):
+        return _attn_tc(q, proj, kpool, vpool, out, [(0, T, q_pos0, block_table)], nh, nkv, hd)
     call("attn_prefill", q, proj, proj.stride(0) if proj is not None else 0, kpool, vpool, block_table, out,
          out.stride(0), T, q_pos0, nh, nkv, hd, int(causal), kv_len, keep,
          keep.stride(0) if keep is not None else 0, ratio, kscale, vscale)

@@ -829,3 +829,51 @@ def test_few_row_products(M, N, Kd):
         assert off(k.gemm_i8_swiglu(q, qs, w8, ws), torch.nn.functional.silu(r8[:, :N]) * r8[:, N:]) < 4e-3
         if M <= 8:
             assert off(k.gemv_i8(w8[:N], ws[:N], Ad, f), r8[:, :N]) < 1e-6
+
+
+@pytest.mark.parametrize("nk,nv,dk,lens", [(16, 32, 128, (1, 64, 65, 130, 300)), (16, 48, 128, (512, 127)), (2, 4, 64, (3, 200, 64))])
+def test_gdn_prefill_of_several_sequences(nk, nv, dk, lens):
+    """One call over stacked sequences against one call each, bit for bit: chunk edges, a slot order of its own, rows before the
+    chunk from the ring, value heads of a key head in one CTA (from 148 (chunk, key head) pairs on) or one each."""
+    k = K()
+    T, n = sum(lens), len(lens)
+    proj, conv_w, A_log, dt_bias, norm_w, conv_dim = _gdn_inputs(T, nk, nv, dk, dk, 77)
+    d = lambda t: t.to(DEV)
+    g = torch.Generator().manual_seed(78)
+    ring = torch.randn(n + 1, k.RING, conv_dim, generator=g).bfloat16().to(DEV)
+    st = (0.1 * torch.randn(n + 1, nv, dk, dk, generator=g)).to(DEV)
+    args = (d(conv_w), d(A_log), d(dt_bias), d(norm_w.float()))
+    kw = dict(nk=nk, nv=nv, dk=dk, dv=dk, eps=1e-6)
+    pj, segs = d(proj), [(m, 5 * i, (i + 2) % (n + 1)) for i, m in enumerate(lens)]
+    r2, s2, want = ring.clone(), st.clone(), torch.empty(T, nv * dk, dtype=torch.bfloat16, device=DEV)
+    scratch = torch.empty(k.gdn_prefill_scratch_floats(T, nk, nv, dk, dk, n), device=DEV)
+    at = 0
+    for m, pos, slot in segs:
+        k.gdn_prefill(pj[at:at + m], *args, r2[slot], s2[slot], scratch, want[at:at + m], pos0=pos, **kw)
+        at += m
+    got = torch.empty_like(want)
+    k.gdn_prefill_group(pj, *args, ring, st, scratch.fill_(float("nan")), got, segs, **kw)
+    assert torch.equal(got, want) and torch.equal(ring, r2) and torch.equal(st, s2)
+
+
+@pytest.mark.parametrize("hd,lens", [(64, (32, 31, 129, 1, 500)), (256, (128, 40, 200))])
+def test_attention_of_several_sequences(hd, lens):
+    """One launch for the sequences of at least 32 rows (query tiles of 128) against one call per sequence, bit for bit."""
+    k = K()
+    nh, nkv, T = 4, 2, sum(lens)
+    g = torch.Generator().manual_seed(5)
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+    before = [70 * i for i in range(len(lens))]
+    pages = [(b + m + 63) // 64 for b, m in zip(before, lens)]
+    order = torch.randperm(sum(pages), generator=g).to(torch.int32).to(DEV)
+    kpool, vpool = rnd(sum(pages) * 64, nkv, hd), rnd(sum(pages) * 64, nkv, hd)
+    q, proj = rnd(T, nh, hd), rnd(T, nh * 2 * hd)
+    segs, at, pg = [], 0, 0
+    want, got = torch.empty(T, nh * hd, dtype=torch.bfloat16, device=DEV), torch.empty(T, nh * hd, dtype=torch.bfloat16, device=DEV)
+    for m, b, p in zip(lens, before, pages):
+        bt = order[pg:pg + p].clone()
+        segs.append((at, m, b, bt))
+        k.attn_prefill(q[at:at + m], proj[at:at + m], kpool, vpool, bt, want[at:at + m], q_pos0=b, nh=nh, nkv=nkv, hd=hd)
+        at, pg = at + m, pg + p
+    k.attn_prefill_group(q, proj, kpool, vpool, got, segs, nh=nh, nkv=nkv, hd=hd)
+    assert torch.equal(got, want)
