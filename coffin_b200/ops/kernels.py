@@ -620,7 +620,7 @@ def gdn_decode(proj, conv_w, A_log, dt_bias, norm_w, ring, state, slots, positio
     assert proj.shape[0] == M * ntok and slots.dtype == torch.int32 and positions.dtype == torch.int32
     call("gdn_decode", proj, proj.stride(0), conv_w, A_log, dt_bias, norm_w, ring, state, slots, positions,
          out, out.stride(0), record, record.shape[1] if record is not None else 0, M, ntok,
-         int(write_state), nk, nv, dk, dv, float(eps), int(gate_sigmoid))
+         int(write_state), nk, nv, dk, dv, float(eps), int(gate_sigmoid), status_word(proj.device))
     _count()
     return out
 

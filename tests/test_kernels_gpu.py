@@ -877,3 +877,32 @@ def test_attention_of_several_sequences(hd, lens):
         at, pg = at + m, pg + p
     k.attn_prefill_group(q, proj, kpool, vpool, got, segs, nh=nh, nkv=nkv, hd=hd)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("nk,nv,M", [(16, 32, 10), (16, 48, 64), (5, 5, 61)])
+def test_gdn_decode_of_many_rows(nk, nv, M):
+    """More (row, head) pairs than two CTAs an SM hold: the streaming kernel against the per-pair one on eight rows at a time.  The
+    norm's sum is taken in another order (fp32, one bf16 rounding) and the compiler contracts other multiplies and adds: a few fp32
+    roundings (2^-24 each) of sums of 128 terms, 1e-5 of the scale.  Padded rows stay untouched."""
+    k = K()
+    dk, n = 128, M + 2
+    proj, conv_w, A_log, dt_bias, norm_w, conv_dim = _gdn_inputs(M, nk, nv, dk, dk, 91)
+    g = torch.Generator().manual_seed(92)
+    ring = torch.randn(n, k.RING, conv_dim, generator=g).bfloat16().to(DEV)
+    st = (0.1 * torch.randn(n, nv, dk, dk, generator=g)).to(DEV)
+    slots = torch.randperm(n, generator=g)[:M].to(torch.int32)
+    slots[3] = slots[M - 1] = -1
+    pos = torch.randint(0, 40, (M,), generator=g, dtype=torch.int32)
+    slots, pos, pj = slots.to(DEV), pos.to(DEV), proj.to(DEV)
+    args = [t.to(DEV) for t in (conv_w, A_log, dt_bias, norm_w.float())]
+    kw = dict(nk=nk, nv=nv, dk=dk, dv=dk, eps=1e-6)
+    r2, s2, want, got = ring.clone(), st.clone(), torch.zeros(M, nv * dk, dtype=torch.bfloat16, device=DEV), torch.zeros(M, nv * dk, dtype=torch.bfloat16, device=DEV)
+    step = max(1, min(8, 290 // nv))
+    for at in range(0, M, step):
+        sl = slice(at, at + step)
+        k.gdn_decode(pj[sl], *args, r2, s2, slots[sl].contiguous(), pos[sl].contiguous(), want[sl], **kw)
+    k.gdn_decode(pj, *args, ring, st, slots, pos, got, **kw)
+    k.check_status()
+    assert torch.equal(ring, r2)
+    close(st, s2, 1e-5)
+    close(got, want, 2 ** -7)
