@@ -7,7 +7,7 @@
 // memory); here the codes travel (TMA, 8 KB per k-block and tile) and are expanded inside the CTA.
 //
 // Roles (6 + NDQ warps, one CTA per SM, persistent over the tile list of cb_moe_dispatch):
-//   warp 0     TMA producer of the [128 x 64] bf16 A tiles (128B swizzle), one per k-block;
+//   warp 0     TMA producer of the [128 x 64] bf16 A tiles (128B swizzle), one per k-block, in boxes of 32 rows;
 //   last warp  TMA producer of the codes, [256 rows x 64 B] per two k-blocks, into a ring of its own that runs
 //              six k-blocks ahead (the codes come from HBM, the activations mostly from L2);
 //   warps 6-   dequant, two groups of NDQ / 2 warps on alternate k-blocks: a thread owns RPT weight rows of the
@@ -30,7 +30,8 @@ namespace {
 using namespace sm100;
 
 constexpr int WM = 128, WN = 256, WAS = 3, WBS = 3, WCS = 3;   // A / expanded-B / code ring depths
-constexpr int NDQ = 8;                           // dequant warps (two groups of NDQ / 2)
+constexpr int NDQ = 16;                          // dequant warps (two groups of NDQ / 2)
+constexpr int WAR = 32;                          // rows of a box of A
 constexpr int RPT = WN / (NDQ * 16);             // weight rows of a tile per dequant thread
 constexpr int kThreadsW4 = (7 + NDQ) * 32;         // the last warp feeds the code ring
 constexpr int kMaxG = 20;          // groups of 128 along K a row may have (K <= 2560)
@@ -127,16 +128,22 @@ gemm_w4_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       uint32_t it = 0;
       // tile = (m-tile, n-tile) with the n-tiles of an m-tile consecutive: the CTAs that run side by side share
       // the activation tile through L2; every weight tile is read once anyway
-      int m0n = 0;
-      if ((int)blockIdx.x < total) m0n = a.g_row0[blockIdx.x / a.n_tiles];
+      // Only the boxes that hold rows of the tile travel: an expert of a 1024-token prompt has 32 of the 128.  The other rows of
+      // the A tile keep what they held; so do the accumulator rows that nobody stores.
+      int m0n = 0, rn = 0;
+      if ((int)blockIdx.x < total) { m0n = a.g_row0[blockIdx.x / a.n_tiles]; rn = a.g_rows[blockIdx.x / a.n_tiles]; }
       for (int tile = blockIdx.x; tile < total && !*abort_flag; tile += gridDim.x) {
-        const int m0 = m0n;
-        if (tile + (int)gridDim.x < total) m0n = a.g_row0[(tile + gridDim.x) / a.n_tiles];     // ahead of its use
+        const int m0 = m0n, boxes = (rn + WAR - 1) / WAR;
+        if (tile + (int)gridDim.x < total) {                                                 // ahead of its use
+          m0n = a.g_row0[(tile + gridDim.x) / a.n_tiles];
+          rn = a.g_rows[(tile + gridDim.x) / a.n_tiles];
+        }
         for (int kb = 0; kb < a.k_blocks; ++kb, ++it) {
           const int s = it % WAS;
           if (!w4_wait(&a_empty[s], ((it / WAS) & 1) ^ 1, abort_flag)) { atomicCAS(a.status, 0, 91); abort_s = 1; break; }
-          mbar_expect_tx(&a_full[s], A_BYTES_W);
-          tma_load_2d(atiles + (size_t)s * A_BYTES_W, &tmA, &a_full[s], kb * 64, m0);
+          mbar_expect_tx(&a_full[s], boxes * WAR * 128);
+          for (int i = 0; i < boxes; ++i)
+            tma_load_2d(atiles + (size_t)s * A_BYTES_W + i * WAR * 128, &tmA, &a_full[s], kb * 64, m0 + i * WAR);
         }
         if (*abort_flag) break;
       }
@@ -191,7 +198,7 @@ gemm_w4_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   } else if (warp >= 6 && warp < 6 + NDQ) {
     // ------------------------------- dequant ----------------------------------------------------------
     // Two groups of four warps take alternate k-blocks, so a group has two k-block times for one tile and
-    // the expansion of k-block n+1 overlaps that of n.  Thread tg of a group owns weight rows tg and tg + 128.
+    // the expansion of k-block n+1 overlaps that of n.  Thread tg of a group owns weight row tg.
     const int grp = (warp - 6) / (NDQ / 2), tg = threadIdx.x - 6 * 32 - grp * (NDQ * 16);
     uint32_t it = 0;
     float4 sreg[RPT][kMaxG / 4];
@@ -254,8 +261,9 @@ gemm_w4_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 #pragma unroll
         for (int h = 0; h < RPT; ++h) {
           const int r = tg + h * (NDQ * 16);
-          const uint4* q = reinterpret_cast<const uint4*>(codes + (size_t)cs * Q_BYTES_W + r * 64 + sub * 32);
-          const uint4 q0 = q[0], q1 = q[1];
+          const uint4* q = reinterpret_cast<const uint4*>(codes + (size_t)cs * Q_BYTES_W + r * 64);
+          const int sw = (r >> 1) & 3;                     // 64-byte swizzle: eight rows of a piece lie in different banks
+          const uint4 q0 = q[(sub * 2) ^ sw], q1 = q[(sub * 2 + 1) ^ sw];
           const bf16 sc = live[h] ? scs[(size_t)(kb >> 1) * WN + h * (NDQ * 16)] : __float2bfloat16(0.f);
           const __nv_bfloat162 s2 = __halves2bfloat162(sc, sc);
           unsigned char* brow = btiles + (size_t)bs * B_BYTES_W + r * 128;
@@ -331,7 +339,7 @@ gemm_w4_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   }
 }
 
-// codes viewed as a 2-D byte tensor [rows, K/2]: box [128 rows, 64 bytes], no swizzle
+// codes viewed as a 2-D byte tensor [rows, K/2]: box [128 rows, 64 bytes]
 int make_code_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t row_bytes) {
   cb_encode_tiled_fn enc = cb_get_encode();
   if (!enc) return CB_ERR_DRIVER;
@@ -341,7 +349,7 @@ int make_code_map(CUtensorMap* map, const void* base, uint64_t rows, uint64_t ro
   cuuint32_t box[2] = {64, 128};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : CB_ERR_DRIVER;
 }
@@ -360,7 +368,7 @@ CB_EXPORT int cb_gemm_w4_grouped(const void* A, int64_t lda, const void* Wq, con
   if (K / 128 > kMaxG || (K / 128) % 4 || K % 256) return CB_ERR_SHAPE;      // the scales of a row travel as float4, the codes four k-blocks at a time
   if (K % 128 || N % 8 || ldc % 8 || (swiglu && Nw % 2) || !status || !g_count || !g_row0 || !g_rows || !g_expert) return CB_ERR_SHAPE;
   CUtensorMap tmA, tmQ;
-  int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)rows, (uint64_t)K, (uint64_t)lda, WM, 64);
+  int rc = cb_make_tmap_2d(&tmA, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, A, (uint64_t)rows, (uint64_t)K, (uint64_t)lda, WAR, 64);
   if (rc) return rc;
   rc = make_code_map(&tmQ, Wq, (uint64_t)(E * Nw), (uint64_t)(K / 2));
   if (rc) return rc;

@@ -362,3 +362,204 @@ CB_EXPORT int cb_w4_dequant(const void* Wq, const void* wscale, void* out, int64
   return (int)cb_launch(w4_dequant_kernel, dim3(grid), dim3(256), 0, (cudaStream_t)stream, (const uint8_t*)Wq,
                         (const float*)wscale, (bf16*)out, N, K);
 }
+
+// ---- routed experts for many slots: every expert's weights are read once ------------------------
+// The slot mode above reads an expert once per slot and quantises the slot's row in every CTA that shares it.  With 64 tokens of
+// eight slots over 256 experts (2.3 slots an expert in use) that is 2.3 passes over the int4 codes and a prologue of three block
+// reductions in front of each: 106 + 64 us a layer for 57 us of codes.  Here the rows are quantised once by a kernel of their own, a
+// CTA takes an expert, collects its slots and multiplies up to eight of them by every 16-row block it reads; codes and scales travel
+// one step ahead in registers.
+namespace {
+
+struct MoeW4Args {
+  const uint8_t* W; const float* wscale;
+  const int8_t* xq; const int* asum; const float* xscale;   // [rows][K] (order of the kernel above), [rows][G], [rows]
+  bf16* y;
+  int N, K, up_off, expert_rows, slots;
+  int64_t ldy;
+  const int* slot_expert; const int* slot_xrow;
+};
+constexpr int kMaxSlots = 1024;
+
+// One row per CTA: absmax scale, int8 values in the kernel's order, sums of the groups of 128.
+__global__ void __launch_bounds__(128) w4_quant_rows_kernel(const bf16* x, int64_t ldx, int8_t* xq, int* asum, float* xscale, int K) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  bf16* row = reinterpret_cast<bf16*>(smem_raw);
+  __shared__ float red[32];
+  griddep_launch();
+  griddep_wait();
+  const int64_t r = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31;
+  float amax = 0.f;
+  for (int c = tid; c < (K >> 3); c += 128) {
+    const uint4 v = *reinterpret_cast<const uint4*>(x + r * ldx + c * 8);
+    *reinterpret_cast<uint4*>(row + c * 8) = v;
+    float f[8];
+    bf16x8_to_float(v, f);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
+  }
+  amax = block_max(amax, red);                               // its barriers also publish the row
+  const float sc = fmaxf(amax, 1e-8f) / 127.f, inv = 1.f / sc;
+  if (tid == 0) xscale[r] = sc;
+  for (int g = tid >> 5; g < K / kGroup; g += 4) {           // a warp per group, four values a lane
+    const int at = g * kGroup + (lane >> 1) * 8 + (lane & 1);                // evens (lane even) or odds of eight channels
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int q = max(-127, min(127, __float2int_rn(__bfloat162float(row[at + 2 * i]) * inv)));
+      w |= (uint32_t)(q & 0xff) << (8 * i);
+    }
+    reinterpret_cast<uint32_t*>(xq + r * K)[g * (kGroup / 4) + lane] = w;
+    int s = __dp4a((int)w, 0x01010101, 0);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) asum[r * (K / kGroup) + g] = s;
+  }
+}
+
+template <bool SWIGLU>
+__global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
+  constexpr int PB = SWIGLU ? 2 : 1, U = SWIGLU ? 2 : 4;      // row blocks of a unit; groups of a step
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int K = a.K, G = K / kGroup, e = blockIdx.y;
+  int8_t* xq = reinterpret_cast<int8_t*>(smem_raw);           // [8][K]
+  int* asum = reinterpret_cast<int*>(smem_raw + (size_t)8 * K);   // [8][G]
+  __shared__ float xscale[8];
+  __shared__ int list[kMaxSlots], cnt_s[kW];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const uint8_t* W = a.W + (int64_t)e * a.expert_rows * (K >> 1);
+  const float* ws = a.wscale + (int64_t)e * a.expert_rows * G;
+  const int nblk = (a.N + 15) / 16, nb = (G + U - 1) / U, bstep = gridDim.x * kW, b0 = blockIdx.x * kW + warp;
+  struct Step { uint4 lo[U][PB], hi[U][PB]; float sl[U][PB], sh[U][PB]; };
+  auto load = [&](Step& s, int blk, int gi) {
+#pragma unroll
+    for (int b = 0; b < PB; ++b) {
+      const int64_t lo = (b ? a.up_off : 0) + min(blk * 16 + g, a.N - 1), hi = (b ? a.up_off : 0) + min(blk * 16 + g + 8, a.N - 1);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool ok = gi + u < G;
+        s.lo[u][b] = ok ? ld_stream(W + lo * (K >> 1) + (gi + u) * 64 + t * 16) : make_uint4(0, 0, 0, 0);
+        s.hi[u][b] = ok ? ld_stream(W + hi * (K >> 1) + (gi + u) * 64 + t * 16) : make_uint4(0, 0, 0, 0);
+        s.sl[u][b] = ok ? __ldg(ws + lo * G + gi + u) : 0.f;
+        s.sh[u][b] = ok ? __ldg(ws + hi * G + gi + u) : 0.f;
+      }
+    }
+  };
+  griddep_launch();
+  Step nxt;
+  if (b0 < nblk) load(nxt, b0, 0);                            // the weights do not depend on the routing
+  griddep_wait();
+  // ---- this expert's slots, in order ----------------------------------------------------------
+  const int per = ((a.slots + kW - 1) / kW + 31) & ~31, s0 = warp * per;
+  int mine = 0;
+  for (int i = s0; i < s0 + per && i < a.slots; i += 32)
+    mine += __popc(__ballot_sync(0xffffffffu, i + lane < a.slots && a.slot_expert[min(i + lane, a.slots - 1)] == e));
+  if (lane == 0) cnt_s[warp] = mine;
+  __syncthreads();
+  int at = 0, count = 0;
+#pragma unroll
+  for (int w = 0; w < kW; ++w) { at += w < warp ? cnt_s[w] : 0; count += cnt_s[w]; }
+  if (count == 0) return;
+  for (int i = s0; i < s0 + per && i < a.slots; i += 32) {
+    const bool on = i + lane < a.slots && a.slot_expert[min(i + lane, a.slots - 1)] == e;
+    const unsigned b = __ballot_sync(0xffffffffu, on);
+    if (on) list[at + __popc(b & ((1u << lane) - 1))] = i + lane;
+    at += __popc(b);
+  }
+  for (int c0 = 0; c0 < count; c0 += 8) {
+    const int M = min(8, count - c0);
+    __syncthreads();                                          // the list is complete; the rows before these are no longer read
+    for (int idx = tid; idx < M * (K >> 4); idx += kT) {
+      const int m = idx / (K >> 4), c = idx % (K >> 4), slot = list[c0 + m];
+      const int64_t r = a.slot_xrow ? a.slot_xrow[slot] : slot;
+      reinterpret_cast<uint4*>(xq + (size_t)m * K)[c] = reinterpret_cast<const uint4*>(a.xq + r * K)[c];
+    }
+    for (int idx = tid; idx < M * G; idx += kT) {
+      const int slot = list[c0 + idx / G];
+      const int64_t r = a.slot_xrow ? a.slot_xrow[slot] : slot;
+      asum[idx] = a.asum[r * G + idx % G];
+      if (idx % G == 0) xscale[idx / G] = a.xscale[r];
+    }
+    __syncthreads();
+    const int m0 = 2 * t, m1 = 2 * t + 1;
+    for (int blk = b0; blk < nblk; blk += bstep) {
+      float acc[PB][4] = {};
+      for (int i = 0; i < nb; ++i) {
+        const Step cur = nxt;
+        const int gi = i * U;
+        if (i + 1 < nb) load(nxt, blk, gi + U);
+        else if (blk + bstep < nblk) load(nxt, blk + bstep, 0);
+        else if (c0 + 8 < count) load(nxt, b0, 0);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (gi + u >= G) break;
+          uint4 x0 = make_uint4(0, 0, 0, 0), x1 = x0;
+          if (g < M) {
+            const uint4* xp = reinterpret_cast<const uint4*>(xq + (size_t)g * K + (gi + u) * kGroup + t * 32);
+            x0 = xp[0];
+            x1 = xp[1];
+          }
+          const int a0 = m0 < M ? asum[m0 * G + gi + u] : 0, a1 = m1 < M ? asum[m1 * G + gi + u] : 0;
+          const uint32_t xb[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+          for (int b = 0; b < PB; ++b) {
+            int d[4] = {0, 0, 0, 0};
+            const uint32_t wl[4] = {cur.lo[u][b].x, cur.lo[u][b].y, cur.lo[u][b].z, cur.lo[u][b].w};
+            const uint32_t wh[4] = {cur.hi[u][b].x, cur.hi[u][b].y, cur.hi[u][b].z, cur.hi[u][b].w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              mma_u8s8(d, wl[k] & 0x0F0F0F0Fu, wh[k] & 0x0F0F0F0Fu, (wl[k] >> 4) & 0x0F0F0F0Fu, (wh[k] >> 4) & 0x0F0F0F0Fu, xb[2 * k], xb[2 * k + 1]);
+            acc[b][0] = fmaf((float)(d[0] - 8 * a0), cur.sl[u][b], acc[b][0]);
+            acc[b][1] = fmaf((float)(d[1] - 8 * a1), cur.sl[u][b], acc[b][1]);
+            acc[b][2] = fmaf((float)(d[2] - 8 * a0), cur.sh[u][b], acc[b][2]);
+            acc[b][3] = fmaf((float)(d[3] - 8 * a1), cur.sh[u][b], acc[b][3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int m = (q & 1) ? m1 : m0, row = blk * 16 + g + ((q & 2) ? 8 : 0);
+        if (m < M && row < a.N) {
+          float v = acc[0][q] * xscale[m];
+          if (SWIGLU) v = silu_f(v) * (acc[PB - 1][q] * xscale[m]);
+          a.y[(int64_t)list[c0 + m] * a.ldy + row] = __float2bfloat16(v);
+        }
+      }
+    }
+  }
+}
+
+template <bool SWIGLU>
+int launch_moe_w4(const MoeW4Args& a, int E, cudaStream_t st) {
+  const size_t smem = (size_t)8 * a.K + (size_t)8 * (a.K / kGroup) * 4;
+  auto kern = moe_w4_kernel<SWIGLU>;
+  if (smem + 8192 > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  // a warp walks at least four 16-row blocks of its expert where there are that many, so that a step is always in flight
+  const int nblk = (a.N + 15) / 16;
+  const unsigned gx = (unsigned)((nblk + 4 * kW - 1) / (4 * kW));
+  const int64_t carve = std::min<int64_t>(100, (2 * (int64_t)(smem + 8192) * 100 + 228 * 1024 - 1) / (228 * 1024));
+  return (int)cb_launch_carve((int)carve, kern, dim3(gx, (unsigned)E), dim3(kT), smem, st, a);
+}
+}  // namespace
+
+// Rows of x [R, K] as int8 in the order of the kernels above, with the sums of their groups and one scale each.
+CB_EXPORT int cb_w4_quant_rows(const void* x, int64_t ldx, void* xq, void* asum, void* xscale, int64_t R, int64_t K, void* stream) {
+  if (R < 1 || K < kGroup || K % kGroup || K > 16384 || ldx % 8 || ((uintptr_t)x & 15) || !xq || !asum || !xscale) return CB_ERR_SHAPE;
+  return (int)cb_launch(w4_quant_rows_kernel, dim3((unsigned)R), dim3(128), (size_t)K * 2, (cudaStream_t)stream, (const bf16*)x, ldx,
+                        (int8_t*)xq, (int*)asum, (float*)xscale, (int)K);
+}
+
+// As cb_moe_gemv_w4, from quantised rows, bf16 results: y[s, :] = dequant(Wq[slot_expert[s]]) x[slot_xrow[s], :].
+CB_EXPORT int cb_moe_gemv_w4_grouped(const void* Wq, const void* wscale, const void* xq, const void* asum, const void* xscale, void* y,
+                                     int64_t n_slots, int64_t E, int64_t N, int64_t K, int64_t ldy, int64_t swiglu, const void* slot_expert,
+                                     const void* slot_xrow, void* stream) {
+  if (!Wq || !wscale || !xq || !asum || !xscale || !y || !slot_expert) return CB_ERR_ARG;
+  if (K < kGroup || K % kGroup || K > 16384 || N < 1 || E < 1 || E > 65535 || n_slots < 1 || n_slots > kMaxSlots) return CB_ERR_SHAPE;
+  MoeW4Args a{(const uint8_t*)Wq, (const float*)wscale, (const int8_t*)xq, (const int*)asum, (const float*)xscale, (bf16*)y, (int)N, (int)K,
+              (int)N, (int)(swiglu ? 2 * N : N), (int)n_slots, ldy, (const int*)slot_expert, (const int*)slot_xrow};
+  return swiglu ? launch_moe_w4<true>(a, (int)E, (cudaStream_t)stream) : launch_moe_w4<false>(a, (int)E, (cudaStream_t)stream);
+}

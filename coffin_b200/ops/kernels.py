@@ -375,12 +375,25 @@ def gemv_w4(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
     return out
 
 
+# Slots per expert from which the routed int4 products take an expert at a time instead of a slot at a time.  256 experts, 8 layers:
+# 128 slots 1354 us by expert, 1168 us by slot; 256 slots 1575 / 1629 us; 512 slots 1905 / 2538 us.
+W4_GROUP_SHARE = 0.75
+
+
 def moe_gemv_w4(Wq, wscale, x, out, slot_expert, slot_xrow, *, swiglu: bool = False) -> torch.Tensor:
     """Routed experts on W4A8 storage: ``Wq [E, rows, K/2]``, ``wscale [E, rows, K/128]``; slot ``s``
     multiplies activation row ``slot_xrow[s]`` by expert ``slot_expert[s]`` (``< 0``: skipped)."""
     n_slots = out.shape[0]
     K = Wq.shape[2] * 2
     N = Wq.shape[1] // 2 if swiglu else Wq.shape[1]
+    if W4_GROUP_SHARE * Wq.shape[0] <= n_slots <= 1024 and out.dtype == torch.bfloat16 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0 and K <= 16384:
+        R, dev = x.shape[0], x.device
+        xq, asum = torch.empty(R, K, dtype=torch.int8, device=dev), torch.empty(R, K // 128, dtype=torch.int32, device=dev)
+        xs = torch.empty(R, dtype=torch.float32, device=dev)
+        call("w4_quant_rows", x, x.stride(0), xq, asum, xs, R, K)
+        call("moe_gemv_w4_grouped", Wq, wscale, xq, asum, xs, out, n_slots, Wq.shape[0], N, K, out.stride(0), int(swiglu), slot_expert, slot_xrow)
+        _count(2)
+        return out
     mode = (1 if swiglu else 0) | (2 if out.dtype == torch.float32 else 0)
     call("moe_gemv_w4", Wq, wscale, x, out, n_slots, N, K, out.stride(0), mode, slot_expert, slot_xrow)
     _count()

@@ -906,3 +906,25 @@ def test_gdn_decode_of_many_rows(nk, nv, M):
     assert torch.equal(ring, r2)
     close(st, s2, 1e-5)
     close(got, want, 2 ** -7)
+
+
+@pytest.mark.parametrize("E,N,Kd,swiglu,slots", [(6, 128, 256, True, 97), (5, 520, 2304, False, 200), (300, 24, 128, True, 512), (3, 2048, 512, False, 1024)])
+def test_moe_gemv_w4a8_by_expert(E, N, Kd, swiglu, slots, monkeypatch):
+    """Experts taken whole (several passes of eight slots, experts without a slot, slots of other ranks, row and K remainders) against
+    the slot-wise kernel: the same integers and scales, fp32 sums of at most 18 groups in another order, one bf16 rounding."""
+    k = K()
+    from coffin_b200.weights.quant import W4A8Weight
+    g = torch.Generator().manual_seed(70)
+    W = torch.randn(E, 2 * N if swiglu else N, Kd, generator=g) * 0.05
+    wq, sc = (t.to(DEV) for t in W4A8Weight.quantize(W).to_nk())
+    x = torch.randn(slots, Kd, generator=g).bfloat16().to(DEV)
+    slot_e = torch.randint(-1, max(1, E * 2 // 3), (slots,), generator=g, dtype=torch.int32).to(DEV)
+    slot_x = torch.randint(0, slots, (slots,), generator=g, dtype=torch.int32).to(DEV)
+    for rows in (slot_x, None):
+        want, got = (torch.full((slots, N), 3.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        monkeypatch.setattr(k, "W4_GROUP_SHARE", 1 << 20)
+        k.moe_gemv_w4(wq, sc, x, want, slot_e, rows, swiglu=swiglu)
+        monkeypatch.setattr(k, "W4_GROUP_SHARE", 0)
+        k.moe_gemv_w4(wq, sc, x, got, slot_e, rows, swiglu=swiglu)
+        assert bool((got[slot_e < 0] == 3.0).all())
+        close(got, want, 2 ** -7)
