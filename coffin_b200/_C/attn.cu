@@ -13,7 +13,7 @@
 // (models/qwen35/full_attn.py:658-789); rope, kv_quant and kv_pool_store are separate launches
 // there (attn.cu:132,249,1200).  The pool here is [slots, nkv, hd] per layer, addressed through
 // a per-row block table (block = 64 tokens).
-#include "common.cuh"
+#include "sm100.cuh"
 
 namespace {
 
@@ -386,6 +386,7 @@ struct DecodeArgs {
   // `ratio` tokens plus the tokens after its last complete block (nsel[m] < 0: every visible token)
   const bf16* q_in; const int* sel; const int* nsel; int topk, ratio;
   float* kscale; float* vscale;       // int8 pools: [slots, nkv] scales (null: bf16 pools)
+  int* status;                        // set when a bounded wait ran out (batch kernel)
 };
 
 constexpr int kDecWarps = 8;          // warps per decode CTA; each takes 4 keys per iteration
@@ -714,33 +715,147 @@ __global__ void __launch_bounds__(kDecWarps * 32, MINB) attn_decode_kernel(const
 // bound when every row brings its own CTAs.  Here one CTA serves one (row, kv head): the REP query
 // heads of the kv head are rows 0..REP-1 of a 16-row mma tile (the rest zero), the four warps take 16
 // keys each of every 64-key tile (S = Q K^T and O += P V as bf16 mma.m16n8k16 from ldmatrix
-// fragments, tiles staged with cp.async), keep their own running maximum and sum, and merge once at
-// the end.  Query / key normalisation, rotary embedding, the KV append of the current token and the
+// fragments, K and V tiles in turn by TMA through a ring of three, so that two are on their way while
+// one is used), keep their own running maximum and sum, and merge once at the end.  Two CTAs an SM
+// share the tiles of all rows evenly, whatever the rows' lengths: with equal splits a row, the SMs
+// with the long rows set the time (8 rows of 517 to 16391 tokens 97 -> 61 us, 64 of 1031 to 2047 98 -> 90 us).  Query / key normalisation, rotary embedding, the KV append of the current token and the
 // sigmoid output gate are part of the kernel as in the single-sequence one.
+constexpr int kBatchRows = 128;     // more would cost the second CTA an SM its shared memory
 template <int HD>
-__global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeArgs a) {
+__global__ void __launch_bounds__(128, 2)
+attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeArgs a, int rows) {
   constexpr int LD = HD + 8, EPL = HD / 32, CPR = HD / 8;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  bf16* Qs = reinterpret_cast<bf16*>(smem_raw);   // [16][LD]
-  bf16* Ks = Qs + 16 * LD;                        // [64][LD]
-  bf16* Vs = Ks + 64 * LD;                        // [64][LD]
-  bf16* kcur = Vs + 64 * LD;                      // [HD] this token's key (normed, rotated)
+  constexpr int TILE = 64 * HD;                   // elements of a K or V tile: HD / 64 blocks of [64 rows x 128 B], 128-byte swizzle
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  bf16* ring = reinterpret_cast<bf16*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);   // [3][TILE]: K and V tiles in turn
+  bf16* Qs = ring + 3 * TILE;                     // [16][LD]
+  bf16* kcur = Qs + 16 * LD;                      // [HD] this token's key (normed, rotated)
   bf16* vcur = kcur + HD;                         // [HD]
-  float* mo = reinterpret_cast<float*>(Ks);       // after the loop: [4 warps][8 rows][HD] partial outputs
+  float* mo = reinterpret_cast<float*>(ring);     // after the loop: [4 warps][8 rows][HD] partial outputs
+  float (*sc_s)[64] = reinterpret_cast<float (*)[64]>(mo + 4 * 8 * HD);     // merge of the runs: [8][64] each
+  float (*l_s)[64] = sc_s + 8;
+  // 16-byte piece c of row r of a tile
+  auto piece = [](int r, int c) { return (c >> 3) * 64 * 64 + r * 64 + (((c & 7) ^ (r & 7)) << 3); };
   __shared__ float mm_s[4][8], ml_s[4][8];
-  __shared__ float sc_s[8][64], l_s[8][64], linv_s[8];
+  __shared__ float linv_s[8];
   __shared__ bool is_last;
-  const int kvh = blockIdx.x, m = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z, rep = a.nh / a.nkv;
+  __shared__ int pre_s[kBatchRows + 1], per_s;
+  __shared__ uint64_t full[3];
+  const int rep = a.nh / a.nkv;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
+  if (tid == 0) {
+    for (int i = 0; i < 3; ++i) sm100::mbar_init(&full[i], 1);
+    sm100::mbar_fence_init();
+  }
   griddep_launch();
   griddep_wait();
-  const int pos = a.positions[m];
-  if (pos < 0) return;                            // padded row
+  // The tiles of all (row, kv head) pairs are shared out in runs of about `per` tiles.  Up to half as many pairs as CTAs: every pair is
+  // cut into runs of its own (a CTA pays one prologue and one merge, about 15 us with what surrounds them).  More: the (row, kv head,
+  // tile) triples in order are cut evenly, runs cross pairs.  A pair's partials have room for a.nsplit runs; with room for one a CTA
+  // takes whole pairs.
+  const int pairs = rows * a.nkv, ctas = gridDim.x;
+  const bool whole = a.nsplit == 1, own = !whole && 2 * pairs <= ctas;
+  if (warp == 0) {
+    int sum = 0, most = 0, per = 1;
+    for (int m0 = 0; m0 < rows; m0 += 32) {
+      const int n = m0 + lane < rows ? a.positions[m0 + lane] : -1, nt = n < 0 ? 0 : n / kBlock + 1;       // a padded row has none
+      sum += nt;
+      most = max(most, nt);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+    }
+    sum *= a.nkv;
+    if (own) per = max((sum + ctas - pairs - 1) / (ctas - pairs), (most + a.nsplit - 1) / a.nsplit);
+    else if (!whole) per = max((sum + ctas - 1) / ctas, (most + a.nsplit - 2) / (a.nsplit - 1));
+    int before = 0;                               // pre_s: runs (own) or tiles of the rows before a row
+    for (int m0 = 0; m0 < rows; m0 += 32) {
+      int n = m0 + lane < rows ? a.positions[m0 + lane] : -1;
+      n = n < 0 ? 0 : n / kBlock + 1;
+      if (own) n = (n + per - 1) / per;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, n, o);
+        if (lane >= o) n += y;
+      }
+      if (m0 + lane < rows) pre_s[m0 + lane + 1] = before + n;
+      before += __shfl_sync(0xffffffffu, n, 31);
+    }
+    if (lane == 0) { pre_s[0] = 0; per_s = per; }
+  }
+  __syncthreads();
+  const int total = pre_s[rows] * a.nkv, per = per_s;
+  int u = whole || own ? blockIdx.x : blockIdx.x * per;
+  const int end = whole ? pairs : (own ? min(total, u + 1) : min(total, u + per));
+  uint32_t seq = 0;                               // halves requested by the runs before: ring position and phase go on
+  while (u < end) {
+  int m, kvh, t0, cnt, nsplit, split;
+  if (whole) {
+    m = u / a.nkv;
+    kvh = u % a.nkv;
+    u += ctas;
+    t0 = split = 0;
+    nsplit = 1;
+    cnt = pre_s[m + 1] - pre_s[m];
+    if (cnt == 0) continue;
+  } else {
+    int lo = 0, hi = rows;                        // the row of this run or triple: the last with pre[m] * nkv <= u
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (pre_s[mid] * a.nkv <= u) lo = mid; else hi = mid;
+    }
+    m = lo;
+    const int n = pre_s[m + 1] - pre_s[m], at = u - pre_s[m] * a.nkv;
+    kvh = at / n;
+    if (own) {
+      const int nt = a.positions[m] / kBlock + 1;
+      nsplit = n;
+      split = at % n;
+      t0 = nt * split / n;
+      cnt = nt * (split + 1) / n - t0;
+      ++u;
+    } else {
+      t0 = at % n;
+      cnt = min(n - t0, end - u);
+      const int first = (u - t0) / per;
+      nsplit = (u - t0 + n - 1) / per - first + 1;
+      split = blockIdx.x - first;
+      u += cnt;
+    }
+  }
+  const int pos = a.positions[m], ntiles = pos / kBlock + 1;
   const bf16* prow = a.proj + (int64_t)m * a.ldp;
   const int rp = a.rope_pos[m];
   const float* cs = a.cos + (int64_t)rp * a.rot;
   const float* sn = a.sin + (int64_t)rp * a.rot;
   const int* bt = a.block_table + (int64_t)m * a.ldbt;
+  // half h of this run: the K (even) or V (odd) tile of its tile h / 2.  One thread asks for a bf16 tile (16 cp.async a thread, or a
+  // bulk copy a row, took longer than the products), int8 rows are converted on the way.
+  auto load_half = [&](int h) {
+    if (h >= 2 * cnt) return;
+    const int64_t slot0 = (int64_t)bt[t0 + (h >> 1)] * kBlock;
+    const uint32_t at = (seq + h) % 3;
+    bf16* dst = ring + at * TILE;
+    if (a.kscale) {
+      const int8_t* pool = reinterpret_cast<const int8_t*>((h & 1) ? a.vpool : a.kpool);
+      const float* scale = (h & 1) ? a.vscale : a.kscale;
+      for (int idx = tid; idx < 64 * CPR; idx += 128) {
+        const int r = idx / CPR, c = idx % CPR;
+        const int64_t row = (slot0 + r) * a.nkv + kvh;
+        *reinterpret_cast<uint4*>(dst + piece(r, c)) = q8x8_to_bf16x8(*reinterpret_cast<const uint2*>(pool + row * HD + c * 8), scale[row]);
+      }
+    } else if (tid == 0) {
+      sm100::mbar_expect_tx(&full[at], TILE * 2);
+#pragma unroll
+      for (int c = 0; c < HD / 64; ++c)
+        sm100::tma_load_2d(dst + c * 64 * 64, (h & 1) ? &tmV : &tmK, &full[at], kvh * HD + c * 64, (int)slot0);
+    }
+  };
+  auto arrived = [&](int h) { return a.kscale || sm100::mbar_wait(&full[(seq + h) % 3], ((seq + h) / 3) & 1); };
+  load_half(0);
+  load_half(1);
   // ---- prologue: q heads -> Qs (bf16), this token's K / V -> pool and shared copies ---------------
   for (int idx = tid; idx < 16 * CPR; idx += 128)
     *reinterpret_cast<uint4*>(Qs + (idx / CPR) * LD + (idx % CPR) * 8) = make_uint4(0, 0, 0, 0);
@@ -754,7 +869,7 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
       norm_rope_lane<HD>(x, a.qg, cs, sn, a.rot, a.eps, lane);
 #pragma unroll
       for (int e = 0; e < EPL; ++e) Qs[r * LD + lane * EPL + e] = __float2bfloat16(x[e]);
-    } else if ((pos / kBlock) % nsplit == split) {   // the split that owns the last tile appends this token
+    } else if (t0 + cnt == ntiles) {             // the run that holds the last tile appends this token
       const int64_t slot = (int64_t)bt[pos / kBlock] * kBlock + pos % kBlock;
       if (r == rep) {
         const bf16* src = prow + (int64_t)a.nh * 2 * HD + (int64_t)kvh * HD + lane * EPL;
@@ -792,34 +907,40 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
 #pragma unroll
   for (int n = 0; n < HD / 8; ++n) o[n][0] = o[n][1] = 0.f;
   float mrow = -INFINITY, lrow = 0.f;
-  const int ntiles = pos / kBlock + 1;
-  __syncthreads();                                // prologue stores visible (a split may have no tile at all)
-  for (int kt = split; kt < ntiles; kt += nsplit) {
-    __syncthreads();                              // previous tile consumed
-    const int64_t slot0 = (int64_t)bt[kt] * kBlock;
-    load_kv_tile<HD, 128>(Ks, Vs, LD, a.kpool, a.vpool, a.kscale, a.vscale, slot0, a.nkv, kvh, tid);
+  // the current token's row comes from this CTA, not from memory
+  auto patch = [&](bf16* tile, const bf16* cur) {
+    for (int c = tid; c < CPR; c += 128)
+      *reinterpret_cast<uint4*>(tile + piece(pos % kBlock, c)) = *reinterpret_cast<const uint4*>(cur + c * 8);
+    sm100::fence_async_smem();
     __syncthreads();
-    if (kt == ntiles - 1) {                       // the current token's row comes from this CTA, not from memory
-      for (int c = tid; c < 2 * CPR; c += 128) {
-        const bool isv = c >= CPR;
-        const int cc = isv ? c - CPR : c;
-        *reinterpret_cast<uint4*>((isv ? Vs : Ks) + (pos % kBlock) * LD + cc * 8) =
-            *reinterpret_cast<const uint4*>((isv ? vcur : kcur) + cc * 8);
-      }
-      __syncthreads();
-    }
-    // ---- S = Q K^T for this warp's 16 keys ---------------------------------------------------
-    float sc[2][4];
+  };
+  __syncthreads();                                // the query tile is complete
+  uint32_t qf[HD / 16][4];
 #pragma unroll
-    for (int n = 0; n < 2; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.f;
-#pragma unroll 4
+  for (int kk = 0; kk < HD / 16; ++kk)
+    ldsm_x4(qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], Qs + (lane & 15) * LD + kk * 16 + (lane >> 4) * 8);
+  bool ok = true;
+  for (int i = 0; i < cnt; ++i) {
+    const int kt = t0 + i;
+    bf16* Ks = ring + ((seq + 2 * i) % 3) * TILE;
+    bf16* Vs = ring + ((seq + 2 * i + 1) % 3) * TILE;
+    if (!(ok = arrived(2 * i))) break;
+    __syncthreads();                              // K is here; the V tile before it is consumed
+    load_half(2 * i + 2);
+    if (kt == ntiles - 1) patch(Ks, kcur);
+    // ---- S = Q K^T for this warp's 16 keys, two chains ------------------------------------------
+    float sc[2][4], s2[2][4];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = s2[n][0] = s2[n][1] = s2[n][2] = s2[n][3] = 0.f;
+#pragma unroll
     for (int kk = 0; kk < HD / 16; ++kk) {
-      uint32_t af[4], b0, b1, b2, b3;
-      ldsm_x4(af[0], af[1], af[2], af[3], Qs + (lane & 15) * LD + kk * 16 + (lane >> 4) * 8);
-      ldsm_x4(b0, b1, b2, b3, Ks + (warp * 16 + (lane & 7) + ((lane >> 4) << 3)) * LD + kk * 16 + ((lane >> 3) & 1) * 8);
-      mma_bf16(sc[0], af, b0, b1);
-      mma_bf16(sc[1], af, b2, b3);
+      uint32_t b0, b1, b2, b3;
+      ldsm_x4(b0, b1, b2, b3, Ks + piece(warp * 16 + (lane & 7) + ((lane >> 4) << 3), kk * 2 + ((lane >> 3) & 1)));
+      mma_bf16(kk & 1 ? s2[0] : sc[0], qf[kk], b0, b1);
+      mma_bf16(kk & 1 ? s2[1] : sc[1], qf[kk], b2, b3);
     }
+#pragma unroll
+    for (int n = 0; n < 2; ++n) { sc[n][0] += s2[n][0]; sc[n][1] += s2[n][1]; }
     // ---- mask + online softmax (base 2), row g of the tile --------------------------------------
     float mnew = mrow;
 #pragma unroll
@@ -846,11 +967,15 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
     pf[3] = 0u;
 #pragma unroll
     for (int n = 0; n < HD / 8; ++n) { o[n][0] *= corr; o[n][1] *= corr; }
+    if (!(ok = arrived(2 * i + 1))) break;
+    __syncthreads();                              // V is here, K is consumed
+    load_half(2 * i + 3);
+    if (kt == ntiles - 1) patch(Vs, vcur);
     // ---- O += P V for the same 16 keys -------------------------------------------------------------
 #pragma unroll
     for (int np = 0; np < HD / 16; ++np) {
       uint32_t b0, b1, b2, b3;
-      ldsm_x4_t(b0, b1, b2, b3, Vs + (warp * 16 + (lane & 15)) * LD + np * 16 + (lane >> 4) * 8);
+      ldsm_x4_t(b0, b1, b2, b3, Vs + piece(warp * 16 + (lane & 15), np * 2 + (lane >> 4)));
       float c0[4] = {o[2 * np][0], o[2 * np][1], 0.f, 0.f}, c1[4] = {o[2 * np + 1][0], o[2 * np + 1][1], 0.f, 0.f};
       mma_bf16(c0, pf, b0, b1);
       mma_bf16(c1, pf, b2, b3);
@@ -861,7 +986,13 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
   // ---- merge the four warps, normalise, gate, store -----------------------------------------------------
   lrow += __shfl_xor_sync(0xffffffffu, lrow, 1);
   lrow += __shfl_xor_sync(0xffffffffu, lrow, 2);
-  __syncthreads();                                // all warps are done with Ks / Vs
+  if (!ok) {                                      // a copy that never came: every thread's wait for it ran out
+    if (lane == 0) atomicExch(a.status, 87);
+    for (int i = 0; i < 2000; ++i) __nanosleep(1000);
+    return;
+  }
+  seq += 2 * cnt;
+  __syncthreads();                                // all warps are done with the tiles
   if (tq == 0) { mm_s[warp][g] = mrow; ml_s[warp][g] = lrow; }
 #pragma unroll
   for (int n = 0; n < HD / 8; ++n)
@@ -883,9 +1014,9 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
     }
     const int h = kvh * rep + r;
     if (nsplit > 1) {                             // unnormalised partial of this split
-      *reinterpret_cast<float4*>(a.part_o + (((int64_t)m * a.nh + h) * nsplit + split) * HD + d) = acc;
+      *reinterpret_cast<float4*>(a.part_o + (((int64_t)m * a.nh + h) * a.nsplit + split) * HD + d) = acc;
       if (d == 0) {
-        float* pml = a.part_ml + (((int64_t)m * a.nh + h) * nsplit + split) * 2;
+        float* pml = a.part_ml + (((int64_t)m * a.nh + h) * a.nsplit + split) * 2;
         pml[0] = M4;
         pml[1] = L;
       }
@@ -899,7 +1030,9 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
     dst[2] = __float2bfloat16(acc.z * li * sigmoid_f(__bfloat162float(gp[2])));
     dst[3] = __float2bfloat16(acc.w * li * sigmoid_f(__bfloat162float(gp[3])));
   }
-  if (nsplit == 1) return;
+  sm100::fence_async_smem();                      // the ring takes copies again
+  __syncthreads();                                // the partial outputs are read
+  if (nsplit == 1) continue;
   // ---- several splits per (row, kv head): the last one to arrive merges all partials and applies the gate ----
   __threadfence();
   __syncthreads();
@@ -909,13 +1042,14 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
     if (is_last) *tk = 0;
   }
   __syncthreads();
-  if (!is_last) return;
+  if (!is_last) continue;
   __threadfence();
-  const float* bo = a.part_o + ((int64_t)m * a.nh + kvh * rep) * nsplit * HD;
-  const float* bml = a.part_ml + ((int64_t)m * a.nh + kvh * rep) * nsplit * 2;
+  const float* bo = a.part_o + ((int64_t)m * a.nh + kvh * rep) * a.nsplit * HD;
+  const float* bml = a.part_ml + ((int64_t)m * a.nh + kvh * rep) * a.nsplit * 2;
   for (int i = tid; i < rep * nsplit; i += 128) {
-    sc_s[i / nsplit][i % nsplit] = __ldcg(bml + (int64_t)i * 2);
-    l_s[i / nsplit][i % nsplit] = __ldcg(bml + (int64_t)i * 2 + 1);
+    const int64_t at = ((int64_t)(i / nsplit) * a.nsplit + i % nsplit) * 2;
+    sc_s[i / nsplit][i % nsplit] = __ldcg(bml + at);
+    l_s[i / nsplit][i % nsplit] = __ldcg(bml + at + 1);
   }
   __syncthreads();
   for (int r = warp; r < rep; r += 4) {           // one warp per head: max, scales, 1 / l
@@ -934,8 +1068,9 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
   __syncthreads();
   for (int idx = tid; idx < rep * (HD / 4); idx += 128) {
     const int r = idx / (HD / 4), d = (idx % (HD / 4)) * 4;
-    const float* src = bo + (int64_t)r * nsplit * HD + d;
+    const float* src = bo + (int64_t)r * a.nsplit * HD + d;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
     for (int sp = 0; sp < nsplit; ++sp) {
       const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (int64_t)sp * HD));
       const float c = sc_s[r][sp];
@@ -949,6 +1084,9 @@ __global__ void __launch_bounds__(128, 2) attn_decode_batch_kernel(const DecodeA
     dst[1] = __float2bfloat16(acc.y * li * sigmoid_f(__bfloat162float(gp[1])));
     dst[2] = __float2bfloat16(acc.z * li * sigmoid_f(__bfloat162float(gp[2])));
     dst[3] = __float2bfloat16(acc.w * li * sigmoid_f(__bfloat162float(gp[3])));
+  }
+  sm100::fence_async_smem();
+  __syncthreads();                                // the merge's scales are read
   }
 }
 
@@ -1039,26 +1177,32 @@ CB_EXPORT int cb_attn_prefill(const void* q, const void* gate, int64_t ldg, cons
 
 CB_EXPORT int cb_attn_decode(const void* proj, int64_t ldp, const void* qg, const void* kg, const void* cos,
                              const void* sin, const void* positions, const void* rope_pos,
-                             const void* block_table, int64_t ldbt, void* kpool, void* vpool, void* part_o,
+                             const void* block_table, int64_t ldbt, void* kpool, void* vpool, int64_t slots, void* part_o,
                              void* part_ml, void* tickets, void* out, int64_t ldo, int64_t M, int64_t nh, int64_t nkv,
                              int64_t hd, int64_t rot, int64_t nsplit, float eps, void* kscale, void* vscale,
-                             void* stream) {
+                             void* status, void* stream) {
   if (M == 0) return 0;
-  if (nh % nkv || nsplit < 1 || nsplit > 64 || !tickets) return CB_ERR_SHAPE;
+  if (nh % nkv || nsplit < 1 || nsplit > 64 || !tickets || !status) return CB_ERR_SHAPE;
   if ((kscale == nullptr) != (vscale == nullptr)) return CB_ERR_ARG;
   DecodeArgs a{(const bf16*)proj, ldp, (const float*)qg, (const float*)kg, (const float*)cos, (const float*)sin,
                (const int*)positions, (const int*)rope_pos, (const int*)block_table, ldbt, (bf16*)kpool,
                (bf16*)vpool, (float*)part_o, (float*)part_ml, (int)nh, (int)nkv, (int)rot, (int)nsplit,
                1.4426950408889634f / sqrtf((float)hd), eps, (unsigned*)tickets, (bf16*)out, ldo,
-               nullptr, nullptr, nullptr, 0, 1, (float*)kscale, (float*)vscale};
-  if (hd == 256 && (rot / 2) % 8 == 0 && nh / nkv <= 8 && g_attn_batch_ctas > 0 && nkv * M >= g_attn_batch_ctas) {
-    // enough (row, kv head) pairs to fill the machine with one CTA each: tensor-core batch kernel
+               nullptr, nullptr, nullptr, 0, 1, (float*)kscale, (float*)vscale, (int*)status};
+  if (hd == 256 && (rot / 2) % 8 == 0 && nh / nkv <= 8 && g_attn_batch_ctas > 0 && nkv * M >= g_attn_batch_ctas && M <= kBatchRows &&
+      (((uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0) {
+    // enough (row, kv head) pairs for the tensor-core batch kernel
     constexpr int HD = 256;
-    const size_t smem = (size_t)(16 + 64 + 64) * (HD + 8) * sizeof(bf16) + 2 * HD * sizeof(bf16);
+    const size_t smem = (size_t)(3 * 64 * HD + 16 * (HD + 8) + 2 * HD) * sizeof(bf16) + 1024;      // two CTAs an SM
+    CUtensorMap tmK = {}, tmV = {};
+    if (!kscale) {
+      int rc = cb_make_tmap_2d(&tmK, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, kpool, (uint64_t)slots, (uint64_t)(nkv * hd), (uint64_t)(nkv * hd), kBlock, 64);
+      if (!rc) rc = cb_make_tmap_2d(&tmV, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vpool, (uint64_t)slots, (uint64_t)(nkv * hd), (uint64_t)(nkv * hd), kBlock, 64);
+      if (rc) return rc;
+    }
     cudaError_t e = cudaFuncSetAttribute(attn_decode_batch_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)cb_launch(attn_decode_batch_kernel<HD>, dim3((unsigned)nkv, (unsigned)M, (unsigned)nsplit), dim3(128), smem,
-                          (cudaStream_t)stream, a);
+    return (int)cb_launch(attn_decode_batch_kernel<HD>, dim3(296), dim3(128), smem, (cudaStream_t)stream, tmK, tmV, a, (int)M);
   }
   return decode_dispatch(a, M, nh, nkv, hd, rot, stream);
 }
@@ -1078,6 +1222,6 @@ CB_EXPORT int cb_attn_sparse(const void* q, const void* proj, int64_t ldp, const
   DecodeArgs a{(const bf16*)proj, ldp, nullptr, nullptr, nullptr, nullptr, (const int*)positions, nullptr,
                (const int*)block_table, ldbt, (bf16*)kpool, (bf16*)vpool, (float*)part_o, (float*)part_ml, (int)nh,
                (int)nkv, 0, (int)nsplit, 1.4426950408889634f / sqrtf((float)hd), 0.f, (unsigned*)tickets, (bf16*)out,
-               ldo, (const bf16*)q, (const int*)sel, (const int*)nsel, (int)topk, (int)ratio, nullptr, nullptr};
+               ldo, (const bf16*)q, (const int*)sel, (const int*)nsel, (int)topk, (int)ratio, nullptr, nullptr, nullptr};
   return decode_dispatch(a, M, nh, nkv, hd, 0, stream);
 }

@@ -799,18 +799,19 @@ def attn_decode(proj, qg, kg, cos, sin, positions, rope_pos, block_table, kpool,
     """``tickets``: zero-initialised int32 ``[M, nkv]`` arrival counters (re-armed by the kernel)."""
     M = positions.numel()
     call("attn_decode", proj, proj.stride(0), qg, kg, cos, sin, positions, rope_pos, block_table,
-         block_table.stride(0), kpool, vpool, part_o, part_ml, tickets, out, out.stride(0), M, nh, nkv, hd, rot,
-         nsplit, float(eps), kscale, vscale)
+         block_table.stride(0), kpool, vpool, kpool.shape[0], part_o, part_ml, tickets, out, out.stride(0), M, nh, nkv, hd, rot,
+         nsplit, float(eps), kscale, vscale, status_word(proj.device))
     _count()
     return out
 
 
 def decode_splits(nkv: int, rows: int) -> int:
     """Key-tile splits so that a decode attention launch (one 8-warp CTA per kv head, split and
-    row) covers about one wave of SMs."""
+    row) covers about one wave of SMs.  The batch kernel shares the tiles of all rows among its CTAs; this is the
+    room for partials of one (row, kv head), for a row eight times as long as the average."""
     pairs = max(1, nkv * rows)
-    if pairs >= ATTN_BATCH_PAIRS:       # tensor-core batch kernel: two 4-warp CTAs per SM
-        return max(1, min(32, 296 // pairs))
+    if pairs >= ATTN_BATCH_PAIRS:
+        return max(4, min(64, 2368 // pairs))
     return max(1, min(32, 148 // pairs))
 
 

@@ -928,3 +928,44 @@ def test_moe_gemv_w4a8_by_expert(E, N, Kd, swiglu, slots, monkeypatch):
         k.moe_gemv_w4(wq, sc, x, got, slot_e, rows, swiglu=swiglu)
         assert bool((got[slot_e < 0] == 3.0).all())
         close(got, want, 2 ** -7)
+
+
+@pytest.mark.parametrize("M,nkv,nsplit", [(8, 4, 64), (9, 4, 1), (16, 2, 2), (70, 1, 9)])
+def test_decode_attention_of_rows_of_any_length(M, nkv, nsplit):
+    """Tiles of all rows shared evenly (runs that start and end inside a row, whole pairs when there is room for one partial, padded
+    rows, a first token) against the kernel that takes a row at a time: scores and sums in fp32, P rounded to bf16 in one of them."""
+    k = K()
+    rep, hd, rot = 4, 256, 64
+    nh = nkv * rep
+    g = torch.Generator().manual_seed(M)
+    pos = torch.randint(0, 900, (M,), generator=g, dtype=torch.int32)
+    pos[0], pos[1], pos[M // 2], pos[M - 1] = 0, 3001, -1, 63
+    pages = [(int(p) + 64) // 64 for p in pos.clamp(min=0)]
+    order, bt, at = torch.randperm(sum(pages), generator=g), torch.zeros(M, max(pages), dtype=torch.int32), 0
+    for m, p in enumerate(pages):
+        bt[m, :p] = order[at:at + p]
+        at += p
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+    kp, vp = rnd(sum(pages) * 64, nkv, hd), rnd(sum(pages) * 64, nkv, hd)
+    proj = rnd(M, nh * 2 * hd + 2 * nkv * hd)
+    gain = torch.ones(hd, device=DEV)
+    cos, sin = O.rope_tables(rot, 1e6, 3100)
+    pos, bt, cos, sin = pos.to(DEV), bt.to(DEV), cos.to(DEV), sin.to(DEV)
+
+    def run(ctas, ns):
+        pools, out = (kp.clone(), vp.clone()), torch.zeros(M, nh * hd, dtype=torch.bfloat16, device=DEV)
+        part_o, part_ml = torch.empty(M, nh, ns, hd, device=DEV), torch.empty(M, nh, ns, 2, device=DEV)
+        tickets = torch.zeros(M, nkv, dtype=torch.int32, device=DEV)
+        k._lib.call_nostream("set_attn_batch_ctas", ctas)
+        try:
+            for _ in range(2):
+                k.attn_decode(proj, gain, gain, cos, sin, pos, pos.clamp(min=0), bt, *pools, part_o, part_ml, tickets, out, nh=nh, nkv=nkv,
+                              hd=hd, rot=rot, nsplit=ns, eps=1e-6)
+        finally:
+            k._lib.call_nostream("set_attn_batch_ctas", 32)
+        assert not bool(tickets.any())
+        return out, pools
+
+    (want, wp), (got, gp) = run(0, 8), run(1, nsplit)
+    assert torch.equal(wp[0], gp[0]) and torch.equal(wp[1], gp[1])
+    close(got, want, 1e-2)
