@@ -1078,8 +1078,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnC
     cp_async_wait_all();
   }
   __syncthreads();
-  // ---- nvv = W (beta V), kcd = W (beta e^c K): warp (row tile) x (V or K half); W is lower triangular, its columns take the
-  // factors of the rows they meet ------
+  // ---- nvv = W (beta V), kcd = W (beta e^c K): warp (row tile) x (V or K half); W is lower triangular; beta goes into its
+  // columns and e^c into the rows of K as the fragments are loaded ------
   {
     const bool isv = (warp >> 2) == 0;
     const float* B = isv ? Vs : Ks;
@@ -1092,8 +1092,8 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnC
     for (int k0 = 0; k0 < r0 + 16; k0 += 8) {
       uint32_t aw[4];
       frag_a(Wi, LDL, r0, k0, g, t, aw);
-      float f0 = bs[k0 + t], f1 = bs[k0 + t + 4];
-      if (!isv) { f0 *= __expf(cs[k0 + t]); f1 *= __expf(cs[k0 + t + 4]); }
+      const float f0 = bs[k0 + t], f1 = bs[k0 + t + 4];
+      const float e0 = isv ? 1.f : __expf(cs[k0 + t]), e1 = isv ? 1.f : __expf(cs[k0 + t + 4]);
       aw[0] = __float_as_uint(__uint_as_float(aw[0]) * f0); aw[1] = __float_as_uint(__uint_as_float(aw[1]) * f0);
       aw[2] = __float_as_uint(__uint_as_float(aw[2]) * f1); aw[3] = __float_as_uint(__uint_as_float(aw[3]) * f1);
 #pragma unroll
@@ -1101,7 +1101,7 @@ __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnC
         if (j < nt) {
           uint32_t b[2];
           frag_b(B, ldb, k0, j * 8, g, t, b);
-          mma_tf32(acc[j], aw[0], aw[1], aw[2], aw[3], b[0], b[1]);
+          mma_tf32(acc[j], aw[0], aw[1], aw[2], aw[3], __float_as_uint(__uint_as_float(b[0]) * e0), __float_as_uint(__uint_as_float(b[1]) * e1));
         }
       }
     }
