@@ -9,13 +9,14 @@
 //              while the kernels ahead of it drain;
 //   warp 1   : MMA issuer;
 //   warps 2-5: epilogue - accumulator out of TMEM through shared memory, so that a warp stores 128 consecutive columns of a row.
-// K is split over the S CTAs of a cluster (S <= 8): every output tile gets enough CTAs to fill the machine in one wave however
-// narrow N is, and the partial tiles are added over distributed shared memory, in slice order, each CTA finishing 1 / S of the
-// tile.  No workspace, no tickets, and the sum does not depend on timing.
-// Measured back to back in a graph (weights of every launch cold): 2560 x 9216, 64 rows 35.6 -> 13.6 us, 2560 x 4096 19.3 -> 8.7 us
-// against the 128-row tiles with partial tiles in global memory; 8 rows 25.0 -> 11.8 us and 10.0 -> 6.9 us against the mma.sync
-// GEMV; gate|up 18432 x 2560 with the product 24.9 -> 17.4 us (5.4 TB/s of W).  What is left is the chain of latencies of one
-// launch (dependency, first A tile, accumulator, cluster exchange, store), about 4 us.
+// K is split over the S CTAs of a cluster (S <= 8), and the partial tiles are added over distributed shared memory, in slice
+// order, each CTA finishing 1 / S of the tile.  No workspace, no tickets, and the sum does not depend on timing.
+// Measured back to back in a graph (weights of every launch cold): 64 rows, 2560 x 9216 35.6 -> 15.0 us, 2560 x 4096 19.3 -> 12.1 us
+// against the 128-row tiles with partial tiles in global memory (with slices that fill the machine 14.6 and 10.4 us); 8 rows 25.0 ->
+// 11.8 us and 10.0 -> 6.9 us against the mma.sync GEMV; gate|up 18432 x 2560 of 64 rows with the product 24.9 -> 21.5 us.  What is left
+// is the chain of latencies of one launch (dependency, first A tile, accumulator, cluster exchange, store), about 4 us.
+#include <algorithm>
+
 #include "act_type.cuh"
 #include "sm100.cuh"
 
@@ -35,6 +36,9 @@ struct RowsArgs {
   int act; float act_a, act_b;
   int M, N, up_off;                                  // N: output columns; SWIGLU: gate row n is paired with row up_off + n
   int n_tiles, k_blocks;
+  int wt;                                            // rows of W a tile: 128 or 64 (SWIGLU: half of them gate, half up)
+  int kper;                                          // k-blocks of a slice, the last one shorter (0: even slices)
+  int scale_rows_first;                              // int8: (sum * row scale) * column scale instead of sum * (row scale * column scale)
   int* status;
 };
 
@@ -99,7 +103,6 @@ __global__ void __launch_bounds__(kRowsThreads, 2)
 gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmA, const RowsArgs a) {
   constexpr int W_BYTES = kRowsTile * kRowsKB, A_BYTES = MT * kRowsKB, STAGE_BYTES = W_BYTES + A_BYTES;
   constexpr int BK = I8 ? 128 : 64;                  // elements of a k-block
-  constexpr int TN = SWIGLU ? 64 : 128;              // output columns of a tile
   constexpr uint32_t TMEM_COLS = 2 * MT;             // two accumulators (a power of two >= 32)
   constexpr uint32_t IDESC = umma_idesc(kRowsTile, MT, 1, I8 ? 2 : 1);
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -112,7 +115,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int S = gridDim.x, ks = blockIdx.x;          // the cluster is the whole x extent of the grid
-  const int kb0 = (int)((int64_t)a.k_blocks * ks / S), kb1 = (int)((int64_t)a.k_blocks * (ks + 1) / S);
+  const int kb0 = a.kper ? ks * a.kper : (int)((int64_t)a.k_blocks * ks / S);
+  const int kb1 = a.kper ? min(a.k_blocks, kb0 + a.kper) : (int)((int64_t)a.k_blocks * (ks + 1) / S);
+  const int wt = a.wt, tn = SWIGLU ? wt / 2 : wt;    // output columns of a tile
+  const int cbits = __ffs(tn) - 3;                   // log2 of its groups of four columns
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
@@ -127,13 +133,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (lane == 0) {
       auto load_w = [&](int tile, int kb, int s) {
         unsigned char* st = ring + (size_t)s * STAGE_BYTES;
-        mbar_expect_tx(&full_bar[s], STAGE_BYTES);
-        if (SWIGLU) {
-          tma_load_2d(st, &tmW, &full_bar[s], kb * BK, tile * TN);
-          tma_load_2d(st + W_BYTES / 2, &tmW, &full_bar[s], kb * BK, a.up_off + tile * TN);
-        } else {
-          tma_load_2d(st, &tmW, &full_bar[s], kb * BK, tile * TN);
-        }
+        mbar_expect_tx(&full_bar[s], wt * kRowsKB + A_BYTES);
+        tma_load_2d(st, &tmW, &full_bar[s], kb * BK, tile * tn);
+        if (SWIGLU) tma_load_2d(st + tn * kRowsKB, &tmW, &full_bar[s], kb * BK, a.up_off + tile * tn);
       };
       auto load_a = [&](int kb, int s) { tma_load_2d(ring + (size_t)s * STAGE_BYTES + W_BYTES, &tmA, &full_bar[s], kb * BK, 0); };
       const int per = kb1 - kb0, first = min(per, STAGES);
@@ -196,7 +198,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (I8) {
       const float rs = a.row_scale[m];
       const float4 cs = *reinterpret_cast<const float4*>(a.col_scale + n);
-      v.x *= rs * cs.x; v.y *= rs * cs.y; v.z *= rs * cs.z; v.w *= rs * cs.w;
+      if (a.scale_rows_first) { v.x = v.x * rs * cs.x; v.y = v.y * rs * cs.y; v.z = v.z * rs * cs.z; v.w = v.w * rs * cs.w; }
+      else { v.x *= rs * cs.x; v.y *= rs * cs.y; v.z *= rs * cs.z; v.w *= rs * cs.w; }
       if (SWIGLU) {
         const float4 cu = *reinterpret_cast<const float4*>(a.col_scale + a.up_off + n);
         u.x *= rs * cu.x; u.y *= rs * cu.y; u.z *= rs * cu.z; u.w *= rs * cu.w;
@@ -234,7 +237,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         // one tile a cluster: the ring is idle now, the whole partial tile goes there as [m][128]
         float* part = reinterpret_cast<float*>(ring);
 #pragma unroll 1
-        for (int c0 = 0; c0 < MT && c0 < a.M; c0 += 16) {
+        for (int c0 = 0; c0 < MT && c0 < a.M && q * 32 < wt; c0 += 16) {
           uint32_t r[16];
           tmem_ld16(lane_base + acc * MT + c0, r);
           tmem_ld_wait();
@@ -246,17 +249,18 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
 #pragma unroll 1
       for (int c0 = 0; c0 < MT && c0 < a.M; c0 += 16) {
         uint32_t r[16];
-        tmem_ld16(lane_base + acc * MT + c0, r);
-        tmem_ld_wait();
+        if (q * 32 < wt) {
+          tmem_ld16(lane_base + acc * MT + c0, r);
+          tmem_ld_wait();
 #pragma unroll
-        for (int i = 0; i < 16; ++i) chunk[i * 128 + q * 32 + lane] = __uint_as_float(r[i]);
+          for (int i = 0; i < 16; ++i) chunk[i * 128 + q * 32 + lane] = __uint_as_float(r[i]);
+        }
         asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-        for (int e = et; e < 16 * (TN / 4); e += 128) {
-          const int m = e / (TN / 4), n = (e % (TN / 4)) * 4;
+        for (int e = et; e < 16 << cbits; e += 128) {
+          const int m = e >> cbits, n = (e & ((1 << cbits) - 1)) * 4;
           const float4 v = rows_gather<I8>(0, (uint32_t)(m * 128 + n) * 4, 1, chunk);
-          const float4 u = SWIGLU ? rows_gather<I8>(0, (uint32_t)(m * 128 + 64 + n) * 4, 1, chunk) : v;
-          finish(c0 + m, tile * TN + n, v, u);
+          const float4 u = SWIGLU ? rows_gather<I8>(0, (uint32_t)(m * 128 + tn + n) * 4, 1, chunk) : v;
+          finish(c0 + m, tile * tn + n, v, u);
         }
         asm volatile("bar.sync 1, 128;" ::: "memory");
       }
@@ -270,12 +274,12 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     cluster_sync_all();                              // every slice's partial tile is in place
     if (warp >= 2 && staged) {
       const uint32_t base = smem_u32(ring);
-      const int tile = blockIdx.y, total = a.M * (TN / 4);
+      const int tile = blockIdx.y, total = a.M << cbits;
       for (int e = ks * 128 + et; e < total; e += S * 128) {
-        const int m = e / (TN / 4), n = (e % (TN / 4)) * 4;
+        const int m = e >> cbits, n = (e & ((1 << cbits) - 1)) * 4;
         const float4 v = rows_gather<I8>(base, (uint32_t)(m * 128 + n) * 4, S, nullptr);
-        const float4 u = SWIGLU ? rows_gather<I8>(base, (uint32_t)(m * 128 + 64 + n) * 4, S, nullptr) : v;
-        finish(m, tile * TN + n, v, u);
+        const float4 u = SWIGLU ? rows_gather<I8>(base, (uint32_t)(m * 128 + tn + n) * 4, S, nullptr) : v;
+        finish(m, tile * tn + n, v, u);
       }
     }
     cluster_sync_all();                              // nobody leaves while its shared memory is being read
@@ -304,15 +308,40 @@ int rows_sms() {
   return sms;
 }
 
-// Slices of K per output tile: as many as one wave of CTAs takes.  Pairs fill both CTAs of every SM (up to 296 CTAs); wider clusters
-// have to fit into the SMs of one GPC and leave some idle, so beyond about 1.4 CTAs an SM a second wave starts.  Measured at 16 rows:
-// 2560 x 4096 (20 tiles) 21.8 / 12.7 / 8.6 / 6.9 us with 1 / 2 / 4 / 8 slices; 12352 x 2560 (97 tiles) 15.6 / 13.8 / 16.6 with 1 / 2 / 4;
-// 6176 x 2560 (49 tiles) 12.0 us with 6 slices (294 CTAs).  Odd slice counts lose to the even ones beside them (TPCs are pairs of SMs).
-int rows_slices(int64_t tiles, int64_t kb) {
+// Decode projections of two to eight rows: as many slices of K per output tile as one wave of CTAs takes.  Pairs fill both CTAs of
+// every SM (up to 296 CTAs); wider clusters have to fit into the SMs of one GPC and leave some idle, so beyond about 1.4 CTAs an SM a
+// second wave starts.  Measured at 16 rows: 2560 x 4096 (20 tiles) 21.8 / 12.7 / 8.6 / 6.9 us with 1 / 2 / 4 / 8 slices; 12352 x 2560
+// (97 tiles) 15.6 / 13.8 / 16.6 with 1 / 2 / 4; 6176 x 2560 (49 tiles) 12.0 us with 6 slices (294 CTAs).  Odd slice counts lose to the
+// even ones beside them (TPCs are pairs of SMs).
+int fill_slices(int64_t tiles, int64_t kb) {
   const int64_t sms = rows_sms();
   int s = 8;
   while (s > 1 && (tiles * s > (s == 2 ? 2 * sms : sms * 7 / 5) || kb < 4 * s)) s = s > 2 ? s - 2 : 1;   // a slice has at least four k-blocks
   return s;
+}
+
+// Batched products: slices of ceil(k_blocks / s) k-blocks, s by the estimate below: the bytes a CTA moves into shared memory with
+// tiles of 256, 128 or 64 rows of W and one CTA an SM, against what adding s partial tiles costs.  The slices are part of a product's
+// value: bf16 residuals and recurrent states carry a changed order of sums through all layers that follow (64 rows of the 32-layer
+// shape: half an rms at single elements of the states), so they stay as they are when kernels change.
+int planned_slices(int64_t M, int64_t N, int64_t Kbytes, int narrowest) {
+  const int64_t sms = rows_sms(), kb = (Kbytes + 127) / 128, K = Kbytes / 2;
+  double best = 1e300;
+  int64_t slices = 1;
+  for (int bn = 256; bn >= narrowest; bn /= 2) {
+    const int64_t tiles = (N + bn - 1) / bn;
+    int64_t s = std::max<int64_t>(1, std::min<int64_t>(32, std::min(sms / tiles, kb / 4)));
+    for (;;) {                           // no slice may be empty: s = ceil(kb / ceil(kb / s))
+      const int64_t kper = (kb + s - 1) / s, s2 = (kb + kper - 1) / kper;
+      if (s2 == s) break;
+      s = s2;
+    }
+    const int64_t waves = (tiles * s + sms - 1) / sms;
+    const double stream = (double)waves * (bn + M) * ((double)K / s) * 2.0 / 130e3;        // us at ~130 GB/s per SM
+    const double cost = stream + (s > 1 ? (double)s * M * bn * 4.0 / 100e3 + 2.0 : 0.0);
+    if (cost < best) { best = cost; slices = s; }
+  }
+  return (int)slices;
 }
 
 template <int MT, int STAGES, bool I8, bool SWIGLU>
@@ -341,19 +370,31 @@ int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmA, const RowsArgs& 
 }
 
 template <bool I8, bool SWIGLU>
-int rows_run(const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_rows, int64_t K, RowsArgs a, cudaStream_t st) {
+int rows_run(const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_rows, int64_t K, int fill, RowsArgs a, cudaStream_t st) {
   constexpr int BK = I8 ? 128 : 64;
   const CUtensorMapDataType dt = I8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const int mt = a.M <= 16 ? 16 : (a.M <= 32 ? 32 : (a.M <= 64 ? 64 : 128));
-  const int tn = SWIGLU ? 64 : 128;
+  a.k_blocks = (int)((K + BK - 1) / BK);
+  a.wt = kRowsTile;
+  const int64_t tiles = (w_rows + kRowsTile - 1) / kRowsTile;
+  const int planned = fill ? 0 : planned_slices(a.M, w_rows, K * (I8 ? 1 : 2), I8 ? 128 : 64);
+  int S = fill_slices(tiles, a.k_blocks);
+  if (I8) {
+    a.scale_rows_first = planned == 1;               // integer sums do not depend on the slices
+  } else if (planned >= 1 && planned <= 8) {
+    S = planned;
+    a.kper = (a.k_blocks + S - 1) / S;
+    // as many CTAs as fit in a wave.  64 rows of A: 12352 x 2560 (97 tiles, one slice) 20.5 us with 128-row tiles, 19.4 with 64-row ones;
+    // 2560 x 9216 (20 tiles, 7 slices) 15.1 and 22.6 us (280 CTAs in clusters of 7 take two waves)
+    if (S > 1 ? 2 * tiles * S <= rows_sms() * 7 / 5 : tiles <= rows_sms()) a.wt = kRowsTile / 2;
+  }
+  const int tn = SWIGLU ? a.wt / 2 : a.wt;
   CUtensorMap tmW, tmA;
   int rc = cb_make_tmap_2d(&tmW, dt, I8 ? 1 : 2, W, (uint64_t)w_rows, (uint64_t)K, (uint64_t)ldw, tn, BK);
   if (rc) return rc;
   rc = cb_make_tmap_2d(&tmA, dt, I8 ? 1 : 2, A, (uint64_t)a.M, (uint64_t)K, (uint64_t)lda, mt, BK);
   if (rc) return rc;
   a.n_tiles = (a.N + tn - 1) / tn;
-  a.k_blocks = (int)((K + BK - 1) / BK);
-  const int S = rows_slices(a.n_tiles, a.k_blocks);
   if (mt == 16) return launch_rows<16, 5, I8, SWIGLU>(tmW, tmA, a, S, st);
   if (mt == 32) return launch_rows<32, 5, I8, SWIGLU>(tmW, tmA, a, S, st);
   if (mt == 64) return launch_rows<64, 4, I8, SWIGLU>(tmW, tmA, a, S, st);
@@ -373,25 +414,26 @@ int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M
 
 }  // namespace
 
-// C[M,N] = A[M,K] x W[N,K]^T, M <= 128; form 0: bf16 (+ residual), 1: fp32, 2: SwiGLU of the rows [0, N) and [N, 2N) of W.
+// C[M,N] = A[M,K] x W[N,K]^T, M <= 128; form 0: bf16 (+ residual), 1: fp32, 2: SwiGLU of the rows [0, N) and [N, 2N) of W.  fill:
+// K split to fill the machine, else by the plan of the batched products.
 CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
-                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, void* status, void* stream) {
+                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a) || K % 8) return CB_ERR_SHAPE;
-  if (form == 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, a, (cudaStream_t)stream);
-  return rows_run<false, false>(A, lda, W, ldw, N, K, a, (cudaStream_t)stream);
+  if (form == 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
+  return rows_run<false, false>(A, lda, W, ldw, N, K, fill != 0, a, (cudaStream_t)stream);
 }
 
 // The same from int8 rows and weights: (A_q x W_q^T) * row_scale[m] * col_scale[n], summed exactly.
 CB_EXPORT int cb_gemm_rows_i8(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
                               int64_t ldr, const void* row_scale, const void* col_scale, int64_t M, int64_t N, int64_t K, int64_t form,
-                              void* status, void* stream) {
+                              int64_t fill, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a)) return CB_ERR_SHAPE;
   if (K % 16 || lda % 16 || ldw % 16 || !row_scale || !col_scale) return CB_ERR_SHAPE;
   a.row_scale = (const float*)row_scale; a.col_scale = (const float*)col_scale;
-  if (form == 2) return rows_run<true, true>(A, lda, W, ldw, 2 * N, K, a, (cudaStream_t)stream);
-  return rows_run<true, false>(A, lda, W, ldw, N, K, a, (cudaStream_t)stream);
+  if (form == 2) return rows_run<true, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
+  return rows_run<true, false>(A, lda, W, ldw, N, K, fill != 0, a, (cudaStream_t)stream);
 }
 
 // Forms of gemm_tc.cu's entry points for few rows (arguments checked there): xIELU in the epilogue; the columns from n_main on as
@@ -401,12 +443,12 @@ int cb_gemm_rows_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, v
   RowsArgs a;
   if (rows_args(C, ldc, nullptr, 0, M, N, K, 0, status, &a)) return CB_ERR_SHAPE;
   a.act = 1; a.act_a = act_a; a.act_b = act_b;
-  return rows_run<false, false>(A, lda, W, ldw, N, K, a, (cudaStream_t)stream);
+  return rows_run<false, false>(A, lda, W, ldw, N, K, 0, a, (cudaStream_t)stream);
 }
 int cb_gemm_rows_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2, int64_t n_main,
                        int64_t M, int64_t N, int64_t K, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, nullptr, 0, M, N, K, 0, status, &a)) return CB_ERR_SHAPE;
   a.C2 = (float*)C2; a.ldc2 = ldc2; a.n_main = (int)n_main;
-  return rows_run<false, false>(A, lda, W, ldw, N, K, a, (cudaStream_t)stream);
+  return rows_run<false, false>(A, lda, W, ldw, N, K, 0, a, (cudaStream_t)stream);
 }

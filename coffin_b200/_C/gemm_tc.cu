@@ -292,7 +292,7 @@ int pick_bn(int M, int N, int sms, bool allow64) {
 int cb_gemm_rows_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N, int64_t K,
                        float act_a, float act_b, void* status, void* stream);
 CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
-                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, void* status, void* stream);
+                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, void* status, void* stream);
 int cb_gemm_rows_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2, int64_t n_main,
                        int64_t M, int64_t N, int64_t K, void* status, void* stream);
 
@@ -403,7 +403,7 @@ CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int6
 CB_EXPORT int cb_gemm_bf16_f32out(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M,
                                   int64_t N, int64_t K, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 4 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, status, stream);
+  if (M <= BM) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, 0, status, stream);
   const int sms = sm_count();
   const int bn = pick_bn((int)M, (int)N, sms, true);
   CUtensorMap tmA, tmB;

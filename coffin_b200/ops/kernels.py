@@ -298,7 +298,7 @@ def gemv(W: torch.Tensor, x: torch.Tensor | None, out: torch.Tensor | None, *, s
     elif norm is not None and M >= NORM_SPLIT_ROWS and pull_site < 0:
         x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
     if x is not None and tpp is None and _rows_gemv_ok(W, x, out, M, N, K):
-        return _gemm_rows(x, W, out, form=2 if swiglu else int(f32))
+        return _gemm_rows(x, W, out, form=2 if swiglu else int(f32), fill=True)
     if GEMV_IMPL == "mma" and M * K * 2 <= 160 * 1024:
         call("gemv_mma_bf16", W, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
              pull_site, push_site)
@@ -344,7 +344,7 @@ def gemv_i8(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
                         quant=(torch.empty(M, K, dtype=torch.int8, device=Wq.device), torch.empty(M, dtype=torch.float32, device=Wq.device)))
         else:
             q = quant_rows(x)
-        return _gemm_rows_i8(*q, Wq, wscale, out, form=2 if swiglu else mode >> 1)
+        return _gemm_rows_i8(*q, Wq, wscale, out, form=2 if swiglu else mode >> 1, fill=True)
     if x is None and M >= NORM_SPLIT_ROWS and pull_site < 0:
         x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
     call("gemv_i8", Wq, wscale, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
@@ -588,17 +588,18 @@ def gemm_i8_swiglu(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_
 ROWS = 128
 
 
-def _gemm_rows(A, W, out, residual=None, form: int = 0):
-    """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows."""
+def _gemm_rows(A, W, out, residual=None, form: int = 0, fill: bool = False):
+    """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows.  ``fill``: slices
+    of K that fill the machine (decode projections of two to eight rows), else those of the batched products, whose sums keep their order."""
     call("gemm_rows_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
-         A.shape[0], out.shape[1], A.shape[1], form, status_word(A.device))
+         A.shape[0], out.shape[1], A.shape[1], form, int(fill), status_word(A.device))
     _count()
     return out
 
 
-def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0):
+def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0, fill: bool = False):
     call("gemm_rows_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
-         a_scale, w_scale, Aq.shape[0], out.shape[1], Aq.shape[1], form, status_word(Aq.device))
+         a_scale, w_scale, Aq.shape[0], out.shape[1], Aq.shape[1], form, int(fill), status_word(Aq.device))
     _count()
     return out
 

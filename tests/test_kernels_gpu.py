@@ -831,6 +831,26 @@ def test_few_row_products(M, N, Kd):
             assert off(k.gemv_i8(w8[:N], ws[:N], Ad, f), r8[:, :N]) < 1e-6
 
 
+@pytest.mark.parametrize("M,N,Kd,kper", [(16, 2560, 4096, 22), (64, 2560, 9216, 21), (33, 264, 2048, 4), (64, 12352, 2560, 40), (9, 2048, 512, 4),
+                                         (100, 1032, 4104, 9), (64, 2048, 4096, 16)])
+def test_few_row_products_keep_the_order_of_their_sums(M, N, Kd, kper):
+    """Slices of ``kper`` k-blocks of 64, each summed along K and added in order, bit for bit: a slice by itself is a product of more than
+    128 rows, which is not split.  (What follows in a model carries every change of rounding through all layers.)"""
+    k = K()
+    from coffin_b200.ops import mixers as X
+    A, W = bf(160, Kd, seed=1).to(DEV), bf(N, Kd, s=Kd ** -0.5, seed=2).to(DEV)
+    want, part = None, torch.empty(160, N, device=DEV)
+    for at in range(0, Kd, 64 * kper):
+        X.gemm_f32out(A[:, at:at + 64 * kper], W[:, at:at + 64 * kper], part)
+        want = part.clone() if want is None else want + part
+    assert torch.equal(X.gemm_f32out(A[:M], W, torch.empty(M, N, device=DEV)), want[:M])
+    assert torch.equal(k.gemm(A[:M], W), want[:M].bfloat16())
+    n = N // 16 * 8
+    main, gates = torch.empty(M, n, dtype=torch.bfloat16, device=DEV), torch.empty(M, N - n, device=DEV)
+    X.gemm_mixed(A[:M], W, main, gates)
+    assert torch.equal(main, want[:M, :n].bfloat16()) and torch.equal(gates, want[:M, n:])
+
+
 @pytest.mark.parametrize("nk,nv,dk,lens", [(16, 32, 128, (1, 64, 65, 130, 300)), (16, 48, 128, (512, 127)), (2, 4, 64, (3, 200, 64))])
 def test_gdn_prefill_of_several_sequences(nk, nv, dk, lens):
     """One call over stacked sequences against one call each, bit for bit: chunk edges, a slot order of its own, rows before the
