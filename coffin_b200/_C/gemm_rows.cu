@@ -38,6 +38,7 @@ struct RowsArgs {
   int n_tiles, k_blocks;
   int wt;                                            // rows of W a tile: 128 or 64 (SWIGLU: half of them gate, half up)
   int kper;                                          // k-blocks of a slice, the last one shorter (0: even slices)
+  int round_halves;                                  // SWIGLU of gate and up as bf16 holds them
   int scale_rows_first;                              // int8: (sum * row scale) * column scale instead of sum * (row scale * column scale)
   int* status;
 };
@@ -204,6 +205,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
         const float4 cu = *reinterpret_cast<const float4*>(a.col_scale + a.up_off + n);
         u.x *= rs * cu.x; u.y *= rs * cu.y; u.z *= rs * cu.z; u.w *= rs * cu.w;
       }
+    }
+    if (SWIGLU && a.round_halves) {
+      v.x = act_round<bf16>(v.x); v.y = act_round<bf16>(v.y); v.z = act_round<bf16>(v.z); v.w = act_round<bf16>(v.w);
+      u.x = act_round<bf16>(u.x); u.y = act_round<bf16>(u.y); u.z = act_round<bf16>(u.z); u.w = act_round<bf16>(u.w);
     }
     if (SWIGLU) { v.x = silu_f(v.x) * u.x; v.y = silu_f(v.y) * u.y; v.z = silu_f(v.z) * u.z; v.w = silu_f(v.w) * u.w; }
     if (a.act) {
@@ -403,10 +408,11 @@ int rows_run(const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_r
 
 int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, void* status,
               RowsArgs* out) {
-  if (M < 1 || M > kRowsTile || N < 1 || K < 1 || N % 8 || form < 0 || form > 2 || !C || !status) return CB_ERR_SHAPE;
+  if (M < 1 || M > kRowsTile || N < 1 || K < 1 || N % 8 || form < 0 || form > 3 || !C || !status) return CB_ERR_SHAPE;
   if (ldc % (form == 1 ? 4 : 8) || (residual && (ldr % 8 || form == 1))) return CB_ERR_SHAPE;
   RowsArgs a = {};
   a.C = C; a.ldc = ldc; a.residual = (const bf16*)residual; a.ldr = ldr; a.c_f32 = form == 1;
+  a.round_halves = form == 3;
   a.M = (int)M; a.N = (int)N; a.up_off = (int)N; a.status = (int*)status;
   *out = a;
   return CB_OK;
@@ -414,13 +420,13 @@ int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M
 
 }  // namespace
 
-// C[M,N] = A[M,K] x W[N,K]^T, M <= 128; form 0: bf16 (+ residual), 1: fp32, 2: SwiGLU of the rows [0, N) and [N, 2N) of W.  fill:
-// K split to fill the machine, else by the plan of the batched products.
+// C[M,N] = A[M,K] x W[N,K]^T, M <= 128; form 0: bf16 (+ residual), 1: fp32, 2: SwiGLU of the rows [0, N) and [N, 2N) of W, 3: the
+// same of gate and up rounded to bf16, as a product and cb_swiglu after it give it.  fill: K split to fill the machine, else by the plan of the batched products.
 CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
                                 int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a) || K % 8) return CB_ERR_SHAPE;
-  if (form == 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
+  if (form >= 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
   return rows_run<false, false>(A, lda, W, ldw, N, K, fill != 0, a, (cudaStream_t)stream);
 }
 
@@ -432,7 +438,7 @@ CB_EXPORT int cb_gemm_rows_i8(const void* A, int64_t lda, const void* W, int64_t
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a)) return CB_ERR_SHAPE;
   if (K % 16 || lda % 16 || ldw % 16 || !row_scale || !col_scale) return CB_ERR_SHAPE;
   a.row_scale = (const float*)row_scale; a.col_scale = (const float*)col_scale;
-  if (form == 2) return rows_run<true, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
+  if (form >= 2) return rows_run<true, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
   return rows_run<true, false>(A, lda, W, ldw, N, K, fill != 0, a, (cudaStream_t)stream);
 }
 

@@ -377,12 +377,13 @@ class Qwen35Model:
 
     def _gemm_gu(self, A, W, gu: torch.Tensor, aq=None, decode: bool = False):
         """Gate|up projection of a prefill chunk or a wide decode bucket (``decode``) into ``gu [T, 2I]``.  The SwiGLU product
-        comes out of the GEMM epilogue (decode buckets; chunks of more rows than one CTA-pair tile) and the ``[T, I]`` view
-        holding it is returned; otherwise ``gu`` is filled with both halves, rounded, and None is returned."""
+        comes out of the GEMM epilogue (decode buckets of bf16 weights; chunks of more rows than one CTA-pair tile) and the ``[T, I]``
+        view holding it is returned; otherwise ``gu`` is filled with both halves, rounded, and None is returned (int8 decode: the next
+        projection quantises the product of the halves as it is, without a rounding to bf16 in between)."""
         if isinstance(W, QW4):
             W = W.expanded()
         T = gu.shape[0]
-        if (decode and T <= K.ROWS and W.shape[0] % 16 == 0) or (K.PAIR_GEMM and T >= K.PAIR_MIN_ROWS and W.shape[0] >= 256):
+        if (decode and T <= K.ROWS and W.shape[0] % 16 == 0 and not isinstance(W, QW)) or (K.PAIR_GEMM and T >= K.PAIR_MIN_ROWS and W.shape[0] >= 256):
             if isinstance(W, QW):
                 q, sc = aq if aq is not None else K.quant_rows(A)
                 return K.gemm_i8_swiglu(q, sc, W.wq, W.scale, out=gu[:, :W.shape[0] // 2])

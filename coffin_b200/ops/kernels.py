@@ -551,7 +551,7 @@ def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = N
     """``out[M, I] = silu(A @ Wgu[:I]^T) * (A @ Wgu[I:]^T)``: the gate|up projection with the SwiGLU
     product taken in the GEMM epilogue (CTA-pair kernel; the even CTA of a pair stages gate rows, the
     odd one the matching up rows), so the ``[M, 2I]`` intermediate is never written.  Smaller products
-    run as projection + ``swiglu``."""
+    give what projection + ``swiglu`` gives (up to 128 rows in one kernel that rounds both halves)."""
     M, K = A.shape
     I = Wgu.shape[0] // 2
     assert A.stride(1) == 1 and Wgu.stride(1) == 1
@@ -559,7 +559,7 @@ def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = N
         out = torch.empty(M, I, dtype=torch.bfloat16, device=A.device)
     assert out.stride(1) == 1
     if M <= ROWS and I % 8 == 0:
-        return _gemm_rows(A, Wgu, out, form=2)
+        return _gemm_rows(A, Wgu, out, form=3)
     if not (PAIR_GEMM and M >= PAIR_MIN_ROWS and I >= 128):
         return swiglu(gemm(A, Wgu), out=out)
     call("gemm_bf16_swiglu", A, A.stride(0), Wgu, Wgu.stride(0), out, out.stride(0), M, I, I, K, status_word(A.device))
@@ -589,7 +589,8 @@ ROWS = 128
 
 
 def _gemm_rows(A, W, out, residual=None, form: int = 0, fill: bool = False):
-    """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows.  ``fill``: slices
+    """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows,
+    3: of the halves rounded to bf16.  ``fill``: slices
     of K that fill the machine (decode projections of two to eight rows), else those of the batched products, whose sums keep their order."""
     call("gemm_rows_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
          A.shape[0], out.shape[1], A.shape[1], form, int(fill), status_word(A.device))

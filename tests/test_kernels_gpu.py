@@ -851,6 +851,23 @@ def test_few_row_products_keep_the_order_of_their_sums(M, N, Kd, kper):
     assert torch.equal(main, want[:M, :n].bfloat16()) and torch.equal(gates, want[:M, n:])
 
 
+@pytest.mark.parametrize("M,I,Kd", [(1, 8, 64), (16, 9216, 2560), (64, 200, 520), (128, 1024, 2048)])
+def test_few_row_swiglu_is_the_product_and_swiglu_after_it(M, I, Kd):
+    """Gate and up are rounded to bf16 before the activation, bit for bit as two launches do it; int8 decode buckets leave both halves to
+    the quantising kernel."""
+    k = K()
+    A, W = bf(M, Kd, seed=1).to(DEV), bf(2 * I, Kd, s=3 * Kd ** -0.5, seed=2).to(DEV)
+    assert torch.equal(k.gemm_swiglu(A, W), k.swiglu(k.gemm(A, W)))
+    if Kd % 16 == 0:
+        from coffin_b200.models.qwen35.model import QW, Qwen35Model
+        w = QW(*k.quant_rows(W))
+        torch.cuda.synchronize()
+        q, s = k.quant_rows(A)
+        gu = torch.zeros(M, 2 * I, dtype=torch.bfloat16, device=DEV)
+        assert object.__new__(Qwen35Model)._gemm_gu(A, w, gu, decode=True) is None
+        assert torch.equal(gu, k.gemm_i8(q, s, w.wq, w.scale))
+
+
 @pytest.mark.parametrize("nk,nv,dk,lens", [(16, 32, 128, (1, 64, 65, 130, 300)), (16, 48, 128, (512, 127)), (2, 4, 64, (3, 200, 64))])
 def test_gdn_prefill_of_several_sequences(nk, nv, dk, lens):
     """One call over stacked sequences against one call each, bit for bit: chunk edges, a slot order of its own, rows before the
