@@ -160,7 +160,9 @@ __global__ void __launch_bounds__(4 * DV, MINB) gdn_decode_kernel(const GdnDecod
 // memory idle while a CTA computes: its loads, its arithmetic and its stores follow one another, and two CTAs an SM do not fill the
 // gaps.  Here one CTA an SM walks a share of the (row, head) pairs with three state buffers in shared memory: bulk copies bring the
 // next state and take the last one away while this one is updated, and the inputs of the convolution travel one pair ahead in
-// registers.  The arithmetic is the kernel's above.  64 rows of 32 heads (268 MB read and written, 41 us): 66 -> 46 us a layer.
+// registers.  The arithmetic is the kernel's above, rounding by rounding (the fused and the
+// separate multiplies and adds are written out, and the norm's sum is taken in block_sum's order): a row's state does not depend on
+// how many rows step with it.  64 rows of 32 heads (268 MB read and written, 41 us): 66 -> 46 us a layer.
 template <int DK, int DV>
 __global__ void __launch_bounds__(4 * DV, 1) gdn_decode_stream_kernel(const GdnDecodeArgs a, int M, int* status) {
   constexpr int G = 4, RPT = DK / G, ST = 3;
@@ -246,8 +248,10 @@ __global__ void __launch_bounds__(4 * DV, 1) gdn_decode_stream_kernel(const GdnD
 #pragma unroll
     for (int r = 0; r < RPT; ++r) s[r] = sp[r * DV];
     if (tid < 2 * DK + DV) {
-      const float v = silu_f(cur.w.x * __bfloat162float(cur.x[0]) + cur.w.y * __bfloat162float(cur.x[1]) + cur.w.z * __bfloat162float(cur.x[2]) +
-                             cur.w.w * __bfloat162float(cur.x[3]));
+      float v = __fmul_rn(cur.w.x, __bfloat162float(cur.x[0]));
+      v = fmaf(cur.w.y, __bfloat162float(cur.x[1]), v);
+      v = fmaf(cur.w.z, __bfloat162float(cur.x[2]), v);
+      v = silu_f(fmaf(cur.w.w, __bfloat162float(cur.x[3]), v));
       const int kh = h / a.rep;
       const int c = tid < DK ? kh * DK + tid : (tid < 2 * DK ? kdim + kh * DK + (tid - DK) : 2 * kdim + h * DV + (tid - 2 * DK));
       if (tid >= 2 * DK || h % a.rep == 0)
@@ -262,7 +266,7 @@ __global__ void __launch_bounds__(4 * DV, 1) gdn_decode_stream_kernel(const GdnD
       float acc = 0.f;
       for (int i = lane; i < DK; i += 32) {
         const float qa = q_s[i], ka = k_s[i];
-        acc += (w == 0) ? qa * qa : (w == 1) ? ka * ka : qa * ka;
+        acc = __fadd_rn(acc, __fmul_rn(w == 1 ? ka : qa, w == 0 ? qa : ka));
       }
       acc = warp_sum(acc);
       if (lane == 0) scal[w] = acc;
@@ -281,17 +285,17 @@ __global__ void __launch_bounds__(4 * DV, 1) gdn_decode_stream_kernel(const GdnD
     const float beta = sigmoid_f(__bfloat162float(cur.bl));
     const float alpha = __expf(-__expf(cur.A) * softplus_f(__bfloat162float(cur.al) + cur.db));
     const float Sk = (sk[0][j] + sk[1][j] + sk[2][j] + sk[3][j]) * rk;
-    const float d = (v_s[j] - alpha * Sk) * beta;
+    const float d = __fmul_rn(fmaf(-alpha, Sk, v_s[j]), beta);
 #pragma unroll
     for (int r = 0; r < RPT; ++r) sp[r * DV] = fmaf(k_s[grp * RPT + r] * rk, d, alpha * s[r]);
     sm100::fence_async_smem();                      // the bulk store below reads what was written here
     if (grp == 0) {                                 // gated RMSNorm over the head, by the first four warps
       const float Sq = (sq[0][j] + sq[1][j] + sq[2][j] + sq[3][j]) * rq;
-      const float o = alpha * Sq + kq * d;
+      const float o = fmaf(alpha, Sq, __fmul_rn(kq, d));
       const float ws = warp_sum(o * o);
       if (lane == 0) red[tid >> 5] = ws;
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float ms = (red[0] + red[1] + red[2] + red[3]) / (float)DV;
+      const float ms = ((red[0] + red[2]) + (red[1] + red[3])) / (float)DV;
       const float z = __bfloat162float(cur.z);
       a.out[(int64_t)m * a.ldo + h * DV + j] = __float2bfloat16(o * rsqrtf(ms + a.eps) * nw * (a.gate_sigmoid ? sigmoid_f(z) : silu_f(z)));
     }

@@ -921,6 +921,7 @@ def test_gdn_decode_of_many_rows(nk, nv, M):
     """More (row, head) pairs than two CTAs an SM hold: the streaming kernel against the per-pair one on eight rows at a time.  The
     norm's sum is taken in another order (fp32, one bf16 rounding) and the compiler contracts other multiplies and adds: a few fp32
     roundings (2^-24 each) of sums of 128 terms, 1e-5 of the scale.  Padded rows stay untouched."""
+
     k = K()
     dk, n = 128, M + 2
     proj, conv_w, A_log, dt_bias, norm_w, conv_dim = _gdn_inputs(M, nk, nv, dk, dk, 91)
@@ -943,6 +944,35 @@ def test_gdn_decode_of_many_rows(nk, nv, M):
     assert torch.equal(ring, r2)
     close(st, s2, 1e-5)
     close(got, want, 2 ** -7)
+
+
+@pytest.mark.parametrize("nk,nv,M", [(16, 32, 64), (16, 48, 17), (5, 5, 61)])
+def test_gdn_decode_of_many_rows_is_that_of_few(nk, nv, M):
+    """A row's state, ring and output are the same bits whether it steps with many rows or with few (states of ordinary size, three
+    steps, first tokens among them)."""
+    k = K()
+    dk = 128
+    conv_dim = 2 * nk * dk + nv * dk
+    g = torch.Generator().manual_seed(93)
+    ring, st = torch.zeros(M, k.RING, conv_dim, dtype=torch.bfloat16, device=DEV), torch.zeros(M, nv, dk, dk, device=DEV)
+    st[::2] = (0.1 * torch.randn(st[::2].shape, generator=g)).to(DEV)
+    slots = torch.randperm(M, generator=g).to(torch.int32).to(DEV)
+    _, conv_w, A_log, dt_bias, norm_w, _ = _gdn_inputs(M, nk, nv, dk, dk, 94)
+    args = [t.to(DEV) for t in (conv_w, A_log, dt_bias, norm_w.float())]
+    kw = dict(nk=nk, nv=nv, dk=dk, dv=dk, eps=1e-6)
+    r2, s2, few = ring.clone(), st.clone(), 290 // nv if nv < 290 else 1
+    for step in range(3):
+        pj = _gdn_inputs(M, nk, nv, dk, dk, 95 + step)[0].to(DEV)
+        pos = torch.full((M,), step, dtype=torch.int32, device=DEV)
+        want, got = (torch.zeros(M, nv * dk, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        torch.cuda.synchronize()
+        for at in range(0, M, few):
+            sl = slice(at, at + few)
+            k.gdn_decode(pj[sl], *args, r2, s2, slots[sl].contiguous(), pos[sl].contiguous(), want[sl], **kw)
+        torch.cuda.synchronize()
+        k.gdn_decode(pj, *args, ring, st, slots, pos, got, **kw)
+        torch.cuda.synchronize()
+        assert torch.equal(st, s2) and torch.equal(ring, r2) and torch.equal(got, want), step
 
 
 @pytest.mark.parametrize("E,N,Kd,swiglu,slots", [(6, 128, 256, True, 97), (5, 520, 2304, False, 200), (300, 24, 128, True, 512), (3, 2048, 512, False, 1024)])
