@@ -712,16 +712,22 @@ __global__ void __launch_bounds__(kDecWarps * 32, MINB) attn_decode_kernel(const
 // ------------------------------------------------------------------------------------------
 // Decode attention for a batch of rows on the tensor cores.  The kernel above is built for the
 // latency of one sequence (many key splits, scalar dot products with warp shuffles) and becomes issue
-// bound when every row brings its own CTAs.  Here one CTA serves one (row, kv head): the REP query
+// bound when every row brings its own CTAs.  Here a CTA serves tiles of one (row, kv head): the REP query
 // heads of the kv head are rows 0..REP-1 of a 16-row mma tile (the rest zero), the four warps take 16
 // keys each of every 64-key tile (S = Q K^T and O += P V as bf16 mma.m16n8k16 from ldmatrix
 // fragments, K and V tiles in turn by TMA through a ring of three, so that two are on their way while
-// one is used), keep their own running maximum and sum, and merge once at the end.  Two CTAs an SM
-// share the tiles of all rows evenly, whatever the rows' lengths: with equal splits a row, the SMs
-// with the long rows set the time (8 rows of 517 to 16391 tokens 97 -> 61 us, 64 of 1031 to 2047 98 -> 90 us).  Query / key normalisation, rotary embedding, the KV append of the current token and the
-// sigmoid output gate are part of the kernel as in the single-sequence one.
-constexpr int kBatchRows = 128;     // more would cost the second CTA an SM its shared memory
-template <int HD>
+// one is used), keep their own running maximum and sum, and merge once at the end.  Query / key
+// normalisation, rotary embedding, the KV append of the current token and the sigmoid output gate are
+// part of the kernel as in the single-sequence one.
+//
+// Wide batches (more than kSharedRows rows): every (row, kv head) has a.nsplit CTAs, which take its tiles in turn.  A row's sums
+// do not depend on the other rows' lengths.  Rows of 1 to 2560 tokens, 4 kv heads, against tiles staged with cp.async and waited for:
+// 16 rows 38.9 -> 33.3 us, 32 rows 69 -> 49 us, 64 rows 114 -> 75 us.
+// SHARED (few rows): the tiles of all rows are shared out by length, a pair cut into runs of adjacent tiles.  With equal splits a
+// row, the SMs with the long rows set the time (8 rows of 517 to 16391 tokens 97 -> 61 us; 64 rows of 1031 to 2047, with runs that
+// also crossed rows, 98 -> 90 us only, and their results moved with their neighbours).
+constexpr int kSharedRows = 8, kSharedCtas = 296;
+template <int HD, bool SHARED>
 __global__ void __launch_bounds__(128, 2)
 attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeArgs a, int rows) {
   constexpr int LD = HD + 8, EPL = HD / 32, CPR = HD / 8;
@@ -739,7 +745,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   __shared__ float mm_s[4][8], ml_s[4][8];
   __shared__ float linv_s[8];
   __shared__ bool is_last;
-  __shared__ int pre_s[kBatchRows + 1], per_s;
+  __shared__ int pre_s[kSharedRows + 1];
   __shared__ uint64_t full[3];
   const int rep = a.nh / a.nkv;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
@@ -749,81 +755,42 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   }
   griddep_launch();
   griddep_wait();
-  // The tiles of all (row, kv head) pairs are shared out in runs of about `per` tiles.  Up to half as many pairs as CTAs: every pair is
-  // cut into runs of its own (a CTA pays one prologue and one merge, about 15 us with what surrounds them).  More: the (row, kv head,
-  // tile) triples in order are cut evenly, runs cross pairs.  A pair's partials have room for a.nsplit runs; with room for one a CTA
-  // takes whole pairs.
-  const int pairs = rows * a.nkv, ctas = gridDim.x;
-  const bool whole = a.nsplit == 1, own = !whole && 2 * pairs <= ctas;
-  if (warp == 0) {
-    int sum = 0, most = 0, per = 1;
-    for (int m0 = 0; m0 < rows; m0 += 32) {
-      const int n = m0 + lane < rows ? a.positions[m0 + lane] : -1, nt = n < 0 ? 0 : n / kBlock + 1;       // a padded row has none
-      sum += nt;
-      most = max(most, nt);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-    }
-    sum *= a.nkv;
-    if (own) per = max((sum + ctas - pairs - 1) / (ctas - pairs), (most + a.nsplit - 1) / a.nsplit);
-    else if (!whole) per = max((sum + ctas - 1) / ctas, (most + a.nsplit - 2) / (a.nsplit - 1));
-    int before = 0;                               // pre_s: runs (own) or tiles of the rows before a row
-    for (int m0 = 0; m0 < rows; m0 += 32) {
-      int n = m0 + lane < rows ? a.positions[m0 + lane] : -1;
-      n = n < 0 ? 0 : n / kBlock + 1;
-      if (own) n = (n + per - 1) / per;
+  int m, kvh, split, nsplit, t0, step, cnt;       // tiles t0, t0 + step, .. (cnt of them) of row m; run `split` of its nsplit
+  if (SHARED) {
+    // every pair is cut into runs of at most `per` tiles (a CTA pays one prologue and one merge, about 15 us with what surrounds
+    // them); its partials have room for a.nsplit runs
+    if (warp == 0) {
+      const int pairs = rows * a.nkv, n = lane < rows ? a.positions[lane] : -1, nt = n < 0 ? 0 : n / kBlock + 1;   // a padded row has none
+      const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)nt) * a.nkv, most = (int)__reduce_max_sync(0xffffffffu, (unsigned)nt);
+      const int per = max((sum + kSharedCtas - pairs - 1) / (kSharedCtas - pairs), (most + a.nsplit - 1) / a.nsplit);
+      int runs = per ? (nt + per - 1) / per : 0;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, n, o);
-        if (lane >= o) n += y;
+        const int y = __shfl_up_sync(0xffffffffu, runs, o);
+        if (lane >= o) runs += y;
       }
-      if (m0 + lane < rows) pre_s[m0 + lane + 1] = before + n;
-      before += __shfl_sync(0xffffffffu, n, 31);
+      if (lane < rows) pre_s[lane + 1] = runs;    // runs of the rows up to this one, per kv head
+      if (lane == 0) pre_s[0] = 0;
     }
-    if (lane == 0) { pre_s[0] = 0; per_s = per; }
-  }
-  __syncthreads();
-  const int total = pre_s[rows] * a.nkv, per = per_s;
-  int u = whole || own ? blockIdx.x : blockIdx.x * per;
-  const int end = whole ? pairs : (own ? min(total, u + 1) : min(total, u + per));
-  uint32_t seq = 0;                               // halves requested by the runs before: ring position and phase go on
-  while (u < end) {
-  int m, kvh, t0, cnt, nsplit, split;
-  if (whole) {
-    m = u / a.nkv;
-    kvh = u % a.nkv;
-    u += ctas;
-    t0 = split = 0;
-    nsplit = 1;
-    cnt = pre_s[m + 1] - pre_s[m];
-    if (cnt == 0) continue;
+    __syncthreads();
+    const int u = blockIdx.x;
+    if (u >= pre_s[rows] * a.nkv) return;
+    m = 0;
+    while (pre_s[m + 1] * a.nkv <= u) ++m;
+    nsplit = pre_s[m + 1] - pre_s[m];
+    const int at = u - pre_s[m] * a.nkv, nt = a.positions[m] / kBlock + 1;
+    kvh = at / nsplit;
+    split = at % nsplit;
+    t0 = nt * split / nsplit;
+    cnt = nt * (split + 1) / nsplit - t0;
+    step = 1;
   } else {
-    int lo = 0, hi = rows;                        // the row of this run or triple: the last with pre[m] * nkv <= u
-    while (hi - lo > 1) {
-      const int mid = (lo + hi) >> 1;
-      if (pre_s[mid] * a.nkv <= u) lo = mid; else hi = mid;
-    }
-    m = lo;
-    const int n = pre_s[m + 1] - pre_s[m], at = u - pre_s[m] * a.nkv;
-    kvh = at / n;
-    if (own) {
-      const int nt = a.positions[m] / kBlock + 1;
-      nsplit = n;
-      split = at % n;
-      t0 = nt * split / n;
-      cnt = nt * (split + 1) / n - t0;
-      ++u;
-    } else {
-      t0 = at % n;
-      cnt = min(n - t0, end - u);
-      const int first = (u - t0) / per;
-      nsplit = (u - t0 + n - 1) / per - first + 1;
-      split = blockIdx.x - first;
-      u += cnt;
-    }
+    kvh = blockIdx.x;
+    m = blockIdx.y;
+    split = t0 = blockIdx.z;
+    nsplit = step = a.nsplit;
+    if (a.positions[m] < 0) return;               // padded row
+    cnt = max(0, (a.positions[m] / kBlock - split + nsplit) / nsplit);       // none for a split beyond the last tile
   }
   const int pos = a.positions[m], ntiles = pos / kBlock + 1;
   const bf16* prow = a.proj + (int64_t)m * a.ldp;
@@ -835,8 +802,8 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   // bulk copy a row, took longer than the products), int8 rows are converted on the way.
   auto load_half = [&](int h) {
     if (h >= 2 * cnt) return;
-    const int64_t slot0 = (int64_t)bt[t0 + (h >> 1)] * kBlock;
-    const uint32_t at = (seq + h) % 3;
+    const int64_t slot0 = (int64_t)bt[t0 + (h >> 1) * step] * kBlock;
+    const int at = h % 3;
     bf16* dst = ring + at * TILE;
     if (a.kscale) {
       const int8_t* pool = reinterpret_cast<const int8_t*>((h & 1) ? a.vpool : a.kpool);
@@ -853,7 +820,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
         sm100::tma_load_2d(dst + c * 64 * 64, (h & 1) ? &tmV : &tmK, &full[at], kvh * HD + c * 64, (int)slot0);
     }
   };
-  auto arrived = [&](int h) { return a.kscale || sm100::mbar_wait(&full[(seq + h) % 3], ((seq + h) / 3) & 1); };
+  auto arrived = [&](int h) { return a.kscale || sm100::mbar_wait(&full[h % 3], (h / 3) & 1); };
   load_half(0);
   load_half(1);
   // ---- prologue: q heads -> Qs (bf16), this token's K / V -> pool and shared copies ---------------
@@ -869,7 +836,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       norm_rope_lane<HD>(x, a.qg, cs, sn, a.rot, a.eps, lane);
 #pragma unroll
       for (int e = 0; e < EPL; ++e) Qs[r * LD + lane * EPL + e] = __float2bfloat16(x[e]);
-    } else if (t0 + cnt == ntiles) {             // the run that holds the last tile appends this token
+    } else if (cnt > 0 && t0 + (cnt - 1) * step == ntiles - 1) {   // the run that holds the last tile appends this token
       const int64_t slot = (int64_t)bt[pos / kBlock] * kBlock + pos % kBlock;
       if (r == rep) {
         const bf16* src = prow + (int64_t)a.nh * 2 * HD + (int64_t)kvh * HD + lane * EPL;
@@ -921,14 +888,14 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     ldsm_x4(qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], Qs + (lane & 15) * LD + kk * 16 + (lane >> 4) * 8);
   bool ok = true;
   for (int i = 0; i < cnt; ++i) {
-    const int kt = t0 + i;
-    bf16* Ks = ring + ((seq + 2 * i) % 3) * TILE;
-    bf16* Vs = ring + ((seq + 2 * i + 1) % 3) * TILE;
+    const int kt = t0 + i * step;
+    bf16* Ks = ring + (2 * i % 3) * TILE;
+    bf16* Vs = ring + ((2 * i + 1) % 3) * TILE;
     if (!(ok = arrived(2 * i))) break;
     __syncthreads();                              // K is here; the V tile before it is consumed
     load_half(2 * i + 2);
     if (kt == ntiles - 1) patch(Ks, kcur);
-    // ---- S = Q K^T for this warp's 16 keys, two chains ------------------------------------------
+    // ---- S = Q K^T for this warp's 16 keys; SHARED: two chains -----------------------------------
     float sc[2][4], s2[2][4];
 #pragma unroll
     for (int n = 0; n < 2; ++n) sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = s2[n][0] = s2[n][1] = s2[n][2] = s2[n][3] = 0.f;
@@ -936,11 +903,11 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     for (int kk = 0; kk < HD / 16; ++kk) {
       uint32_t b0, b1, b2, b3;
       ldsm_x4(b0, b1, b2, b3, Ks + piece(warp * 16 + (lane & 7) + ((lane >> 4) << 3), kk * 2 + ((lane >> 3) & 1)));
-      mma_bf16(kk & 1 ? s2[0] : sc[0], qf[kk], b0, b1);
-      mma_bf16(kk & 1 ? s2[1] : sc[1], qf[kk], b2, b3);
+      mma_bf16(SHARED && (kk & 1) ? s2[0] : sc[0], qf[kk], b0, b1);
+      mma_bf16(SHARED && (kk & 1) ? s2[1] : sc[1], qf[kk], b2, b3);
     }
 #pragma unroll
-    for (int n = 0; n < 2; ++n) { sc[n][0] += s2[n][0]; sc[n][1] += s2[n][1]; }
+    for (int n = 0; SHARED && n < 2; ++n) { sc[n][0] += s2[n][0]; sc[n][1] += s2[n][1]; }
     // ---- mask + online softmax (base 2), row g of the tile --------------------------------------
     float mnew = mrow;
 #pragma unroll
@@ -991,7 +958,6 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     for (int i = 0; i < 2000; ++i) __nanosleep(1000);
     return;
   }
-  seq += 2 * cnt;
   __syncthreads();                                // all warps are done with the tiles
   if (tq == 0) { mm_s[warp][g] = mrow; ml_s[warp][g] = lrow; }
 #pragma unroll
@@ -1030,9 +996,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     dst[2] = __float2bfloat16(acc.z * li * sigmoid_f(__bfloat162float(gp[2])));
     dst[3] = __float2bfloat16(acc.w * li * sigmoid_f(__bfloat162float(gp[3])));
   }
-  sm100::fence_async_smem();                      // the ring takes copies again
-  __syncthreads();                                // the partial outputs are read
-  if (nsplit == 1) continue;
+  if (nsplit == 1) return;
   // ---- several splits per (row, kv head): the last one to arrive merges all partials and applies the gate ----
   __threadfence();
   __syncthreads();
@@ -1042,7 +1006,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     if (is_last) *tk = 0;
   }
   __syncthreads();
-  if (!is_last) continue;
+  if (!is_last) return;
   __threadfence();
   const float* bo = a.part_o + ((int64_t)m * a.nh + kvh * rep) * a.nsplit * HD;
   const float* bml = a.part_ml + ((int64_t)m * a.nh + kvh * rep) * a.nsplit * 2;
@@ -1084,9 +1048,6 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     dst[1] = __float2bfloat16(acc.y * li * sigmoid_f(__bfloat162float(gp[1])));
     dst[2] = __float2bfloat16(acc.z * li * sigmoid_f(__bfloat162float(gp[2])));
     dst[3] = __float2bfloat16(acc.w * li * sigmoid_f(__bfloat162float(gp[3])));
-  }
-  sm100::fence_async_smem();
-  __syncthreads();                                // the merge's scales are read
   }
 }
 
@@ -1189,7 +1150,7 @@ CB_EXPORT int cb_attn_decode(const void* proj, int64_t ldp, const void* qg, cons
                (bf16*)vpool, (float*)part_o, (float*)part_ml, (int)nh, (int)nkv, (int)rot, (int)nsplit,
                1.4426950408889634f / sqrtf((float)hd), eps, (unsigned*)tickets, (bf16*)out, ldo,
                nullptr, nullptr, nullptr, 0, 1, (float*)kscale, (float*)vscale, (int*)status};
-  if (hd == 256 && (rot / 2) % 8 == 0 && nh / nkv <= 8 && g_attn_batch_ctas > 0 && nkv * M >= g_attn_batch_ctas && M <= kBatchRows &&
+  if (hd == 256 && (rot / 2) % 8 == 0 && nh / nkv <= 8 && g_attn_batch_ctas > 0 && nkv * M >= g_attn_batch_ctas &&
       (((uintptr_t)kpool | (uintptr_t)vpool) & 15) == 0) {
     // enough (row, kv head) pairs for the tensor-core batch kernel
     constexpr int HD = 256;
@@ -1200,9 +1161,12 @@ CB_EXPORT int cb_attn_decode(const void* proj, int64_t ldp, const void* qg, cons
       if (!rc) rc = cb_make_tmap_2d(&tmV, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, vpool, (uint64_t)slots, (uint64_t)(nkv * hd), (uint64_t)(nkv * hd), kBlock, 64);
       if (rc) return rc;
     }
-    cudaError_t e = cudaFuncSetAttribute(attn_decode_batch_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const bool shared = M <= kSharedRows && nsplit > 1 && 2 * nkv * M <= kSharedCtas;
+    auto kern = shared ? attn_decode_batch_kernel<HD, true> : attn_decode_batch_kernel<HD, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return (int)cb_launch(attn_decode_batch_kernel<HD>, dim3(296), dim3(128), smem, (cudaStream_t)stream, tmK, tmV, a, (int)M);
+    return (int)cb_launch(kern, shared ? dim3(kSharedCtas) : dim3((unsigned)nkv, (unsigned)M, (unsigned)nsplit), dim3(128), smem,
+                          (cudaStream_t)stream, tmK, tmV, a, (int)M);
   }
   return decode_dispatch(a, M, nh, nkv, hd, rot, stream);
 }

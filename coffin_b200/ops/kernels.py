@@ -809,14 +809,17 @@ def attn_decode(proj, qg, kg, cos, sin, positions, rope_pos, block_table, kpool,
 
 def decode_splits(nkv: int, rows: int) -> int:
     """Key-tile splits so that a decode attention launch (one 8-warp CTA per kv head, split and
-    row) covers about one wave of SMs.  The batch kernel shares the tiles of all rows among its CTAs; this is the
-    room for partials of one (row, kv head), for a row eight times as long as the average."""
+    row) covers about one wave of SMs.  Up to ``ATTN_SHARED_ROWS`` rows the batch kernel shares the tiles of all rows
+    among its CTAs; this is then the room for partials of one (row, kv head), for a row eight times as long as the average."""
     pairs = max(1, nkv * rows)
-    if pairs >= ATTN_BATCH_PAIRS:
+    if pairs < ATTN_BATCH_PAIRS:
+        return max(1, min(32, 148 // pairs))
+    if rows <= ATTN_SHARED_ROWS and 2 * pairs <= 296:
         return max(4, min(64, 2368 // pairs))
-    return max(1, min(32, 148 // pairs))
+    return max(1, min(32, 296 // pairs))             # tensor-core batch kernel: two 4-warp CTAs per SM
 
 
+ATTN_SHARED_ROWS = 8         # as in attn.cu
 # (row, kv head) pairs from which cb_attn_decode runs the tensor-core batch kernel
 ATTN_BATCH_PAIRS = int(os.environ.get("COFFIN_ATTN_BATCH_PAIRS", "32"))
 if ATTN_BATCH_PAIRS != 32:

@@ -1036,3 +1036,31 @@ def test_decode_attention_of_rows_of_any_length(M, nkv, nsplit):
     (want, wp), (got, gp) = run(0, 8), run(1, nsplit)
     assert torch.equal(wp[0], gp[0]) and torch.equal(wp[1], gp[1])
     close(got, want, 1e-2)
+
+
+@pytest.mark.parametrize("M,nkv", [(16, 4), (33, 2), (64, 4), (130, 1)])
+def test_decode_attention_of_wide_batches_takes_a_row_by_itself(M, nkv):
+    """From nine rows on a row's output is the same bits whatever the lengths of the others, with one split a row and several, splits
+    without a tile, and the row's token in the last one."""
+    k = K()
+    rep, hd, rot = 4, 256, 64
+    nh, ns = nkv * rep, k.decode_splits(nkv, M)
+    g = torch.Generator().manual_seed(M)
+    bt = torch.randperm(M * 20, generator=g).to(torch.int32).view(M, 20).to(DEV)
+    rnd = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+    kp, vp = rnd(M * 20 * 64, nkv, hd), rnd(M * 20 * 64, nkv, hd)
+    proj = rnd(M, nh * 2 * hd + 2 * nkv * hd)
+    gain = torch.ones(hd, device=DEV)
+    cos, sin = (t.to(DEV) for t in O.rope_tables(rot, 1e6, 1300))
+    one = torch.randint(0, 1280, (M,), generator=g, dtype=torch.int32)
+    one[:3] = torch.tensor([0, 63, 1279])
+    two = torch.randint(0, 1280, (M,), generator=g, dtype=torch.int32)
+    two[:M // 2] = one[:M // 2]
+    outs = []
+    for pos in (one, two):
+        pos, pools, out = pos.to(DEV), (kp.clone(), vp.clone()), torch.zeros(M, nh * hd, dtype=torch.bfloat16, device=DEV)
+        part_o, part_ml = torch.empty(M, nh, ns, hd, device=DEV), torch.empty(M, nh, ns, 2, device=DEV)
+        k.attn_decode(proj, gain, gain, cos, sin, pos, pos, bt, *pools, part_o, part_ml, torch.zeros(M, nkv, dtype=torch.int32, device=DEV),
+                      out, nh=nh, nkv=nkv, hd=hd, rot=rot, nsplit=ns, eps=1e-6)
+        outs.append(out[:M // 2])
+    assert torch.equal(*outs)
