@@ -42,6 +42,10 @@ struct GdnDecodeArgs {
   int gate_sigmoid;       // output gate: 0 = silu(z) (Qwen3.5), 1 = sigmoid(z) (Qwen4-exp option)
   int nk, nv, rep;
   float eps;
+  // states, slots and positions are settled: everything that wrote them completed before the launches began that may overlap this one
+  // (a step captured once in a graph of its own).  Only then are they read ahead of the dependency wait: the kernels of this library
+  // let their dependents start before they have waited themselves, so a launch may overlap several of those before it.
+  int settled;
 };
 
 // MINB = 2: the same kernel compiled for two resident CTAs per SM, used when a batch of rows
@@ -56,18 +60,18 @@ __global__ void __launch_bounds__(4 * DV, MINB) gdn_decode_kernel(const GdnDecod
   const int h = blockIdx.x, m = blockIdx.y, kh = h / a.rep;
   const int tid = threadIdx.x, j = tid % DV, grp = tid / DV;
   const int kdim = a.nk * DK, conv_dim = 2 * kdim + a.nv * DV;
+  griddep_launch();
+  if (!a.settled) griddep_wait();
   const int slot = a.slots[m];
   if (slot < 0) return;
   const int pos0 = a.positions[m];
 
-  // The recurrent state was written by this layer's previous step, long complete: fetch it
-  // before waiting for the projection kernel.
+  // a settled state is fetched before the projection kernel is waited for
   float* sp = a.state + (((int64_t)slot * a.nv + h) * DK + grp * RPT) * DV + j;
   float s[RPT];
-  griddep_launch();
 #pragma unroll
   for (int r = 0; r < RPT; ++r) s[r] = sp[(int64_t)r * DV];
-  griddep_wait();
+  if (a.settled) griddep_wait();
 
   const float nexpA = -__expf(a.A_log[h]), dtb = a.dt_bias[h];
   const float nw = a.norm_w[j];
@@ -180,6 +184,8 @@ __global__ void __launch_bounds__(4 * DV, 1) gdn_decode_stream_kernel(const GdnD
     for (int i = 0; i < ST; ++i) sm100::mbar_init(&full[i], 1);
     sm100::mbar_fence_init();
   }
+  griddep_launch();
+  if (!a.settled) griddep_wait();
   if (tid < 32) {                                   // rows that are in use, in order
     int n = 0;
     for (int m0 = 0; m0 < M; m0 += 32) {
@@ -199,13 +205,11 @@ __global__ void __launch_bounds__(4 * DV, 1) gdn_decode_stream_kernel(const GdnD
     sm100::mbar_expect_tx(&full[b], BYTES);
     sm100::bulk_load(bufs + (size_t)b * DK * DV, state_of(it), BYTES, &full[b]);
   };
-  griddep_launch();
-  // the states were written by this layer's previous step, long complete: two are requested before the projection kernel is waited for
-  if (tid == 0) {
+  if (tid == 0) {                                   // settled: two states are requested before the projection kernel is waited for
     if ((int)blockIdx.x < items) load(blockIdx.x, 0);
     if ((int)blockIdx.x + stride < items) load(blockIdx.x + stride, 1);
   }
-  griddep_wait();
+  if (a.settled) griddep_wait();
 
   // what one pair needs beside its state: a channel of the convolution per thread, z of its column, the head's scalars
   struct In { float4 w; bf16 x[4]; bf16 z, bl, al; float A, db; };
@@ -1501,11 +1505,12 @@ CB_EXPORT int cb_gdn_decode(const void* proj, int64_t ldp, const void* conv_w, c
                             const void* dt_bias, const void* norm_w, void* ring, void* state,
                             const void* slots, const void* positions, void* out, int64_t ldo,
                             void* record, int64_t rec_w, int64_t M, int64_t ntok, int64_t write_state,
-                            int64_t nk, int64_t nv, int64_t dk, int64_t dv, float eps, int64_t gate_sigmoid,
+                            int64_t nk, int64_t nv, int64_t dk, int64_t dv, float eps, int64_t gate_sigmoid, int64_t settled,
                             void* status, void* stream) {
   if (nv % nk || M < 1 || ntok < 1 || ntok > 12 || !status) return CB_ERR_SHAPE;
   GdnDecodeArgs a;
   a.gate_sigmoid = (int)gate_sigmoid;
+  a.settled = settled != 0;
   a.proj = (const bf16*)proj; a.ldp = ldp; a.conv_w = (const float*)conv_w; a.A_log = (const float*)A_log;
   a.dt_bias = (const float*)dt_bias; a.norm_w = (const float*)norm_w; a.ring = (bf16*)ring;
   a.state = (float*)state; a.slots = (const int*)slots; a.positions = (const int*)positions;

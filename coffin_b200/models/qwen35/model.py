@@ -738,7 +738,7 @@ class Qwen35Model:
                 K.gdn_decode(proj, lw.conv_w, lw.A_log, lw.dt_bias, lw.norm_w, self.ring[j], self.state[j],
                              b["slots"], b["positions"], act, nk=c.linear_num_key_heads,
                              nv=c.linear_num_value_heads, dk=c.linear_key_head_dim, dv=c.linear_value_head_dim,
-                             eps=self.eps)
+                             eps=self.eps, settled=K.capturing())
             else:
                 j = self.full_ids[li]
                 act = b["act_full"]
@@ -850,7 +850,7 @@ class Qwen35Model:
                 K.gdn_decode(proj, lw.conv_w, lw.A_log, lw.dt_bias, lw.norm_w, self.ring[j], self.state[j],
                              b["slots"], b["positions"], act, nk=c.linear_num_key_heads,
                              nv=c.linear_num_value_heads, dk=c.linear_key_head_dim, dv=c.linear_value_head_dim,
-                             eps=self.eps)
+                             eps=self.eps, settled=K.capturing())
             else:
                 j = self.full_ids[li]
                 act = b["act_full"]

@@ -567,7 +567,8 @@ class Qwen4ExpModel:
             K.gdn_decode(proj, L.conv_w, L.A_log, L.dt_bias, L.norm_w, self.ring[j], self.state[j], ws["one_slot"],
                          ws["one_pos"], act, ntok=T, record=ws["record"][j], write_state=False, **kw)
         elif slots is not None:
-            K.gdn_decode(proj, L.conv_w, L.A_log, L.dt_bias, L.norm_w, self.ring[j], self.state[j], slots, positions, act, **kw)
+            K.gdn_decode(proj, L.conv_w, L.A_log, L.dt_bias, L.norm_w, self.ring[j], self.state[j], slots, positions, act,
+                         settled=K.capturing(), **kw)
         else:
             K.gdn_prefill(proj, L.conv_w, L.A_log, L.dt_bias, L.norm_w, self.ring[j, slot], self.state[j, slot],
                           ws["gdn"], act, pos0=pos0, **kw)

@@ -50,6 +50,11 @@ def capture_graph(graph: "torch.cuda.CUDAGraph", pool=None):
             gc.enable()
 
 
+def capturing() -> bool:
+    """Whether the current launches go into a graph: a replay starts when everything enqueued before it has completed."""
+    return torch.cuda.is_current_stream_capturing()
+
+
 def _count(n: int = 1) -> None:
     global LAUNCHES
     LAUNCHES += n
@@ -630,12 +635,14 @@ def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: 
 # ------------------------------------------------------------------ gated delta net
 def gdn_decode(proj, conv_w, A_log, dt_bias, norm_w, ring, state, slots, positions, out, *, nk, nv, dk, dv,
                eps, ntok: int = 1, record: torch.Tensor | None = None, write_state: bool = True,
-               gate_sigmoid: bool = False) -> torch.Tensor:
+               gate_sigmoid: bool = False, settled: bool = False) -> torch.Tensor:
+    """``settled``: nothing that may still run when this launch starts has written ``state``, ``slots`` or ``positions`` (one step
+    in a captured graph of its own); they are then read ahead of the kernels before."""
     M = slots.numel()
     assert proj.shape[0] == M * ntok and slots.dtype == torch.int32 and positions.dtype == torch.int32
     call("gdn_decode", proj, proj.stride(0), conv_w, A_log, dt_bias, norm_w, ring, state, slots, positions,
          out, out.stride(0), record, record.shape[1] if record is not None else 0, M, ntok,
-         int(write_state), nk, nv, dk, dv, float(eps), int(gate_sigmoid), status_word(proj.device))
+         int(write_state), nk, nv, dk, dv, float(eps), int(gate_sigmoid), int(settled), status_word(proj.device))
     _count()
     return out
 

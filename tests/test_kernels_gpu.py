@@ -975,6 +975,44 @@ def test_gdn_decode_of_many_rows_is_that_of_few(nk, nv, M):
         assert torch.equal(st, s2) and torch.equal(ring, r2) and torch.equal(got, want), step
 
 
+@pytest.mark.parametrize("M", [4, 40])
+def test_gdn_decode_steps_that_follow_one_another(M):
+    """Steps enqueued back to back on one state, with nothing between them (the step before may still run when one starts), and a
+    commit of recorded tokens in front: the same bits as with the device waited for after every launch."""
+    k = K()
+    nk, nv, dk, ntok, steps = 16, 32, 128, 2, 12
+    g = torch.Generator().manual_seed(7)
+    _, conv_w, A_log, dt_bias, norm_w, conv_dim = _gdn_inputs(M, nk, nv, dk, dk, 96)
+    args = [t.to(DEV) for t in (conv_w, A_log, dt_bias, norm_w.float())]
+    kw = dict(nk=nk, nv=nv, dk=dk, dv=dk, eps=1e-6)
+    pjs = [_gdn_inputs(M, nk, nv, dk, dk, 100 + i)[0].to(DEV) for i in range(steps)]
+    pair = _gdn_inputs(M * ntok, nk, nv, dk, dk, 99)[0].to(DEV)
+    slots, pos = torch.randperm(M, generator=g).to(torch.int32).to(DEV), torch.zeros(M, dtype=torch.int32, device=DEV)
+    ring0 = torch.randn(M, k.RING, conv_dim, generator=g).bfloat16().to(DEV)
+    st0 = (0.1 * torch.randn(M, nv, dk, dk, generator=g)).to(DEV)
+    record = torch.zeros(M, ntok, nv * (2 * dk + 1), device=DEV)
+    accept = torch.full((M,), ntok, dtype=torch.int32, device=DEV)
+    at = [pos + ntok + i for i in range(steps)]
+    res = []
+    for wait in (True, False):
+        ring, st = ring0.clone(), st0.clone()
+        outs = [torch.zeros(M, nv * dk, dtype=torch.bfloat16, device=DEV) for _ in range(steps)]
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        torch.cuda.synchronize()
+        k.gdn_decode(pair, *args, ring, st, slots, pos, torch.empty(M * ntok, nv * dk, dtype=torch.bfloat16, device=DEV), ntok=ntok,
+                     record=record, write_state=False, **kw)
+        sync()
+        k.gdn_commit(st, record, slots, accept, nv=nv, dk=dk, dv=dk)
+        sync()
+        for i in range(steps):
+            k.gdn_decode(pjs[i], *args, ring, st, slots, at[i], outs[i], **kw)
+            sync()
+        torch.cuda.synchronize()
+        k.check_status()
+        res.append((ring, st, *outs))
+    assert all(torch.equal(x, y) for x, y in zip(*res))
+
+
 @pytest.mark.parametrize("E,N,Kd,swiglu,slots", [(6, 128, 256, True, 97), (5, 520, 2304, False, 200), (300, 24, 128, True, 512), (3, 2048, 512, False, 1024)])
 def test_moe_gemv_w4a8_by_expert(E, N, Kd, swiglu, slots, monkeypatch):
     """Experts taken whole (several passes of eight slots, experts without a slot, slots of other ranks, row and K remainders) against
