@@ -512,6 +512,13 @@ CB_EXPORT int cb_swiglu(const void* gu, void* out, int64_t M, int64_t I, int64_t
                         (const bf16*)gu, (bf16*)out, I, ldg, ldo, total);
 }
 
+// An ordinary launch with nothing to do: it starts when everything enqueued before it has completed, and so does whatever follows it.
+namespace { __global__ void settle_kernel() {} }
+CB_EXPORT int cb_settle(void* stream) {
+  settle_kernel<<<1, 1, 0, (cudaStream_t)stream>>>();
+  return (int)cudaGetLastError();
+}
+
 // scratch: cb_argmax_scratch_bytes(M) bytes, zero-initialised once by the caller.
 CB_EXPORT int64_t cb_argmax_scratch_bytes(int64_t M) { return M * (int64_t)sizeof(ArgmaxScratch); }
 

@@ -3,8 +3,9 @@
 //
 // The weights are the M operand of tcgen05.mma (128 rows of W a tile) and the activation rows its N operand (MT = 16, 32, 64
 // or 128 columns), so nothing is multiplied or staged for rows that do not exist beyond MT.
-//   warp 0   : TMA producer - [128 x 128 B] tiles of W and [MT x 128 B] tiles of A into a ring.  W does not depend on the
-//              kernel before this one: the first ring of W tiles is requested BEFORE the dependency wait, A's after it.  The ring
+//   warp 0   : TMA producer - [128 x 128 B] tiles of W and [MT x 128 B] tiles of A into a ring.  The first ring of W tiles is
+//              requested BEFORE the dependency wait, A's after it.  The launch may overlap the ones before it only where the caller
+//              says that W is resident, written long before; otherwise it is an ordinary launch, which starts after them.  The ring
 //              is small enough for two CTAs an SM, so that under programmatic dependent launch this projection's stream starts
 //              while the kernels ahead of it drain;
 //   warp 1   : MMA issuer;
@@ -350,7 +351,7 @@ int planned_slices(int64_t M, int64_t N, int64_t Kbytes, int narrowest) {
 }
 
 template <int MT, int STAGES, bool I8, bool SWIGLU>
-int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmA, const RowsArgs& a, int S, cudaStream_t st) {
+int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmA, const RowsArgs& a, int S, int resident, cudaStream_t st) {
   const size_t smem = (size_t)STAGES * (kRowsTile + MT) * kRowsKB + 16 * 128 * 4 + 1024;
   auto kern = gemm_rows_kernel<MT, STAGES, I8, SWIGLU>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -369,13 +370,14 @@ int launch_rows(const CUtensorMap& tmW, const CUtensorMap& tmA, const RowsArgs& 
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = g_cb_use_pdl ? 2 : 1;
+  cfg.numAttrs = g_cb_use_pdl && resident ? 2 : 1;
   if (g_cb_trace_names) cb_trace_name((const void*)kern);
   return (int)cudaLaunchKernelEx(&cfg, kern, tmW, tmA, a);
 }
 
 template <bool I8, bool SWIGLU>
-int rows_run(const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_rows, int64_t K, int fill, RowsArgs a, cudaStream_t st) {
+int rows_run(const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_rows, int64_t K, int fill, int resident, RowsArgs a,
+             cudaStream_t st) {
   constexpr int BK = I8 ? 128 : 64;
   const CUtensorMapDataType dt = I8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const int mt = a.M <= 16 ? 16 : (a.M <= 32 ? 32 : (a.M <= 64 ? 64 : 128));
@@ -400,10 +402,10 @@ int rows_run(const void* A, int64_t lda, const void* W, int64_t ldw, int64_t w_r
   rc = cb_make_tmap_2d(&tmA, dt, I8 ? 1 : 2, A, (uint64_t)a.M, (uint64_t)K, (uint64_t)lda, mt, BK);
   if (rc) return rc;
   a.n_tiles = (a.N + tn - 1) / tn;
-  if (mt == 16) return launch_rows<16, 5, I8, SWIGLU>(tmW, tmA, a, S, st);
-  if (mt == 32) return launch_rows<32, 5, I8, SWIGLU>(tmW, tmA, a, S, st);
-  if (mt == 64) return launch_rows<64, 4, I8, SWIGLU>(tmW, tmA, a, S, st);
-  return launch_rows<128, 3, I8, SWIGLU>(tmW, tmA, a, S, st);
+  if (mt == 16) return launch_rows<16, 5, I8, SWIGLU>(tmW, tmA, a, S, resident, st);
+  if (mt == 32) return launch_rows<32, 5, I8, SWIGLU>(tmW, tmA, a, S, resident, st);
+  if (mt == 64) return launch_rows<64, 4, I8, SWIGLU>(tmW, tmA, a, S, resident, st);
+  return launch_rows<128, 3, I8, SWIGLU>(tmW, tmA, a, S, resident, st);
 }
 
 int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, void* status,
@@ -421,40 +423,41 @@ int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M
 }  // namespace
 
 // C[M,N] = A[M,K] x W[N,K]^T, M <= 128; form 0: bf16 (+ residual), 1: fp32, 2: SwiGLU of the rows [0, N) and [N, 2N) of W, 3: the
-// same of gate and up rounded to bf16, as a product and cb_swiglu after it give it.  fill: K split to fill the machine, else by the plan of the batched products.
+// same of gate and up rounded to bf16, as a product and cb_swiglu after it give it.  fill: K split to fill the machine, else by the plan of the batched
+// products.  resident: no launch that may still run has written W.
 CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
-                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, void* status, void* stream) {
+                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, int64_t resident, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a) || K % 8) return CB_ERR_SHAPE;
-  if (form >= 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
-  return rows_run<false, false>(A, lda, W, ldw, N, K, fill != 0, a, (cudaStream_t)stream);
+  if (form >= 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, fill != 0, resident != 0, a, (cudaStream_t)stream);
+  return rows_run<false, false>(A, lda, W, ldw, N, K, fill != 0, resident != 0, a, (cudaStream_t)stream);
 }
 
 // The same from int8 rows and weights: (A_q x W_q^T) * row_scale[m] * col_scale[n], summed exactly.
 CB_EXPORT int cb_gemm_rows_i8(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
                               int64_t ldr, const void* row_scale, const void* col_scale, int64_t M, int64_t N, int64_t K, int64_t form,
-                              int64_t fill, void* status, void* stream) {
+                              int64_t fill, int64_t resident, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a)) return CB_ERR_SHAPE;
   if (K % 16 || lda % 16 || ldw % 16 || !row_scale || !col_scale) return CB_ERR_SHAPE;
   a.row_scale = (const float*)row_scale; a.col_scale = (const float*)col_scale;
-  if (form >= 2) return rows_run<true, true>(A, lda, W, ldw, 2 * N, K, fill != 0, a, (cudaStream_t)stream);
-  return rows_run<true, false>(A, lda, W, ldw, N, K, fill != 0, a, (cudaStream_t)stream);
+  if (form >= 2) return rows_run<true, true>(A, lda, W, ldw, 2 * N, K, fill != 0, resident != 0, a, (cudaStream_t)stream);
+  return rows_run<true, false>(A, lda, W, ldw, N, K, fill != 0, resident != 0, a, (cudaStream_t)stream);
 }
 
 // Forms of gemm_tc.cu's entry points for few rows (arguments checked there): xIELU in the epilogue; the columns from n_main on as
 // fp32 in C2.
 int cb_gemm_rows_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N, int64_t K,
-                       float act_a, float act_b, void* status, void* stream) {
+                       float act_a, float act_b, int64_t resident, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, nullptr, 0, M, N, K, 0, status, &a)) return CB_ERR_SHAPE;
   a.act = 1; a.act_a = act_a; a.act_b = act_b;
-  return rows_run<false, false>(A, lda, W, ldw, N, K, 0, a, (cudaStream_t)stream);
+  return rows_run<false, false>(A, lda, W, ldw, N, K, 0, resident != 0, a, (cudaStream_t)stream);
 }
 int cb_gemm_rows_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2, int64_t n_main,
-                       int64_t M, int64_t N, int64_t K, void* status, void* stream) {
+                       int64_t M, int64_t N, int64_t K, int64_t resident, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, nullptr, 0, M, N, K, 0, status, &a)) return CB_ERR_SHAPE;
   a.C2 = (float*)C2; a.ldc2 = ldc2; a.n_main = (int)n_main;
-  return rows_run<false, false>(A, lda, W, ldw, N, K, 0, a, (cudaStream_t)stream);
+  return rows_run<false, false>(A, lda, W, ldw, N, K, 0, resident != 0, a, (cudaStream_t)stream);
 }

@@ -290,11 +290,11 @@ int pick_bn(int M, int N, int sms, bool allow64) {
 
 // Products of at most 128 rows (gemm_rows.cu).
 int cb_gemm_rows_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N, int64_t K,
-                       float act_a, float act_b, void* status, void* stream);
+                       float act_a, float act_b, int64_t resident, void* status, void* stream);
 CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
-                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, void* status, void* stream);
+                                int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, int64_t resident, void* status, void* stream);
 int cb_gemm_rows_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2, int64_t n_main,
-                       int64_t M, int64_t N, int64_t K, void* status, void* stream);
+                       int64_t M, int64_t N, int64_t K, int64_t resident, void* status, void* stream);
 
 // CTA-pair kernel (gemm_tc2.cu): tile width it would use for [M, N], or 0 for "not this product".
 int cb_gemm_pair_plan(int64_t M, int64_t N);
@@ -343,9 +343,9 @@ CB_EXPORT int cb_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ld
 // C[M,N] = xIELU(A[M,K] x W[N,K]^T), bf16, with the coefficients (act_a, act_b) of its two branches: the activation is taken
 // in the epilogue.
 CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N,
-                                 int64_t K, float act_a, float act_b, void* status, void* stream) {
+                                 int64_t K, float act_a, float act_b, int64_t resident, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 8 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_xielu(A, lda, W, ldw, C, ldc, M, N, K, act_a, act_b, status, stream);
+  if (M <= BM) return cb_gemm_rows_xielu(A, lda, W, ldw, C, ldc, M, N, K, act_a, act_b, resident, status, stream);
   const int tile = cb_gemm_pair_plan(M, N);
   if (tile) return cb_gemm_pair_xielu(A, lda, W, ldw, C, ldc, M, N, K, tile, act_a, act_b, status, stream);
   const int sms = sm_count();
@@ -372,9 +372,9 @@ CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int6
 // One product, two results: columns [0, n_main) of A[M,K] x W[N,K]^T as bf16 in C, the others (gate pre-activations) as
 // fp32 in C2.  n_main % 8 == 0.
 CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2,
-                                 int64_t n_main, int64_t M, int64_t N, int64_t K, void* status, void* stream) {
+                                 int64_t n_main, int64_t M, int64_t N, int64_t K, int64_t resident, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 8 || ldc2 % 4 || n_main % 8 || n_main < 0 || n_main > N || !C2 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, status, stream);
+  if (M <= BM) return cb_gemm_rows_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, resident, status, stream);
   const int tile = cb_gemm_pair_plan(M, N);
   if (tile) return cb_gemm_pair_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, tile, status, stream);
   const int sms = sm_count();
@@ -401,9 +401,9 @@ CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int6
 // C[M,N] (fp32) = A[M,K] (bf16) x W[N,K]^T (bf16): the accumulator leaves unrounded (gate pre-activations of the
 // recurrent mixers, logits of many rows).  K % 8 == 0, N % 8 == 0, ldc % 4 == 0.
 CB_EXPORT int cb_gemm_bf16_f32out(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M,
-                                  int64_t N, int64_t K, void* status, void* stream) {
+                                  int64_t N, int64_t K, int64_t resident, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 4 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, 0, status, stream);
+  if (M <= BM) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, 0, resident, status, stream);
   const int sms = sm_count();
   const int bn = pick_bn((int)M, (int)N, sms, true);
   CUtensorMap tmA, tmB;

@@ -335,8 +335,7 @@ CB_EXPORT int cb_moe_gemv_w4(const void* Wq, const void* wscale, const void* x, 
 namespace {
 __global__ void __launch_bounds__(256) w4_dequant_kernel(const uint8_t* __restrict__ Wq, const float* __restrict__ scale,
                                                          bf16* __restrict__ out, int64_t N, int64_t K) {
-  // dependents are not launched early: the products that follow request the weights written here ahead of their own wait
-  cbtrace::stamp(0);
+  griddep_launch();
   griddep_wait();
   const int64_t half = K >> 1, G = K / kGroup;
   for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < N * (half >> 2); i += (int64_t)gridDim.x * 256) {

@@ -155,7 +155,7 @@ class LatentAttention(Mixer):
             if self._lent:
                 b.cache[key] = g
         kv = model.buf("kv", x["rows"], m.heads * (self.qd + self.vd))
-        K.gemm(g, self.w_kv, out=kv)
+        K.gemm(g, self.w_kv, out=kv, resident=True)
         split = m.heads * self.qd
         fl.set_pools(kv[:, :split], kv[:, split:])
         fl.flash(q, x["tables"], b.seg_row, x["pos"], None, None, segs=b.n_pre, max_rows=b.max_rows, positions=b.positions, act=act, gates=gates)

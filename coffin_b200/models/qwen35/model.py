@@ -110,6 +110,7 @@ class QW4:
         if kept is not None:
             return kept
         out = self.dequant()
+        K.settle()                      # products read weights ahead of the launches before them
         from .moe import keep_expansion
         if keep_expansion(out):
             self._kept = out
@@ -368,12 +369,12 @@ class Qwen35Model:
         owners instead of writing ``out`` (``_tp_finish`` completes the all-reduce)."""
         if isinstance(W, QW):
             q, sc = aq if aq is not None else K.quant_rows(A, swiglu=swiglu_in)     # aq: rows quantised by the producing kernel
-            return K.gemm_i8(q, sc, W.wq, W.scale, out=out, residual=residual, push=push)
+            return K.gemm_i8(q, sc, W.wq, W.scale, out=out, residual=residual, push=push, resident=True)
         if isinstance(W, QW4):
             W = W.expanded()                # bf16 copy (kept while HBM allows); the tcgen05 GEMM does the rest
         if swiglu_in:
             A = K.swiglu(A)
-        return K.gemm(A, W, out=out, residual=residual, push=push)
+        return K.gemm(A, W, out=out, residual=residual, push=push, resident=True)
 
     def _gemm_gu(self, A, W, gu: torch.Tensor, aq=None, decode: bool = False):
         """Gate|up projection of a prefill chunk or a wide decode bucket (``decode``) into ``gu [T, 2I]``.  The SwiGLU product
@@ -387,7 +388,7 @@ class Qwen35Model:
             if isinstance(W, QW):
                 q, sc = aq if aq is not None else K.quant_rows(A)
                 return K.gemm_i8_swiglu(q, sc, W.wq, W.scale, out=gu[:, :W.shape[0] // 2])
-            return K.gemm_swiglu(A, W, out=gu[:, :W.shape[0] // 2])
+            return K.gemm_swiglu(A, W, out=gu[:, :W.shape[0] // 2], resident=True)
         self._gemm(A, W, out=gu, aq=aq)
         return None
 

@@ -212,7 +212,7 @@ class MoEWeights:
         # (eight 8-row GEMV launches per layer were a fifth of a 64-row step)
         wide = T > 8
         if wide:
-            K.gemm(normed, self.router, out=b["logits"][:T])
+            K.gemm(normed, self.router, out=b["logits"][:T], resident=True)
         else:
             K.gemv(self.router, normed, b["logits"][:T])
         K.call("moe_router", b["logits"], b["logits"].stride(0), T, E, k, int(c.norm_topk_prob), b["idx"], b["w"],
@@ -232,8 +232,8 @@ class MoEWeights:
         shared = gate = None
         if self.sh_gu is not None:
             if wide:
-                K.gemm_swiglu(normed, self.sh_gu, out=b["sh_inter"][:T])
-                K.gemm(b["sh_inter"][:T], self.sh_down, out=b["sh_out"][:T])
+                K.gemm_swiglu(normed, self.sh_gu, out=b["sh_inter"][:T], resident=True)
+                K.gemm(b["sh_inter"][:T], self.sh_down, out=b["sh_out"][:T], resident=True)
             else:
                 K.gemv(self.sh_gu, normed, b["sh_inter"][:T], swiglu=True)
                 K.gemv(self.sh_down, b["sh_inter"][:T], b["sh_out"][:T])
@@ -263,7 +263,7 @@ class MoEWeights:
             if self.ep_world > 1:
                 out = model._tp_reduce(out)
             return out
-        logits = K.gemm(normed, self.router).float()                       # [T, pad8(E+1)]
+        logits = K.gemm(normed, self.router, resident=True).float()                       # [T, pad8(E+1)]
         idx = torch.empty(T, k, dtype=torch.int32, device=normed.device)
         w = torch.empty(T, k, dtype=torch.float32, device=normed.device)
         K.call("moe_router", logits, logits.stride(0), T, E, k, int(c.norm_topk_prob), idx, w, self.e_lo, self.e_hi)
@@ -298,8 +298,8 @@ class MoEWeights:
             y = K.gemm_grouped(inter, self._stack(self.down), disp)
         shared = gate = None
         if self.sh_gu is not None:
-            sh = K.gemm_swiglu(normed, self.sh_gu)
-            shared = K.gemm(sh, self.sh_down)
+            sh = K.gemm_swiglu(normed, self.sh_gu, resident=True)
+            shared = K.gemm(sh, self.sh_down, resident=True)
             gate = logits[:, E:].contiguous()
         out = torch.empty(T, H, dtype=torch.bfloat16, device=normed.device)
         K.call("moe_combine_pos", y, w, disp["pos"], shared, gate, gate.stride(0) if gate is not None else 0, out, T, H, k)

@@ -218,7 +218,7 @@ class VisionTower:
         N = patches.shape[0]
         nh, hd, H = c.num_heads, c.head_dim, c.hidden_size
         pos, cos, sin = self._geometry(grid)
-        x = K.gemm(patches.to(self.device, torch.bfloat16).contiguous(), self.patch_w, residual=self._bias(self.patch_b, N))
+        x = K.gemm(patches.to(self.device, torch.bfloat16).contiguous(), self.patch_w, residual=self._bias(self.patch_b, N), resident=True)
         x = x + pos
         npad = (N + 63) // 64 * 64
         table = torch.arange(npad // 64, dtype=torch.int32, device=self.device)
@@ -227,7 +227,7 @@ class VisionTower:
         use_kernel = hd in (64, 256)
         for b in self.blocks:
             y = self._layernorm(x, b["n1w"], b["n1b"])
-            qkv = K.gemm(y, b["qkv_w"], residual=self._bias(b["qkv_b"], N)).reshape(N, 3, nh, hd)
+            qkv = K.gemm(y, b["qkv_w"], residual=self._bias(b["qkv_b"], N), resident=True).reshape(N, 3, nh, hd)
             q = _rope(qkv[:, 0].float(), cos, sin).to(torch.bfloat16).contiguous()
             k = _rope(qkv[:, 1].float(), cos, sin).to(torch.bfloat16)
             if use_kernel:
@@ -238,14 +238,14 @@ class VisionTower:
             else:   # head widths the flash kernel has no instance for
                 att = torch.einsum("qhd,khd->hqk", q.float(), k.float()) * hd ** -0.5
                 o = torch.einsum("hqk,khd->qhd", att.softmax(-1), qkv[:, 2].float()).reshape(N, -1).to(torch.bfloat16)
-            x = K.gemm(o, b["proj_w"], residual=x + self._bias(b["proj_b"], N))
+            x = K.gemm(o, b["proj_w"], residual=x + self._bias(b["proj_b"], N), resident=True)
             y = self._layernorm(x, b["n2w"], b["n2b"])
-            y = self._gelu(K.gemm(y, b["fc1_w"], residual=self._bias(b["fc1_b"], N)))
-            x = K.gemm(y, b["fc2_w"], residual=x + self._bias(b["fc2_b"], N))
+            y = self._gelu(K.gemm(y, b["fc1_w"], residual=self._bias(b["fc1_b"], N), resident=True))
+            x = K.gemm(y, b["fc2_w"], residual=x + self._bias(b["fc2_b"], N), resident=True)
         m = c.spatial_merge_size ** 2
         y = self._layernorm(x, self.mn_w, self.mn_b).reshape(N // m, m * H)
-        y = F.gelu(K.gemm(y, self.m1_w, residual=self._bias(self.m1_b, N // m)).float()).to(torch.bfloat16)
-        return K.gemm(y, self.m2_w, residual=self._bias(self.m2_b, N // m))
+        y = F.gelu(K.gemm(y, self.m1_w, residual=self._bias(self.m1_b, N // m), resident=True).float()).to(torch.bfloat16)
+        return K.gemm(y, self.m2_w, residual=self._bias(self.m2_b, N // m), resident=True)
 
 
 # ----------------------------------------------------------------------------------------------

@@ -417,8 +417,8 @@ class Qwen4ExpModel:
                 return K.gemv_i8(W.wq, W.scale, x, out)
             qx, sc = K.quant_rows(x)
             if out.dtype == torch.bfloat16:
-                return K.gemm_i8(qx, sc, W.wq, W.scale, out=out)
-            out.copy_(K.gemm_i8(qx, sc, W.wq, W.scale))
+                return K.gemm_i8(qx, sc, W.wq, W.scale, out=out, resident=True)
+            out.copy_(K.gemm_i8(qx, sc, W.wq, W.scale, resident=True))
             return out
         if isinstance(W, QW4):
             if small:
@@ -427,8 +427,8 @@ class Qwen4ExpModel:
         if small:
             return K.gemv(W, x, out)
         if out.dtype == torch.bfloat16:
-            return K.gemm(x, W, out=out)
-        out.copy_(K.gemm(x, W))
+            return K.gemm(x, W, out=out, resident=True)
+        out.copy_(K.gemm(x, W, resident=True))
         return out
 
     def _embed(self, tokens: torch.Tensor) -> torch.Tensor:
@@ -500,15 +500,15 @@ class Qwen4ExpModel:
             self._linear(hw.Wd, normed, ws["low"])
             K.hyper_up(normed, ws["low"], hw.Wu, hw.Wi, ws["mixed"], inject_buf if hw.Wi is not None else None, H=H, hc=hc)
             return ws["mixed"], (inject_buf if hw.Wi is not None else None)
-        low = K.gemm(normed, hw.Wd)
+        low = K.gemm(normed, hw.Wd, resident=True)
         act = torch.nn.functional.silu(low.float() / hc).to(torch.bfloat16)
-        gate = torch.sigmoid(K.gemm(act, hw.Wu).float())
+        gate = torch.sigmoid(K.gemm(act, hw.Wu, resident=True).float())
         torch.mul(gate, normed.float(), out=gate)
         ws["mixed"].copy_(gate.view(T, hc, H).mean(1))
         K._count(4)
         inject = None
         if hw.Wi8 is not None:
-            inject_buf.copy_(2.0 * torch.sigmoid(K.gemm(normed, hw.Wi8)[:, :hc].float() / hc))
+            inject_buf.copy_(2.0 * torch.sigmoid(K.gemm(normed, hw.Wi8, resident=True)[:, :hc].float() / hc))
             inject = inject_buf
             K._count(1)
         return ws["mixed"], inject

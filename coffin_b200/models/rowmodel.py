@@ -248,8 +248,8 @@ class RowModel:
         if T <= 8 and T * Kd * 2 <= 160 * 1024:
             return K.gemv(W, x.contiguous(), out)
         if out.dtype == torch.float32:
-            return X.gemm_f32out(x, W, out)
-        return K.gemm(x, W, out=out)
+            return X.gemm_f32out(x, W, out, resident=True)
+        return K.gemm(x, W, out=out, resident=True)
 
     def project(self, P, h: torch.Tensor, b: RowBatch, name: str = "proj") -> tuple[torch.Tensor, torch.Tensor]:
         """``(main, gates)`` of an input projection, one product: fp32 for few rows (and in 32-bit mode), else the main columns
@@ -263,7 +263,7 @@ class RowModel:
         if P.n == P.n_main:
             return self.linear(P.w, h, main), main[:, P.n_main:]
         gates = self.buf("gates", T, P.gate.shape[0], torch.float32)
-        X.gemm_mixed(h, P.w, main, gates)
+        X.gemm_mixed(h, P.w, main, gates, resident=True)
         return main, gates
 
     def feed_forward(self, L, h: torch.Tensor, T: int) -> torch.Tensor:
@@ -278,7 +278,7 @@ class RowModel:
         elif K.PAIR_GEMM and T >= K.PAIR_MIN_ROWS and I >= 128:
             K.gemm_swiglu(h, L.w_gu, out=inter)
         else:
-            K.swiglu(K.gemm(h, L.w_gu, out=self.buf("gu", T, 2 * I)), out=inter)
+            K.swiglu(K.gemm(h, L.w_gu, out=self.buf("gu", T, 2 * I), resident=True), out=inter)
         return self.linear(L.w_down, inter, y)
 
     def angles(self, b: RowBatch, base: float, dims: int, turns: torch.Tensor) -> torch.Tensor:

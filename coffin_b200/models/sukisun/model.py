@@ -98,7 +98,7 @@ class SukisunModel(RowModel):
             pend = dict(y=self.linear(L.mixer.w_out, act, self.buf("y", T, L.mixer.w_out.shape[0])))
             if L.w_up is not None:
                 X.depth_step(x, plane, h, gain=L.gain2, eps=self.eps, **pend)
-                inter = X.linear_xielu(L.w_up, h, self.buf("inter", T, L.w_up.shape[0]), *L.act)
+                inter = X.linear_xielu(L.w_up, h, self.buf("inter", T, L.w_up.shape[0]), *L.act, resident=True)
                 pend = dict(y=self.linear(L.w_down, inter, self.buf("y", T, L.w_down.shape[0])))
             pend.update(weights=L.dwa, **L.plan)
             if self.layer_hook is not None:

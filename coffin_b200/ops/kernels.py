@@ -303,7 +303,7 @@ def gemv(W: torch.Tensor, x: torch.Tensor | None, out: torch.Tensor | None, *, s
     elif norm is not None and M >= NORM_SPLIT_ROWS and pull_site < 0:
         x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
     if x is not None and tpp is None and _rows_gemv_ok(W, x, out, M, N, K):
-        return _gemm_rows(x, W, out, form=2 if swiglu else int(f32), fill=True)
+        return _gemm_rows(x, W, out, form=2 if swiglu else int(f32), fill=True, resident=True)
     if GEMV_IMPL == "mma" and M * K * 2 <= 160 * 1024:
         call("gemv_mma_bf16", W, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
              pull_site, push_site)
@@ -349,7 +349,7 @@ def gemv_i8(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
                         quant=(torch.empty(M, K, dtype=torch.int8, device=Wq.device), torch.empty(M, dtype=torch.float32, device=Wq.device)))
         else:
             q = quant_rows(x)
-        return _gemm_rows_i8(*q, Wq, wscale, out, form=2 if swiglu else mode >> 1, fill=True)
+        return _gemm_rows_i8(*q, Wq, wscale, out, form=2 if swiglu else mode >> 1, fill=True, resident=True)
     if x is None and M >= NORM_SPLIT_ROWS and pull_site < 0:
         x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
     call("gemv_i8", Wq, wscale, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
@@ -427,6 +427,11 @@ def w4_dequant(Wq: torch.Tensor, wscale: torch.Tensor, out: torch.Tensor | None 
     call("w4_dequant", Wq, wscale, out, N, K)
     _count()
     return out
+
+
+def settle() -> None:
+    """What was enqueued before is complete when anything enqueued after this starts (launches of this library may overlap)."""
+    call("settle")
 
 
 def moe_dispatch(idx: torch.Tensor, n_experts: int, tile: int = 128) -> dict:
@@ -520,12 +525,13 @@ def quant_rows(x: torch.Tensor, swiglu: bool = False) -> tuple[torch.Tensor, tor
 
 
 def gemm(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor | None = None,
-         residual: torch.Tensor | None = None, bn: int = 0, push=None) -> torch.Tensor | None:
+         residual: torch.Tensor | None = None, bn: int = 0, push=None, resident: bool = False) -> torch.Tensor | None:
     """Prefill projection on tcgen05: ``out[M, N] = A[M, K] @ W[N, K]^T (+ residual)``, bf16.
 
     ``push`` (a ``parallel.tp.TpComm`` with a prefill region): nothing is written to ``out``; every
     output row stays in this rank's peer-visible buffer, from which the rank that owns it pulls it (first half of the fused
-    all-reduce; ``TpComm.finish_reduce`` is the second)."""
+    all-reduce; ``TpComm.finish_reduce`` is the second).  ``resident``: ``W`` was written long before, by nothing that may
+    still run (a model's weights); products of few rows then request it ahead of the launches before theirs."""
     M, K = A.shape
     N = W.shape[0]
     assert A.stride(1) == 1 and W.stride(1) == 1
@@ -538,7 +544,7 @@ def gemm(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor | None = None,
         out = torch.empty(M, N, dtype=torch.bfloat16, device=A.device)
     assert out.stride(1) == 1
     if M <= ROWS and bn == 0:
-        return _gemm_rows(A, W, out, residual, 1 if out.dtype == torch.float32 else 0)
+        return _gemm_rows(A, W, out, residual, 1 if out.dtype == torch.float32 else 0, resident=resident)
     call("gemm_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual,
          residual.stride(0) if residual is not None else 0, M, N, K, bn, None, 0, status_word(A.device))
     _count()
@@ -552,7 +558,7 @@ if not PAIR_GEMM:
     _lib.call_nostream("set_gemm_pair", 0)
 
 
-def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = None, resident: bool = False) -> torch.Tensor:
     """``out[M, I] = silu(A @ Wgu[:I]^T) * (A @ Wgu[I:]^T)``: the gate|up projection with the SwiGLU
     product taken in the GEMM epilogue (CTA-pair kernel; the even CTA of a pair stages gate rows, the
     odd one the matching up rows), so the ``[M, 2I]`` intermediate is never written.  Smaller products
@@ -564,9 +570,9 @@ def gemm_swiglu(A: torch.Tensor, Wgu: torch.Tensor, out: torch.Tensor | None = N
         out = torch.empty(M, I, dtype=torch.bfloat16, device=A.device)
     assert out.stride(1) == 1
     if M <= ROWS and I % 8 == 0:
-        return _gemm_rows(A, Wgu, out, form=3)
+        return _gemm_rows(A, Wgu, out, form=3, resident=resident)
     if not (PAIR_GEMM and M >= PAIR_MIN_ROWS and I >= 128):
-        return swiglu(gemm(A, Wgu), out=out)
+        return swiglu(gemm(A, Wgu, resident=resident), out=out)
     call("gemm_bf16_swiglu", A, A.stride(0), Wgu, Wgu.stride(0), out, out.stride(0), M, I, I, K, status_word(A.device))
     _count()
     return out
@@ -593,26 +599,26 @@ def gemm_i8_swiglu(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_
 ROWS = 128
 
 
-def _gemm_rows(A, W, out, residual=None, form: int = 0, fill: bool = False):
+def _gemm_rows(A, W, out, residual=None, form: int = 0, fill: bool = False, resident: bool = False):
     """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows,
     3: of the halves rounded to bf16.  ``fill``: slices
     of K that fill the machine (decode projections of two to eight rows), else those of the batched products, whose sums keep their order."""
     call("gemm_rows_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
-         A.shape[0], out.shape[1], A.shape[1], form, int(fill), status_word(A.device))
+         A.shape[0], out.shape[1], A.shape[1], form, int(fill), int(resident), status_word(A.device))
     _count()
     return out
 
 
-def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0, fill: bool = False):
+def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0, fill: bool = False, resident: bool = False):
     call("gemm_rows_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
-         a_scale, w_scale, Aq.shape[0], out.shape[1], Aq.shape[1], form, int(fill), status_word(Aq.device))
+         a_scale, w_scale, Aq.shape[0], out.shape[1], Aq.shape[1], form, int(fill), int(resident), status_word(Aq.device))
     _count()
     return out
 
 
 def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: torch.Tensor,
             out: torch.Tensor | None = None, residual: torch.Tensor | None = None, bn: int = 0,
-            push=None) -> torch.Tensor | None:
+            push=None, resident: bool = False) -> torch.Tensor | None:
     """W8A8 projection: int8 x int8 -> int32 on tcgen05 (kind::i8), ``* a_scale[m] * w_scale[n]``."""
     M, K = Aq.shape
     N = Wq.shape[0]
@@ -624,7 +630,7 @@ def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: 
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=Aq.device)
     if M <= ROWS and bn == 0:
-        return _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual, 1 if out.dtype == torch.float32 else 0)
+        return _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual, 1 if out.dtype == torch.float32 else 0, resident=resident)
     call("gemm_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual,
          residual.stride(0) if residual is not None else 0, a_scale, w_scale, M, N, K, bn, None, 0,
          status_word(Aq.device))

@@ -42,23 +42,23 @@ def _is_f32(t: torch.Tensor) -> int:
 
 
 # ------------------------------------------------------------------ projections
-def gemm_f32out(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
-    """``out[M, N] (fp32) = A[M, K] @ W[N, K]^T`` from bf16 operands on tcgen05, accumulator unrounded."""
+def gemm_f32out(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor, resident: bool = False) -> torch.Tensor:
+    """``out[M, N] (fp32) = A[M, K] @ W[N, K]^T`` from bf16 operands on tcgen05, accumulator unrounded.  ``resident``: as in ``kernels.gemm``."""
     M, Kd = A.shape
     N = W.shape[0]
     assert out.dtype == torch.float32 and out.stride(1) == 1 and A.stride(1) == 1 and W.stride(1) == 1
-    call("gemm_bf16_f32out", A, A.stride(0), W, W.stride(0), out, out.stride(0), M, N, Kd,
+    call("gemm_bf16_f32out", A, A.stride(0), W, W.stride(0), out, out.stride(0), M, N, Kd, int(resident),
          K.status_word(A.device))
     K._count()
     return out
 
 
-def gemm_mixed(A: torch.Tensor, W: torch.Tensor, main: torch.Tensor, gates: torch.Tensor) -> None:
+def gemm_mixed(A: torch.Tensor, W: torch.Tensor, main: torch.Tensor, gates: torch.Tensor, resident: bool = False) -> None:
     """One product ``A @ W^T``: its first columns rounded to bf16 in ``main``, the others unrounded in ``gates`` (fp32)."""
     M, Kd = A.shape
     N, n_main = W.shape[0], main.shape[1]
     assert gates.dtype == torch.float32 and gates.shape[1] == N - n_main and main.stride(1) == gates.stride(1) == A.stride(1) == 1
-    call("gemm_bf16_mixed", A, A.stride(0), W, W.stride(0), main, main.stride(0), gates, gates.stride(0), n_main, M, N, Kd,
+    call("gemm_bf16_mixed", A, A.stride(0), W, W.stride(0), main, main.stride(0), gates, gates.stride(0), n_main, M, N, Kd, int(resident),
          K.status_word(A.device))
     K._count()
 
@@ -80,7 +80,7 @@ def swiglu_f32(gu: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
     return out
 
 
-def linear_xielu(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor, a: float, b: float) -> torch.Tensor:
+def linear_xielu(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor, a: float, b: float, resident: bool = False) -> torch.Tensor:
     """``out = xielu(x @ W^T)``, ``xielu(z) = z / 2 + (a z^2 if z > 0 else b (exp(z) - 1 - z))``."""
     T, Kd = x.shape
     if out.dtype == torch.float32:
@@ -89,7 +89,7 @@ def linear_xielu(W: torch.Tensor, x: torch.Tensor, out: torch.Tensor, a: float, 
     elif T <= 8 and T * Kd * 2 <= 160 * 1024:
         call("gemv_mma_bf16_xielu", W, x.contiguous(), out, T, W.shape[0], Kd, out.stride(0), float(a), float(b))
     else:
-        call("gemm_bf16_xielu", x, x.stride(0), W, W.stride(0), out, out.stride(0), T, W.shape[0], Kd, float(a), float(b),
+        call("gemm_bf16_xielu", x, x.stride(0), W, W.stride(0), out, out.stride(0), T, W.shape[0], Kd, float(a), float(b), int(resident),
              K.status_word(x.device))
     K._count(2 if out.dtype == torch.float32 else 1)
     return out

@@ -868,6 +868,60 @@ def test_few_row_swiglu_is_the_product_and_swiglu_after_it(M, I, Kd):
         assert torch.equal(gu, k.gemm_i8(q, s, w.wq, w.scale))
 
 
+def test_few_row_products_of_weights_just_written():
+    """The second operand written by the launch right in front, or by the one before that, into a block that held other values: int4
+    expansions (resident after ``settle``, or not said to be resident), quantised rows, rows of another product."""
+    k = K()
+    from coffin_b200.ops import mixers as X
+    from coffin_b200.weights.quant import W4A8Weight
+    M, N, Kd, turns = 24, 4096, 2560, 6
+    A = bf(M, Kd, seed=1).to(DEV)
+    codes = [tuple(t.to(DEV) for t in W4A8Weight.quantize(bf(N, Kd, seed=10 + i).float() * 0.1).to_nk()) for i in range(turns)]
+    plain = [bf(N, Kd, seed=30 + i).to(DEV) for i in range(turns)]
+    near = [bf(N, 512, seed=50 + i).to(DEV) for i in range(turns)]
+    low = bf(Kd, 512, seed=70, s=0.05).to(DEV)
+    W, f32 = torch.empty(N, Kd, dtype=torch.bfloat16, device=DEV), torch.empty(M, N, device=DEV)
+    res = []
+    for wait in (True, False):
+        sync = torch.cuda.synchronize if wait else (lambda: None)
+        outs = []
+        for i in range(turns):
+            sync()
+            k.w4_dequant(*codes[i], out=W)
+            sync()
+            outs.append(k.gemm(A, W))
+            sync()
+            k.w4_dequant(*codes[-1 - i], out=W)
+            k.settle()
+            outs.append(k.gemm(A, W, resident=True))
+            sync()
+            q8 = k.quant_rows(plain[i])
+            a8 = k.quant_rows(A)
+            sync()
+            outs += [k.gemm_i8(*a8, *q8), k.gemm_i8_swiglu(*a8, *q8)]
+            sync()
+            k.gemm(near[i], low, out=W)
+            sync()
+            outs.append(X.gemm_f32out(A, W, f32).clone())
+            sync()
+            k.gemm(near[-1 - i], low, out=W)
+            sync()
+            outs.append(k.gemm_swiglu(A, W))
+            sync()
+            k.gemm(near[i], low, out=W)
+            sync()
+            outs.append(X.linear_xielu(W, A, torch.empty(M, N, dtype=torch.bfloat16, device=DEV), 0.8, 0.9))
+            main, gates = torch.empty(M, N - 64, dtype=torch.bfloat16, device=DEV), torch.empty(M, 64, device=DEV)
+            k.gemm(near[-1 - i], low, out=W)
+            sync()
+            X.gemm_mixed(A, W, main, gates)
+            outs += [main, gates]
+        torch.cuda.synchronize()
+        res.append(outs)
+    for i, (x, y) in enumerate(zip(*res)):
+        assert torch.equal(x, y), i
+
+
 @pytest.mark.parametrize("nk,nv,dk,lens", [(16, 32, 128, (1, 64, 65, 130, 300)), (16, 48, 128, (512, 127)), (2, 4, 64, (3, 200, 64))])
 def test_gdn_prefill_of_several_sequences(nk, nv, dk, lens):
     """One call over stacked sequences against one call each, bit for bit: chunk edges, a slot order of its own, rows before the
