@@ -98,13 +98,13 @@ def _row_family(name: str, cls: str) -> Callable:
 
 #: kernel sources a family needs; families without an entry use the whole library
 _KERNELS: dict[str, tuple[str, ...]] = {
-    "zufilorn": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemv_mma.cu", "gemm_f32.cu", "streams.cu",
+    "zufilorn": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemm_rows.cu", "gemv_mma.cu", "gemm_f32.cu", "streams.cu",
                  "linrec.cu", "linrec_chunk.cu", "attn_maps.cu", "attn_maps_flash.cu", "attn_maps_tc.cu"),
-    "sukisun": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemv_mma.cu", "gemm_f32.cu", "depth.cu", "linrec.cu", "ssd.cu",
+    "sukisun": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemm_rows.cu", "gemv_mma.cu", "gemm_f32.cu", "depth.cu", "linrec.cu", "ssd.cu",
                 "latent.cu", "rope.cu", "attn_maps.cu", "attn_maps_flash.cu", "attn_maps_tc.cu"),
-    "fasolorn": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemv_mma.cu", "gemm_f32.cu", "residual.cu", "routed.cu", "gemv_units.cu",
+    "fasolorn": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemm_rows.cu", "gemv_mma.cu", "gemm_f32.cu", "residual.cu", "routed.cu", "gemv_units.cu",
                  "moe.cu", "latent.cu", "rope.cu", "attn_maps.cu", "attn_maps_flash.cu", "attn_maps_tc.cu"),
-    "nodutar": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemv_mma.cu", "gemm_f32.cu", "residual.cu", "routed.cu", "gemv_units.cu",
+    "nodutar": ("elementwise.cu", "gemm_tc.cu", "gemm_tc2.cu", "gemm_rows.cu", "gemv_mma.cu", "gemm_f32.cu", "residual.cu", "routed.cu", "gemv_units.cu",
                 "moe.cu", "rope.cu", "linrec.cu", "linrec_chunk.cu", "attn_maps.cu", "attn_maps_flash.cu", "attn_maps_tc.cu"),
 }
 

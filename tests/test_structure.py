@@ -4,7 +4,10 @@ second backend (the reference keeps the same kind of gates in tests/test_backend
 tests/test_backends_purity.py)."""
 import ast
 import re
+import subprocess
 from pathlib import Path
+
+import pytest
 
 ROOT = Path(__file__).resolve().parents[1]
 PKG = ROOT / "coffin_b200"
@@ -126,3 +129,18 @@ def test_kernel_sources_are_built_for_sm_100a_only():
     src = (PKG / "_C" / "build.py").read_text()
     assert "arch=compute_100a,code=sm_100a" in src and "-lineinfo" in src
     assert not re.search(r"sm_(8\d|9\d)\b", src), "another architecture crept into the build flags"
+
+
+@pytest.mark.parametrize("arch", ["zufilorn", "sukisun", "fasolorn", "nodutar"])
+def test_library_of_one_family_resolves_what_it_uses(arch, tmp_path):
+    """A library of a family's kernel sources alone loads (no source refers to one that is left out) and exports the products of few
+    rows, of many and in 32 bits that every such family calls."""
+    import ctypes
+    from coffin_b200._C import build as B
+    from coffin_b200.models import kernel_sources
+    objs = [str(B._compile(s, False)[0]) for s in B.sources() if s.name in kernel_sources(arch)]
+    so = tmp_path / "family.so"
+    subprocess.run([B.nvcc(), *B.ARCH, "-shared", "-o", str(so), *objs], check=True)
+    lib = ctypes.CDLL(str(so))
+    for name in ("cb_gemm_rows_bf16", "cb_gemm_bf16", "cb_gemm_bf16_f32out", "cb_gemm_bf16_xielu", "cb_gemm_f32", "cb_gemv_mma_bf16", "cb_settle"):
+        assert hasattr(lib, name), name
