@@ -302,7 +302,7 @@ def gemv(W: torch.Tensor, x: torch.Tensor | None, out: torch.Tensor | None, *, s
         tpp = tp.cstruct_ref() if push_site >= 0 else None
     elif norm is not None and M >= NORM_SPLIT_ROWS and pull_site < 0:
         x, res_in, add, gain, res_out = _norm_rows(res_in, add, gain, res_out, eps), None, None, None, None
-    if x is not None and tpp is None and _rows_gemv_ok(W, x, out, M, N, K):
+    if x is not None and tpp is None and mode != 3 and _rows_gemv_ok(W, x, out, M, N, K):
         return _gemm_rows(x, W, out, form=2 if swiglu else int(f32), fill=True, resident=True)
     if GEMV_IMPL == "mma" and M * K * 2 <= 160 * 1024:
         call("gemv_mma_bf16", W, x, out, M, N, K, ldy, mode, N, res_in, add, gain, res_out, float(eps), tpp,
@@ -340,7 +340,7 @@ def gemv_i8(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
             x, res_in, add, gain, res_out = _pull_norm_rows(tp, pull_site, res_in, gain, res_out, eps), None, None, None, None
             pull_site = -1
             tpp = tp.cstruct_ref() if push_site >= 0 else None
-    if tpp is None and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K // 2):
+    if tpp is None and mode != 3 and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K // 2):
         # several rows: quantised once by a small kernel (the norm's own, where there is one), then the tcgen05 product
         if x is None:
             if add is None and res_out is not None and res_out.data_ptr() != res_in.data_ptr():
@@ -526,7 +526,8 @@ def quant_rows(x: torch.Tensor, swiglu: bool = False) -> tuple[torch.Tensor, tor
 
 def gemm(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor | None = None,
          residual: torch.Tensor | None = None, bn: int = 0, push=None, resident: bool = False) -> torch.Tensor | None:
-    """Prefill projection on tcgen05: ``out[M, N] = A[M, K] @ W[N, K]^T (+ residual)``, bf16.
+    """Prefill projection on tcgen05: ``out[M, N] = A[M, K] @ W[N, K]^T (+ residual)``, bf16.  An fp32 ``out`` takes the unrounded sums
+    (no residual).
 
     ``push`` (a ``parallel.tp.TpComm`` with a prefill region): nothing is written to ``out``; every
     output row stays in this rank's peer-visible buffer, from which the rank that owns it pulls it (first half of the fused
@@ -545,6 +546,11 @@ def gemm(A: torch.Tensor, W: torch.Tensor, out: torch.Tensor | None = None,
     assert out.stride(1) == 1
     if M <= ROWS and bn == 0:
         return _gemm_rows(A, W, out, residual, 1 if out.dtype == torch.float32 else 0, resident=resident)
+    if out.dtype == torch.float32:
+        assert residual is None and bn == 0, "an fp32 result takes no residual and no tile width"
+        call("gemm_bf16_f32out", A, A.stride(0), W, W.stride(0), out, out.stride(0), M, N, K, int(resident), status_word(A.device))
+        _count()
+        return out
     call("gemm_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual,
          residual.stride(0) if residual is not None else 0, M, N, K, bn, None, 0, status_word(A.device))
     _count()
@@ -599,19 +605,28 @@ def gemm_i8_swiglu(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_
 ROWS = 128
 
 
+def _rows_out(W, out, M: int, form: int) -> int:
+    """Columns of the result, which ``out`` has room for in the type that the kernel stores."""
+    N = W.shape[0] // 2 if form >= 2 else W.shape[0]
+    assert out.shape[0] >= M and out.shape[1] >= N and out.dtype == (torch.float32 if form == 1 else torch.bfloat16), (out.shape, out.dtype, form)
+    return N
+
+
 def _gemm_rows(A, W, out, residual=None, form: int = 0, fill: bool = False, resident: bool = False):
     """Form 0: ``A @ W^T (+ residual)`` in bf16, 1: the same in fp32, 2: SwiGLU of the two halves of ``W``'s rows,
     3: of the halves rounded to bf16.  ``fill``: slices
     of K that fill the machine (decode projections of two to eight rows), else those of the batched products, whose sums keep their order."""
+    N = _rows_out(W, out, A.shape[0], form)
     call("gemm_rows_bf16", A, A.stride(0), W, W.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
-         A.shape[0], out.shape[1], A.shape[1], form, int(fill), int(resident), status_word(A.device))
+         A.shape[0], N, A.shape[1], form, int(fill), int(resident), status_word(A.device))
     _count()
     return out
 
 
 def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0, fill: bool = False, resident: bool = False):
+    N = _rows_out(Wq, out, Aq.shape[0], form)
     call("gemm_rows_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual, residual.stride(0) if residual is not None else 0,
-         a_scale, w_scale, Aq.shape[0], out.shape[1], Aq.shape[1], form, int(fill), int(resident), status_word(Aq.device))
+         a_scale, w_scale, Aq.shape[0], N, Aq.shape[1], form, int(fill), int(resident), status_word(Aq.device))
     _count()
     return out
 
@@ -619,7 +634,8 @@ def _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual=None, form: int = 0, f
 def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: torch.Tensor,
             out: torch.Tensor | None = None, residual: torch.Tensor | None = None, bn: int = 0,
             push=None, resident: bool = False) -> torch.Tensor | None:
-    """W8A8 projection: int8 x int8 -> int32 on tcgen05 (kind::i8), ``* a_scale[m] * w_scale[n]``."""
+    """W8A8 projection: int8 x int8 -> int32 on tcgen05 (kind::i8), ``* a_scale[m] * w_scale[n]``.  An fp32 ``out``
+    takes the unrounded products of up to 128 rows."""
     M, K = Aq.shape
     N = Wq.shape[0]
     if push is not None:
@@ -631,6 +647,7 @@ def gemm_i8(Aq: torch.Tensor, a_scale: torch.Tensor, Wq: torch.Tensor, w_scale: 
         out = torch.empty(M, N, dtype=torch.bfloat16, device=Aq.device)
     if M <= ROWS and bn == 0:
         return _gemm_rows_i8(Aq, a_scale, Wq, w_scale, out, residual, 1 if out.dtype == torch.float32 else 0, resident=resident)
+    assert out.dtype == torch.bfloat16, "an int8 product of more than 128 rows leaves as bf16"
     call("gemm_i8", Aq, Aq.stride(0), Wq, Wq.stride(0), out, out.stride(0), residual,
          residual.stride(0) if residual is not None else 0, a_scale, w_scale, M, N, K, bn, None, 0,
          status_word(Aq.device))

@@ -868,6 +868,42 @@ def test_few_row_swiglu_is_the_product_and_swiglu_after_it(M, I, Kd):
         assert torch.equal(gu, k.gemm_i8(q, s, w.wq, w.scale))
 
 
+@pytest.mark.parametrize("M", [2, 128, 129, 300])
+def test_products_store_the_type_of_their_result(M):
+    """An fp32 result holds fp32 sums at any number of rows, a wider one keeps its other columns, and what has no such form is refused:
+    the SwiGLU projections of decode rows, int8 products of more than 128 rows, a residual."""
+    k = K()
+    N, Kd = 264, 512
+    A, W = bf(M, Kd, seed=1).to(DEV), bf(N, Kd, s=Kd ** -0.5, seed=2).to(DEV)
+    ref = A.double() @ W.double().t()
+    for out in (torch.full((M, N), 3.0, device=DEV), torch.full((M + 1, N + 8), 3.0, device=DEV)):
+        k.gemm(A, W, out=out)
+        assert ((out[:M, :N].double() - ref).norm() / ref.norm()).item() < 1e-5
+        assert bool((out[M:] == 3.0).all()) and bool((out[:, N:] == 3.0).all())
+    wide = torch.full((M, N + 8), 3.0, dtype=torch.bfloat16, device=DEV)
+    assert torch.equal(k.gemm(A, W, out=wide)[:, :N], k.gemm(A, W)) and bool((wide[:, N:] == 3.0).all())
+    f = torch.empty(M, N, device=DEV)
+    refused = (AssertionError, k._lib.KernelError)
+    with pytest.raises(refused):
+        k.gemm(A, W, out=f, residual=torch.zeros(M, N, dtype=torch.bfloat16, device=DEV))
+    q8, w8 = k.quant_rows(A), k.quant_rows(W)
+    if M > 128:
+        with pytest.raises(refused):
+            k.gemm_i8(*q8, *w8, out=f)
+    else:
+        with pytest.raises(refused):
+            k.gemm(A, W, out=wide[:, :N - 8])
+        k.gemm_i8(*q8, *w8, out=f)
+        want = (q8[0].double() @ w8[0].double().t()) * q8[1].double()[:, None] * w8[1].double()
+        assert ((f.double() - want).norm() / want.norm()).item() < 1e-6
+    if M <= 8:
+        half = torch.empty(M, N // 2, device=DEV)
+        with pytest.raises(refused):
+            k.gemv(W, A, half, swiglu=True)
+        with pytest.raises(refused):
+            k.gemv_i8(*w8, A, half, swiglu=True)
+
+
 def test_few_row_products_of_weights_just_written():
     """The second operand written by the launch right in front, or by the one before that, into a block that held other values: int4
     expansions (resident after ``settle``, or not said to be resident), quantised rows, rows of another product."""
