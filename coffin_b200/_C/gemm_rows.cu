@@ -199,11 +199,12 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (m >= a.M || n >= a.N) return;                // N is a multiple of 8
     if (I8) {
       const float rs = a.row_scale[m];
-      const float4 cs = *reinterpret_cast<const float4*>(a.col_scale + n);
+      const float* cp = a.col_scale + n;             // scales may start anywhere: no vector loads
+      const float4 cs = make_float4(cp[0], cp[1], cp[2], cp[3]);
       if (a.scale_rows_first) { v.x = v.x * rs * cs.x; v.y = v.y * rs * cs.y; v.z = v.z * rs * cs.z; v.w = v.w * rs * cs.w; }
       else { v.x *= rs * cs.x; v.y *= rs * cs.y; v.z *= rs * cs.z; v.w *= rs * cs.w; }
       if (SWIGLU) {
-        const float4 cu = *reinterpret_cast<const float4*>(a.col_scale + a.up_off + n);
+        const float4 cu = make_float4(cp[a.up_off], cp[a.up_off + 1], cp[a.up_off + 2], cp[a.up_off + 3]);
         u.x *= rs * cu.x; u.y *= rs * cu.y; u.z *= rs * cu.z; u.w *= rs * cu.w;
       }
     }
@@ -412,6 +413,7 @@ int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M
               RowsArgs* out) {
   if (M < 1 || M > kRowsTile || N < 1 || K < 1 || N % 8 || form < 0 || form > 3 || !C || !status) return CB_ERR_SHAPE;
   if (ldc % (form == 1 ? 4 : 8) || (residual && (ldr % 8 || form == 1))) return CB_ERR_SHAPE;
+  if (((uintptr_t)C & (form == 1 ? 15 : 7)) || ((uintptr_t)residual & 7)) return CB_ERR_SHAPE;      // results travel by fours
   RowsArgs a = {};
   a.C = C; a.ldc = ldc; a.residual = (const bf16*)residual; a.ldr = ldr; a.c_f32 = form == 1;
   a.round_halves = form == 3;
@@ -458,6 +460,7 @@ int cb_gemm_rows_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, v
                        int64_t M, int64_t N, int64_t K, int64_t resident, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, nullptr, 0, M, N, K, 0, status, &a)) return CB_ERR_SHAPE;
+  if ((uintptr_t)C2 & 15) return CB_ERR_SHAPE;
   a.C2 = (float*)C2; a.ldc2 = ldc2; a.n_main = (int)n_main;
   return rows_run<false, false>(A, lda, W, ldw, N, K, 0, resident != 0, a, (cudaStream_t)stream);
 }

@@ -340,7 +340,7 @@ def gemv_i8(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
             x, res_in, add, gain, res_out = _pull_norm_rows(tp, pull_site, res_in, gain, res_out, eps), None, None, None, None
             pull_site = -1
             tpp = tp.cstruct_ref() if push_site >= 0 else None
-    if tpp is None and mode != 3 and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K // 2):
+    if tpp is None and mode != 3 and K % 16 == 0 and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K):
         # several rows: quantised once by a small kernel (the norm's own, where there is one), then the tcgen05 product
         if x is None:
             if add is None and res_out is not None and res_out.data_ptr() != res_in.data_ptr():

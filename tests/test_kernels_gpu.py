@@ -904,6 +904,29 @@ def test_products_store_the_type_of_their_result(M):
             k.gemv_i8(*w8, A, half, swiglu=True)
 
 
+@pytest.mark.parametrize("M", [2, 8, 100])
+def test_int8_products_of_few_rows_take_scales_from_anywhere(M):
+    """Rows [1:] of a weight have their scales 4 bytes behind a vector's border, as slices of an int8 projection do."""
+    k = K()
+    N, Kd = 264, 512
+    A, W = bf(M, Kd, seed=1).to(DEV), bf(2 * N + 1, Kd, s=Kd ** -0.5, seed=2).to(DEV)
+    wq, ws = k.quant_rows(W)
+    a8 = k.quant_rows(A)
+    part, scale = wq[1:].contiguous(), ws[1:].clone()
+    torch.cuda.synchronize()
+    assert ws[1:].data_ptr() % 16 == 4
+    assert torch.equal(k.gemm_i8(*a8, part, ws[1:]), k.gemm_i8(*a8, part, scale))
+    assert torch.equal(k.gemm_i8_swiglu(*a8, part, ws[1:]), k.gemm_i8_swiglu(*a8, part, scale))
+    if M <= 8:
+        outs = [torch.empty(M, 2 * N, dtype=torch.bfloat16, device=DEV) for _ in range(2)]
+        assert torch.equal(*(k.gemv_i8(part, s, A, o) for s, o in zip((ws[1:], scale), outs)))
+        outs = [o[:, :N].contiguous() for o in outs]
+        assert torch.equal(*(k.gemv_i8(part, s, A, o, swiglu=True) for s, o in zip((ws[1:], scale), outs)))
+    off = torch.empty(M * N + 1, device=DEV)[1:].view(M, N)
+    with pytest.raises(k._lib.KernelError):          # results travel by fours
+        k.gemm(A, W[:N], out=off)
+
+
 def test_few_row_products_of_weights_just_written():
     """The second operand written by the launch right in front, or by the one before that, into a block that held other values: int4
     expansions (resident after ``settle``, or not said to be resident), quantised rows, rows of another product."""
