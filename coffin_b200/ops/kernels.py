@@ -248,7 +248,7 @@ def _norm_rows(res_in: torch.Tensor, add, gain: torch.Tensor, res_out, eps: floa
 
 def _rows_gemv_ok(W, x, out, M: int, N: int, K: int) -> bool:
     """Whether a decode projection of several rows takes the tcgen05 kernel."""
-    return (GEMV_IMPL == "mma" and M >= 2 and N % 8 == 0 and K % 8 == 0 and out.stride(0) % 8 == 0 and out.stride(1) == 1 and W.is_contiguous()
+    return (GEMV_IMPL == "mma" and 2 <= M <= 8 and N % 8 == 0 and K % 8 == 0 and out.stride(0) % 8 == 0 and out.stride(1) == 1 and W.is_contiguous()
             and (W.data_ptr() | x.data_ptr() | out.data_ptr()) % 16 == 0)
 
 

@@ -902,6 +902,12 @@ def test_products_store_the_type_of_their_result(M):
             k.gemv(W, A, half, swiglu=True)
         with pytest.raises(refused):
             k.gemv_i8(*w8, A, half, swiglu=True)
+    else:                                            # decode projections take up to eight rows
+        b = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        with pytest.raises(refused):
+            k.gemv(W, A, b)
+        with pytest.raises(refused):
+            k.gemv_i8(*w8, A, b)
 
 
 @pytest.mark.parametrize("M", [2, 8, 100])
