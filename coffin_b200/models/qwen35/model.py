@@ -660,7 +660,8 @@ class Qwen35Model:
         if b is None:
             c, dev, bf = self.cfg, self.device, torch.bfloat16
             H = c.hidden_size
-            nsplit = K.decode_splits(c.num_key_value_heads, M)
+            nsplit = K.decode_splits(c.num_key_value_heads, M, K.attn_shares_tiles(c.num_attention_heads, c.num_key_value_heads, c.head_dim,
+                                                                                   c.rotary_dim))
             b = {
                 "tokens": torch.zeros(M, dtype=torch.int64, device=dev),
                 "positions": torch.full((M,), -1, dtype=torch.int32, device=dev),

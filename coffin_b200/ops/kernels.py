@@ -837,16 +837,22 @@ def attn_decode(proj, qg, kg, cos, sin, positions, rope_pos, block_table, kpool,
     return out
 
 
-def decode_splits(nkv: int, rows: int) -> int:
+def decode_splits(nkv: int, rows: int, shared: bool = False) -> int:
     """Key-tile splits so that a decode attention launch (one 8-warp CTA per kv head, split and
-    row) covers about one wave of SMs.  Up to ``ATTN_SHARED_ROWS`` rows the batch kernel shares the tiles of all rows
-    among its CTAs; this is then the room for partials of one (row, kv head), for a row eight times as long as the average."""
+    row; from ``ATTN_BATCH_PAIRS`` pairs on two CTAs per SM) covers about one wave of SMs.  ``shared``: the launch is one that the batch
+    kernel takes (:func:`attn_shares_tiles`); up to ``ATTN_SHARED_ROWS`` rows it then shares the tiles of all rows among its CTAs, and
+    this is the room for partials of one (row, kv head), for a row eight times as long as the average."""
     pairs = max(1, nkv * rows)
     if pairs < ATTN_BATCH_PAIRS:
         return max(1, min(32, 148 // pairs))
-    if rows <= ATTN_SHARED_ROWS and 2 * pairs <= 296:
+    if shared and 0 < ATTN_BATCH_PAIRS and rows <= ATTN_SHARED_ROWS and 2 * pairs <= 296:
         return max(4, min(64, 2368 // pairs))
-    return max(1, min(32, 296 // pairs))             # tensor-core batch kernel: two 4-warp CTAs per SM
+    return max(1, min(32, 296 // pairs))
+
+
+def attn_shares_tiles(nh: int, nkv: int, hd: int, rot: int) -> bool:
+    """Whether :func:`attn_decode` has the tensor-core batch kernel for these heads (the condition of ``cb_attn_decode``)."""
+    return hd == 256 and (rot // 2) % 8 == 0 and nh // nkv <= 8
 
 
 ATTN_SHARED_ROWS = 8         # as in attn.cu

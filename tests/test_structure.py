@@ -144,3 +144,16 @@ def test_library_of_one_family_resolves_what_it_uses(arch, tmp_path):
     lib = ctypes.CDLL(str(so))
     for name in ("cb_gemm_rows_bf16", "cb_gemm_bf16", "cb_gemm_bf16_f32out", "cb_gemm_bf16_xielu", "cb_gemm_f32", "cb_gemv_mma_bf16", "cb_settle"):
         assert hasattr(lib, name), name
+
+
+def test_decode_attention_splits_cover_one_wave():
+    """CTAs of a decode attention launch: about one wave where the splits are the grid, room for partials only where the batch kernel shares
+    the tiles of few rows (heads of 256)."""
+    from coffin_b200.ops import kernels as K
+    for nkv in (1, 2, 4, 8, 16):
+        for rows in (1, 2, 4, 8, 16, 32, 64, 128):
+            pairs, ns = nkv * rows, K.decode_splits(nkv, rows)
+            assert ns == max(1, min(32, (148 if pairs < 32 else 296) // pairs))
+            few = 32 <= pairs <= 148 and rows <= 8
+            assert K.decode_splits(nkv, rows, True) == (min(64, 2368 // pairs) if few else ns)
+    assert K.attn_shares_tiles(16, 4, 256, 64) and not K.attn_shares_tiles(4, 2, 64, 16) and not K.attn_shares_tiles(64, 4, 256, 64)
