@@ -121,27 +121,34 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
   const int kb1 = a.kper ? min(a.k_blocks, kb0 + a.kper) : (int)((int64_t)a.k_blocks * (ks + 1) / S);
   const int wt = a.wt, tn = SWIGLU ? wt / 2 : wt;    // output columns of a tile
   const int cbits = __ffs(tn) - 3;                   // log2 of its groups of four columns
+  const int first = min(kb1 - kb0, STAGES);
+  auto load_w = [&](int tile, int kb, int s) {
+    unsigned char* st = ring + (size_t)s * STAGE_BYTES;
+    mbar_expect_tx(&full_bar[s], wt * kRowsKB + A_BYTES);
+    tma_load_2d(st, &tmW, &full_bar[s], kb * BK, tile * tn);
+    if (SWIGLU) tma_load_2d(st + tn * kRowsKB, &tmW, &full_bar[s], kb * BK, a.up_off + tile * tn);
+  };
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
     abort_s = 0;
     mbar_fence_init();
+    for (int i = 0; i < first; ++i) load_w(blockIdx.y, kb0 + i, i);
   }
+  // tensor memory is taken before dependents may start: one that took it first would hold it while it waits for this kernel
+  if (warp == 1) {
+    tmem_alloc(&tmem_base_s, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
   __syncthreads();
+  tc_fence_after();
   griddep_launch();
 
   if (warp == 0) {
     // ------------------------------- TMA producer -----------------------------------------
     if (lane == 0) {
-      auto load_w = [&](int tile, int kb, int s) {
-        unsigned char* st = ring + (size_t)s * STAGE_BYTES;
-        mbar_expect_tx(&full_bar[s], wt * kRowsKB + A_BYTES);
-        tma_load_2d(st, &tmW, &full_bar[s], kb * BK, tile * tn);
-        if (SWIGLU) tma_load_2d(st + tn * kRowsKB, &tmW, &full_bar[s], kb * BK, a.up_off + tile * tn);
-      };
       auto load_a = [&](int kb, int s) { tma_load_2d(ring + (size_t)s * STAGE_BYTES + W_BYTES, &tmA, &full_bar[s], kb * BK, 0); };
-      const int per = kb1 - kb0, first = min(per, STAGES);
-      for (int i = 0; i < first; ++i) load_w(blockIdx.y, kb0 + i, i);
       griddep_wait();
       for (int i = 0; i < first; ++i) load_a(kb0 + i, i);
       uint32_t it = 0;
@@ -156,13 +163,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
       }
     }
   } else {
-    if (warp == 1) {
-      tmem_alloc(&tmem_base_s, TMEM_COLS);
-      tmem_relinquish();
-    }
-    tc_fence_before();
-    asm volatile("bar.sync 2, 160;" ::: "memory");   // all but the producer, which is loading already
-    tc_fence_after();
     const uint32_t tmem_base = tmem_base_s;
     if (warp == 1) {
       // ------------------------------- MMA issuer -----------------------------------------
