@@ -366,19 +366,22 @@ CB_EXPORT int cb_w4_dequant(const void* Wq, const void* wscale, void* out, int64
 // The slot mode above reads an expert once per slot and quantises the slot's row in every CTA that shares it.  With 64 tokens of
 // eight slots over 256 experts (2.3 slots an expert in use) that is 2.3 passes over the int4 codes and a prologue of three block
 // reductions in front of each: 106 + 64 us a layer for 57 us of codes.  Here the rows are quantised once by a kernel of their own, a
-// CTA takes an expert, collects its slots and multiplies up to eight of them by every 16-row block it reads; codes and scales travel
-// one step ahead in registers.
+// CTA takes an expert and multiplies up to eight of its slots by every 16-row block it reads; codes and scales travel
+// one step ahead in registers.  An expert with more than eight slots has its other passes in CTAs of their own behind those of the
+// first passes (as many as the slots could ask for; each finds its expert and pass from a count of the slots, most find none), so
+// that the time does not grow with the most wanted expert.  Both products of a layer, 256 experts, 64 rows of eight slots: even
+// routing 102 -> 92 us (by slot 167), half the rows alike 226 -> 92 (by slot 152), two experts wanted by every row 358 -> 93 (by slot 165).
 namespace {
 
 struct MoeW4Args {
   const uint8_t* W; const float* wscale;
   const int8_t* xq; const int* asum; const float* xscale;   // [rows][K] (order of the kernel above), [rows][G], [rows]
   bf16* y;
-  int N, K, up_off, expert_rows, slots;
+  int N, K, up_off, expert_rows, slots, E;
   int64_t ldy;
   const int* slot_expert; const int* slot_xrow;
 };
-constexpr int kMaxSlots = 1024;
+constexpr int kMaxSlots = 1024, kMaxExperts = 2048;
 
 // One row per CTA: absmax scale, int8 values in the kernel's order, sums of the groups of 128.
 __global__ void __launch_bounds__(128) w4_quant_rows_kernel(const bf16* x, int64_t ldx, int8_t* xq, int* asum, float* xscale, int K) {
@@ -421,12 +424,13 @@ template <bool SWIGLU>
 __global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
   constexpr int PB = SWIGLU ? 2 : 1, U = SWIGLU ? 2 : 4;      // row blocks of a unit; groups of a step
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int K = a.K, G = K / kGroup, e = blockIdx.y;
+  const int K = a.K, G = K / kGroup;
   int8_t* xq = reinterpret_cast<int8_t*>(smem_raw);           // [8][K]
   int* asum = reinterpret_cast<int*>(smem_raw + (size_t)8 * K);   // [8][G]
   __shared__ float xscale[8];
-  __shared__ int list[kMaxSlots], cnt_s[kW];
+  __shared__ int list[8], cnt_s[kW], pick_s[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  int e = blockIdx.y, c0 = 0;                                 // expert and first of this pass's slots
   const uint8_t* W = a.W + (int64_t)e * a.expert_rows * (K >> 1);
   const float* ws = a.wscale + (int64_t)e * a.expert_rows * G;
   const int nblk = (a.N + 15) / 16, nb = (G + U - 1) / U, bstep = gridDim.x * kW, b0 = blockIdx.x * kW + warp;
@@ -447,8 +451,50 @@ __global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
   };
   griddep_launch();
   Step nxt;
-  if (b0 < nblk) load(nxt, b0, 0);                            // the weights do not depend on the routing
-  griddep_wait();
+  if (e < a.E) {
+    if (b0 < nblk) load(nxt, b0, 0);                          // the weights do not depend on the routing
+    griddep_wait();
+  } else {
+    // the (e - E)-th of the passes behind the first ones, experts in order
+    int* hist = reinterpret_cast<int*>(smem_raw);
+    griddep_wait();
+    for (int i = tid; i < a.E; i += kT) hist[i] = 0;
+    if (tid == 0) pick_s[0] = -1;
+    __syncthreads();
+    for (int i = tid; i < a.slots; i += kT) {
+      const int x = a.slot_expert[i];
+      if (x >= 0 && x < a.E) atomicAdd(&hist[x], 1);
+    }
+    __syncthreads();
+    const int own = (a.E + kT - 1) / kT, e0 = tid * own, e1 = min(a.E, e0 + own);
+    int more = 0;
+    for (int i = e0; i < e1; ++i) more += max(0, (hist[i] - 1) >> 3);
+    int upto = more;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    if (lane == 31) cnt_s[warp] = upto;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < kW; ++w) upto += w < warp ? cnt_s[w] : 0;
+    int o = e - a.E - (upto - more);                          // this pass among those of the thread's experts
+    if (o >= 0 && o < more)
+      for (int i = e0; i < e1; ++i) {
+        const int p = max(0, (hist[i] - 1) >> 3);
+        if (o < p) { pick_s[0] = i; pick_s[1] = o + 1; break; }
+        o -= p;
+      }
+    __syncthreads();
+    e = pick_s[0];
+    if (e < 0) return;
+    c0 = 8 * pick_s[1];
+    W = a.W + (int64_t)e * a.expert_rows * (K >> 1);
+    ws = a.wscale + (int64_t)e * a.expert_rows * G;
+    if (b0 < nblk) load(nxt, b0, 0);
+    __syncthreads();                                          // cnt_s is used again
+  }
   // ---- this expert's slots, in order ----------------------------------------------------------
   const int per = ((a.slots + kW - 1) / kW + 31) & ~31, s0 = warp * per;
   int mine = 0;
@@ -459,23 +505,24 @@ __global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
   int at = 0, count = 0;
 #pragma unroll
   for (int w = 0; w < kW; ++w) { at += w < warp ? cnt_s[w] : 0; count += cnt_s[w]; }
-  if (count == 0) return;
+  if (count <= c0) return;
   for (int i = s0; i < s0 + per && i < a.slots; i += 32) {
     const bool on = i + lane < a.slots && a.slot_expert[min(i + lane, a.slots - 1)] == e;
     const unsigned b = __ballot_sync(0xffffffffu, on);
-    if (on) list[at + __popc(b & ((1u << lane) - 1))] = i + lane;
+    const int pos = at + __popc(b & ((1u << lane) - 1)) - c0;
+    if (on && pos >= 0 && pos < 8) list[pos] = i + lane;
     at += __popc(b);
   }
-  for (int c0 = 0; c0 < count; c0 += 8) {
+  {
     const int M = min(8, count - c0);
-    __syncthreads();                                          // the list is complete; the rows before these are no longer read
+    __syncthreads();                                          // the list is complete
     for (int idx = tid; idx < M * (K >> 4); idx += kT) {
-      const int m = idx / (K >> 4), c = idx % (K >> 4), slot = list[c0 + m];
+      const int m = idx / (K >> 4), c = idx % (K >> 4), slot = list[m];
       const int64_t r = a.slot_xrow ? a.slot_xrow[slot] : slot;
       reinterpret_cast<uint4*>(xq + (size_t)m * K)[c] = reinterpret_cast<const uint4*>(a.xq + r * K)[c];
     }
     for (int idx = tid; idx < M * G; idx += kT) {
-      const int slot = list[c0 + idx / G];
+      const int slot = list[idx / G];
       const int64_t r = a.slot_xrow ? a.slot_xrow[slot] : slot;
       asum[idx] = a.asum[r * G + idx % G];
       if (idx % G == 0) xscale[idx / G] = a.xscale[r];
@@ -489,7 +536,6 @@ __global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
         const int gi = i * U;
         if (i + 1 < nb) load(nxt, blk, gi + U);
         else if (blk + bstep < nblk) load(nxt, blk + bstep, 0);
-        else if (c0 + 8 < count) load(nxt, b0, 0);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           if (gi + u >= G) break;
@@ -522,7 +568,7 @@ __global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
         if (m < M && row < a.N) {
           float v = acc[0][q] * xscale[m];
           if (SWIGLU) v = silu_f(v) * (acc[PB - 1][q] * xscale[m]);
-          a.y[(int64_t)list[c0 + m] * a.ldy + row] = __float2bfloat16(v);
+          a.y[(int64_t)list[m] * a.ldy + row] = __float2bfloat16(v);
         }
       }
     }
@@ -530,8 +576,8 @@ __global__ void __launch_bounds__(kT, 2) moe_w4_kernel(const MoeW4Args a) {
 }
 
 template <bool SWIGLU>
-int launch_moe_w4(const MoeW4Args& a, int E, cudaStream_t st) {
-  const size_t smem = (size_t)8 * a.K + (size_t)8 * (a.K / kGroup) * 4;
+int launch_moe_w4(const MoeW4Args& a, cudaStream_t st) {
+  const size_t smem = std::max((size_t)8 * a.K + (size_t)8 * (a.K / kGroup) * 4, (size_t)a.E * 4);
   auto kern = moe_w4_kernel<SWIGLU>;
   if (smem + 8192 > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -541,7 +587,7 @@ int launch_moe_w4(const MoeW4Args& a, int E, cudaStream_t st) {
   const int nblk = (a.N + 15) / 16;
   const unsigned gx = (unsigned)((nblk + 4 * kW - 1) / (4 * kW));
   const int64_t carve = std::min<int64_t>(100, (2 * (int64_t)(smem + 8192) * 100 + 228 * 1024 - 1) / (228 * 1024));
-  return (int)cb_launch_carve((int)carve, kern, dim3(gx, (unsigned)E), dim3(kT), smem, st, a);
+  return (int)cb_launch_carve((int)carve, kern, dim3(gx, (unsigned)(a.E + (a.slots - 1) / 8)), dim3(kT), smem, st, a);
 }
 }  // namespace
 
@@ -557,8 +603,8 @@ CB_EXPORT int cb_moe_gemv_w4_grouped(const void* Wq, const void* wscale, const v
                                      int64_t n_slots, int64_t E, int64_t N, int64_t K, int64_t ldy, int64_t swiglu, const void* slot_expert,
                                      const void* slot_xrow, void* stream) {
   if (!Wq || !wscale || !xq || !asum || !xscale || !y || !slot_expert) return CB_ERR_ARG;
-  if (K < kGroup || K % kGroup || K > 16384 || N < 1 || E < 1 || E > 65535 || n_slots < 1 || n_slots > kMaxSlots) return CB_ERR_SHAPE;
+  if (K < kGroup || K % kGroup || K > 16384 || N < 1 || E < 1 || E > kMaxExperts || n_slots < 1 || n_slots > kMaxSlots) return CB_ERR_SHAPE;
   MoeW4Args a{(const uint8_t*)Wq, (const float*)wscale, (const int8_t*)xq, (const int*)asum, (const float*)xscale, (bf16*)y, (int)N, (int)K,
-              (int)N, (int)(swiglu ? 2 * N : N), (int)n_slots, ldy, (const int*)slot_expert, (const int*)slot_xrow};
-  return swiglu ? launch_moe_w4<true>(a, (int)E, (cudaStream_t)stream) : launch_moe_w4<false>(a, (int)E, (cudaStream_t)stream);
+              (int)N, (int)(swiglu ? 2 * N : N), (int)n_slots, (int)E, ldy, (const int*)slot_expert, (const int*)slot_xrow};
+  return swiglu ? launch_moe_w4<true>(a, (cudaStream_t)stream) : launch_moe_w4<false>(a, (cudaStream_t)stream);
 }

@@ -1154,6 +1154,34 @@ def test_moe_gemv_w4a8_by_expert(E, N, Kd, swiglu, slots, monkeypatch):
         close(got, want, 2 ** -7)
 
 
+@pytest.mark.parametrize("E,T,kind", [(256, 33, "padded"), (256, 64, "wanted"), (600, 64, "padded"), (2, 128, "wanted"), (7, 9, "one")])
+def test_moe_gemv_w4a8_by_expert_of_uneven_routing(E, T, kind, monkeypatch):
+    """Passes of eight slots of one expert in CTAs of their own: the rows behind the last sequence all alike, experts that every row wants
+    (9, 64 and 65 slots), all slots on one expert, one after it; every slot's result that of the slot-wise kernel."""
+    k = K()
+    from coffin_b200.weights.quant import W4A8Weight
+    g = torch.Generator().manual_seed(E + T)
+    top = min(8, E)
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(T)]).to(torch.int32)
+    if kind == "padded":
+        idx[T // 2:] = idx[-1]
+    elif kind == "wanted":
+        idx[:, 0] = E - 1
+        idx[:min(T, 9), 1] = 0
+    else:
+        idx[:] = E - 2
+    N, Kd = 40, 256
+    wq, sc = (t.to(DEV) for t in W4A8Weight.quantize(torch.randn(E, N, Kd, generator=g) * 0.05).to_nk())
+    x = torch.randn(T, Kd, generator=g).bfloat16().to(DEV)
+    slots, rows = idx.reshape(-1).contiguous().to(DEV), torch.arange(T, dtype=torch.int32, device=DEV).repeat_interleave(top).contiguous()
+    want, got = (torch.full((T * top, N), 3.0, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    monkeypatch.setattr(k, "W4_GROUP_SHARE", 1 << 20)
+    k.moe_gemv_w4(wq, sc, x, want, slots, rows)
+    monkeypatch.setattr(k, "W4_GROUP_SHARE", 0)
+    k.moe_gemv_w4(wq, sc, x, got, slots, rows)
+    close(got, want, 2 ** -7)
+
+
 @pytest.mark.parametrize("M,nkv,nsplit", [(8, 4, 64), (9, 4, 1), (16, 2, 2), (70, 1, 9)])
 def test_decode_attention_of_rows_of_any_length(M, nkv, nsplit):
     """Tiles of all rows shared evenly (runs that start and end inside a row, whole pairs when there is room for one partial, padded
