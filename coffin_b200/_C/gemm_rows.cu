@@ -199,12 +199,14 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant_
     if (m >= a.M || n >= a.N) return;                // N is a multiple of 8
     if (I8) {
       const float rs = a.row_scale[m];
-      const float* cp = a.col_scale + n;             // scales may start anywhere: no vector loads
-      const float4 cs = make_float4(cp[0], cp[1], cp[2], cp[3]);
+      // scales may start anywhere (111 rows, 20176 x 544: 14.9 us with vector loads, 16.6 without)
+      const bool vec = ((uintptr_t)a.col_scale & 15) == 0;
+      auto scales = [&](const float* p) { return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]); };
+      const float4 cs = scales(a.col_scale + n);
       if (a.scale_rows_first) { v.x = v.x * rs * cs.x; v.y = v.y * rs * cs.y; v.z = v.z * rs * cs.z; v.w = v.w * rs * cs.w; }
       else { v.x *= rs * cs.x; v.y *= rs * cs.y; v.z *= rs * cs.z; v.w *= rs * cs.w; }
       if (SWIGLU) {
-        const float4 cu = make_float4(cp[a.up_off], cp[a.up_off + 1], cp[a.up_off + 2], cp[a.up_off + 3]);
+        const float4 cu = scales(a.col_scale + a.up_off + n);
         u.x *= rs * cu.x; u.y *= rs * cu.y; u.z *= rs * cu.z; u.w *= rs * cu.w;
       }
     }
@@ -331,7 +333,7 @@ int fill_slices(int64_t tiles, int64_t kb) {
 // tiles of 256, 128 or 64 rows of W and one CTA an SM, against what adding s partial tiles costs.  The slices are part of a product's
 // value: bf16 residuals and recurrent states carry a changed order of sums through all layers that follow (64 rows of the 32-layer
 // shape: half an rms at single elements of the states), so they stay as they are when kernels change.
-int planned_slices(int64_t M, int64_t N, int64_t Kbytes, int narrowest) {
+int planned_slices(int64_t M, int64_t N, int64_t Kbytes, int narrowest, int* width = nullptr) {
   const int64_t sms = rows_sms(), kb = (Kbytes + 127) / 128, K = Kbytes / 2;
   double best = 1e300;
   int64_t slices = 1;
@@ -346,7 +348,11 @@ int planned_slices(int64_t M, int64_t N, int64_t Kbytes, int narrowest) {
     const int64_t waves = (tiles * s + sms - 1) / sms;
     const double stream = (double)waves * (bn + M) * ((double)K / s) * 2.0 / 130e3;        // us at ~130 GB/s per SM
     const double cost = stream + (s > 1 ? (double)s * M * bn * 4.0 / 100e3 + 2.0 : 0.0);
-    if (cost < best) { best = cost; slices = s; }
+    if (cost < best) {
+      best = cost;
+      slices = s;
+      if (width) *width = bn;
+    }
   }
   return (int)slices;
 }
@@ -424,6 +430,18 @@ int rows_args(void* C, int64_t ldc, const void* residual, int64_t ldr, int64_t M
 
 }  // namespace
 
+// Width of the 128-row tiles that take a bf16 product instead of this kernel (0: this kernel takes it).  Above 64 rows the rows fill
+// such a tile, and an unsplit product has no partial tiles to save: 128 rows, 12352 x 2560 25.1 us here, 20.3 us there; 20000 x 1024 18.9
+// and 15.4 us; 72 rows, 40000 x 2560 51.7 and 50.6 us.  In slices it stays (128 rows, 4096 x 1024: 9.8 and 22.2 us).  The same sums.
+int cb_gemm_rows_tile(int64_t M, int64_t N, int64_t K) {
+  int bn = 256;
+  return M > 64 && M <= kRowsTile && planned_slices(M, N, K * 2, 64, &bn) == 1 ? bn : 0;
+}
+CB_EXPORT int cb_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual, int64_t ldr,
+                           int64_t M, int64_t N, int64_t K, int64_t bn, const void* pf, int64_t pf_seq, void* status, void* stream);
+CB_EXPORT int cb_gemm_bf16_f32out(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N,
+                                  int64_t K, int64_t resident, void* status, void* stream);
+
 // C[M,N] = A[M,K] x W[N,K]^T, M <= 128; form 0: bf16 (+ residual), 1: fp32, 2: SwiGLU of the rows [0, N) and [N, 2N) of W, 3: the
 // same of gate and up rounded to bf16, as a product and cb_swiglu after it give it.  fill: K split to fill the machine, else by the plan of the batched
 // products.  resident: no launch that may still run has written W.
@@ -431,6 +449,9 @@ CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64
                                 int64_t ldr, int64_t M, int64_t N, int64_t K, int64_t form, int64_t fill, int64_t resident, void* status, void* stream) {
   RowsArgs a;
   if (rows_args(C, ldc, residual, ldr, M, N, K, form, status, &a) || K % 8) return CB_ERR_SHAPE;
+  const int bn = form < 2 && !fill && !(((uintptr_t)C | (uintptr_t)residual) & 15) ? cb_gemm_rows_tile(M, N, K) : 0;
+  if (bn && form == 0) return cb_gemm_bf16(A, lda, W, ldw, C, ldc, residual, ldr, M, N, K, bn, nullptr, 0, status, stream);
+  if (bn) return cb_gemm_bf16_f32out(A, lda, W, ldw, C, ldc, M, N, K, resident, status, stream);
   if (form >= 2) return rows_run<false, true>(A, lda, W, ldw, 2 * N, K, fill != 0, resident != 0, a, (cudaStream_t)stream);
   return rows_run<false, false>(A, lda, W, ldw, N, K, fill != 0, resident != 0, a, (cudaStream_t)stream);
 }

@@ -288,7 +288,8 @@ int pick_bn(int M, int N, int sms, bool allow64) {
 
 }  // namespace
 
-// Products of at most 128 rows (gemm_rows.cu).
+// Products of at most 128 rows (gemm_rows.cu), but those that it leaves to the tiles here.
+int cb_gemm_rows_tile(int64_t M, int64_t N, int64_t K);
 int cb_gemm_rows_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N, int64_t K,
                        float act_a, float act_b, int64_t resident, void* status, void* stream);
 CB_EXPORT int cb_gemm_rows_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, const void* residual,
@@ -345,7 +346,7 @@ CB_EXPORT int cb_gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ld
 CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M, int64_t N,
                                  int64_t K, float act_a, float act_b, int64_t resident, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 8 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_xielu(A, lda, W, ldw, C, ldc, M, N, K, act_a, act_b, resident, status, stream);
+  if (M <= BM && (((uintptr_t)C & 15) || !cb_gemm_rows_tile(M, N, K))) return cb_gemm_rows_xielu(A, lda, W, ldw, C, ldc, M, N, K, act_a, act_b, resident, status, stream);
   const int tile = cb_gemm_pair_plan(M, N);
   if (tile) return cb_gemm_pair_xielu(A, lda, W, ldw, C, ldc, M, N, K, tile, act_a, act_b, status, stream);
   const int sms = sm_count();
@@ -374,7 +375,7 @@ CB_EXPORT int cb_gemm_bf16_xielu(const void* A, int64_t lda, const void* W, int6
 CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, void* C2, int64_t ldc2,
                                  int64_t n_main, int64_t M, int64_t N, int64_t K, int64_t resident, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 8 || ldc2 % 4 || n_main % 8 || n_main < 0 || n_main > N || !C2 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, resident, status, stream);
+  if (M <= BM && (((uintptr_t)C & 15) || !cb_gemm_rows_tile(M, N, K))) return cb_gemm_rows_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, resident, status, stream);
   const int tile = cb_gemm_pair_plan(M, N);
   if (tile) return cb_gemm_pair_mixed(A, lda, W, ldw, C, ldc, C2, ldc2, n_main, M, N, K, tile, status, stream);
   const int sms = sm_count();
@@ -403,7 +404,7 @@ CB_EXPORT int cb_gemm_bf16_mixed(const void* A, int64_t lda, const void* W, int6
 CB_EXPORT int cb_gemm_bf16_f32out(const void* A, int64_t lda, const void* W, int64_t ldw, void* C, int64_t ldc, int64_t M,
                                   int64_t N, int64_t K, int64_t resident, void* status, void* stream) {
   if (M < 1 || N < 1 || K < 1 || K % 8 || N % 8 || ldc % 4 || !status) return CB_ERR_SHAPE;
-  if (M <= BM) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, 0, resident, status, stream);
+  if (M <= BM && (((uintptr_t)C & 15) || !cb_gemm_rows_tile(M, N, K))) return cb_gemm_rows_bf16(A, lda, W, ldw, C, ldc, nullptr, 0, M, N, K, 1, 0, resident, status, stream);
   const int sms = sm_count();
   const int bn = pick_bn((int)M, (int)N, sms, true);
   CUtensorMap tmA, tmB;

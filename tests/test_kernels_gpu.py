@@ -832,7 +832,8 @@ def test_few_row_products(M, N, Kd):
 
 
 @pytest.mark.parametrize("M,N,Kd,kper", [(16, 2560, 4096, 22), (64, 2560, 9216, 21), (33, 264, 2048, 4), (64, 12352, 2560, 40), (9, 2048, 512, 4),
-                                         (100, 1032, 4104, 9), (64, 2048, 4096, 16)])
+                                         (100, 1032, 4104, 9), (64, 2048, 4096, 16),
+                                         (65, 12352, 520, 9), (128, 20000, 1024, 16)])
 def test_few_row_products_keep_the_order_of_their_sums(M, N, Kd, kper):
     """Slices of ``kper`` k-blocks of 64, each summed along K and added in order, bit for bit: a slice by itself is a product of more than
     128 rows, which is not split.  (What follows in a model carries every change of rounding through all layers.)"""
