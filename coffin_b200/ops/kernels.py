@@ -246,10 +246,23 @@ def _norm_rows(res_in: torch.Tensor, add, gain: torch.Tensor, res_out, eps: floa
     return buf
 
 
-def _rows_gemv_ok(W, x, out, M: int, N: int, K: int) -> bool:
+def _rows_gemv(M: int, N: int, K: int, i8: bool) -> bool:
+    """Whether a decode projection of ``M`` rows takes the tcgen05 kernel, by size: it splits K over a cluster, which pays from a length on.
+    us of the GEMV / of that kernel, 2 rows: 512 x 1024 4.0 / 4.9, 4096 x 1024 4.9 / 6.4, 4096 x 1536 7.9 / 7.3, 16384 x 1024 10.5 / 10.4;
+    8 rows: 4096 x 1024 6.0 / 6.4, 4096 x 1536 8.9 / 7.6.  int8 rows are quantised by a launch of their own, 2 us: 2 rows, 4096 x 4096
+    9.6 / 11.5, 5120 x 6144 14.5 / 13.6, 50000 x 1024 15.5 / 15.6; 4 rows: 4096 x 1024 6.9 / 8.4, 16384 x 2560 17.5 / 15.1; 5 rows:
+    4096 x 2560 11.7 / 10.2."""
+    if not 2 <= M <= 8:
+        return False
+    if i8:
+        return M >= 5 or K > 4096 or N * K * M * M >= 200_000_000
+    return K > 1024 or N >= 16384
+
+
+def _rows_gemv_ok(W, x, out, M: int, N: int, K: int, i8: bool = False) -> bool:
     """Whether a decode projection of several rows takes the tcgen05 kernel."""
-    return (GEMV_IMPL == "mma" and 2 <= M <= 8 and N % 8 == 0 and K % 8 == 0 and out.stride(0) % 8 == 0 and out.stride(1) == 1 and W.is_contiguous()
-            and (W.data_ptr() | x.data_ptr() | out.data_ptr()) % 16 == 0)
+    return (GEMV_IMPL == "mma" and _rows_gemv(M, N, K, i8) and N % 8 == 0 and K % 8 == 0 and out.stride(0) % 8 == 0 and out.stride(1) == 1
+            and W.is_contiguous() and (W.data_ptr() | x.data_ptr() | out.data_ptr()) % 16 == 0)
 
 
 def gemv(W: torch.Tensor, x: torch.Tensor | None, out: torch.Tensor | None, *, swiglu: bool = False,
@@ -340,7 +353,7 @@ def gemv_i8(Wq: torch.Tensor, wscale: torch.Tensor, x: torch.Tensor | None, out:
             x, res_in, add, gain, res_out = _pull_norm_rows(tp, pull_site, res_in, gain, res_out, eps), None, None, None, None
             pull_site = -1
             tpp = tp.cstruct_ref() if push_site >= 0 else None
-    if tpp is None and mode != 3 and K % 16 == 0 and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K):
+    if tpp is None and mode != 3 and K % 16 == 0 and _rows_gemv_ok(Wq, x if x is not None else res_in, out, M, N, K, True):
         # several rows: quantised once by a small kernel (the norm's own, where there is one), then the tcgen05 product
         if x is None:
             if add is None and res_out is not None and res_out.data_ptr() != res_in.data_ptr():

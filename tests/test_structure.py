@@ -157,3 +157,14 @@ def test_decode_attention_splits_cover_one_wave():
             few = 32 <= pairs <= 148 and rows <= 8
             assert K.decode_splits(nkv, rows, True) == (min(64, 2368 // pairs) if few else ns)
     assert K.attn_shares_tiles(16, 4, 256, 64) and not K.attn_shares_tiles(4, 2, 64, 16) and not K.attn_shares_tiles(64, 4, 256, 64)
+
+
+def test_decode_projections_of_several_rows_by_size():
+    """Short sums stay on the GEMV, long ones and wide weights take the products of few rows (sizes at which both were measured)."""
+    from coffin_b200.ops.kernels import _rows_gemv
+    for M in range(2, 9):
+        assert not _rows_gemv(M, 4096, 1024, False) and not _rows_gemv(M, 256, 256, False)
+        assert _rows_gemv(M, 512, 1536, False) and _rows_gemv(M, 16384, 1024, False)
+        assert _rows_gemv(M, 5120, 6144, True) and _rows_gemv(M, 152064, 5120, True)
+    assert not _rows_gemv(4, 4096, 1024, True) and not _rows_gemv(2, 4096, 4096, True) and _rows_gemv(5, 4096, 1024, True)
+    assert not _rows_gemv(1, 16384, 4096, False) and not _rows_gemv(9, 16384, 4096, True)
