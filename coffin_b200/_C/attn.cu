@@ -719,15 +719,18 @@ __global__ void __launch_bounds__(kDecWarps * 32, MINB) attn_decode_kernel(const
 // one is used), keep their own running maximum and sum, and merge once at the end.  Query / key
 // normalisation, rotary embedding, the KV append of the current token and the sigmoid output gate are
 // part of the kernel as in the single-sequence one.
+// Q8 (int8 pages): a thread holds its share of the next tile's bytes in registers while the one before is multiplied, and converts them
+// into the ring.  Converted where they were loaded, 64 rows of 1100 tokens took 337 us, with K and V loaded together and waited for
+// 219 us, so 93 us.
 //
 // Wide batches (more than kSharedRows rows): every (row, kv head) has a.nsplit CTAs, which take its tiles in turn.  A row's sums
 // do not depend on the other rows' lengths.  Rows of 1 to 2560 tokens, 4 kv heads, against tiles staged with cp.async and waited for:
-// 16 rows 38.9 -> 33.3 us, 32 rows 69 -> 49 us, 64 rows 114 -> 75 us.
+// 16 rows 38.9 -> 33.3 us, 32 rows 69 -> 49 us, 64 rows 114 -> 75 us; 16 rows of 65 tokens 11.9 -> 12.9 us.
 // SHARED (few rows): the tiles of all rows are shared out by length, a pair cut into runs of adjacent tiles.  With equal splits a
-// row, the SMs with the long rows set the time (8 rows of 517 to 16391 tokens 97 -> 61 us; 64 rows of 1031 to 2047, with runs that
+// row, the SMs with the long rows set the time (8 rows of 517 to 16391 tokens 97 -> 61 us, of 300 tokens each 12.9 -> 14.0 us; 64 rows of 1031 to 2047, with runs that
 // also crossed rows, 98 -> 90 us only, and their results moved with their neighbours).
 constexpr int kSharedRows = 8, kSharedCtas = 296;
-template <int HD, bool SHARED>
+template <int HD, bool SHARED, bool Q8>
 __global__ void __launch_bounds__(128, 2)
 attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const DecodeArgs a, int rows) {
   constexpr int LD = HD + 8, EPL = HD / 32, CPR = HD / 8;
@@ -745,13 +748,16 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   __shared__ float mm_s[4][8], ml_s[4][8];
   __shared__ float linv_s[8];
   __shared__ bool is_last;
-  __shared__ int pre_s[kSharedRows + 1];
   __shared__ uint64_t full[3];
   const int rep = a.nh / a.nkv;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
   if (tid == 0) {
     for (int i = 0; i < 3; ++i) sm100::mbar_init(&full[i], 1);
     sm100::mbar_fence_init();
+    if (!Q8) {
+      sm100::tma_prefetch_desc(&tmK);
+      sm100::tma_prefetch_desc(&tmV);
+    }
   }
   griddep_launch();
   griddep_wait();
@@ -759,26 +765,22 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   if (SHARED) {
     // every pair is cut into runs of at most `per` tiles (a CTA pays one prologue and one merge, about 15 us with what surrounds
     // them); its partials have room for a.nsplit runs
-    if (warp == 0) {
-      const int pairs = rows * a.nkv, n = lane < rows ? a.positions[lane] : -1, nt = n < 0 ? 0 : n / kBlock + 1;   // a padded row has none
-      const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)nt) * a.nkv, most = (int)__reduce_max_sync(0xffffffffu, (unsigned)nt);
-      const int per = max((sum + kSharedCtas - pairs - 1) / (kSharedCtas - pairs), (most + a.nsplit - 1) / a.nsplit);
-      int runs = per ? (nt + per - 1) / per : 0;
+    const int pairs = rows * a.nkv, n = lane < rows ? a.positions[lane] : -1, tiles = n < 0 ? 0 : n / kBlock + 1;   // a padded row has none
+    const int sum = (int)__reduce_add_sync(0xffffffffu, (unsigned)tiles) * a.nkv, most = (int)__reduce_max_sync(0xffffffffu, (unsigned)tiles);
+    const int per = max((sum + kSharedCtas - pairs - 1) / (kSharedCtas - pairs), (most + a.nsplit - 1) / a.nsplit);
+    const int runs = per ? (tiles + per - 1) / per : 0;
+    int upto = runs;                              // runs of the rows up to this one, per kv head
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, runs, o);
-        if (lane >= o) runs += y;
-      }
-      if (lane < rows) pre_s[lane + 1] = runs;    // runs of the rows up to this one, per kv head
-      if (lane == 0) pre_s[0] = 0;
+    for (int o = 1; o < kSharedRows; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
     }
-    __syncthreads();
     const int u = blockIdx.x;
-    if (u >= pre_s[rows] * a.nkv) return;
-    m = 0;
-    while (pre_s[m + 1] * a.nkv <= u) ++m;
-    nsplit = pre_s[m + 1] - pre_s[m];
-    const int at = u - pre_s[m] * a.nkv, nt = a.positions[m] / kBlock + 1;
+    const unsigned later = __ballot_sync(0xffffffffu, lane < rows && upto * a.nkv > u);
+    if (!later) return;
+    m = __ffs(later) - 1;                         // the row of run u
+    nsplit = __shfl_sync(0xffffffffu, runs, m);
+    const int nt = __shfl_sync(0xffffffffu, tiles, m), at = u - (__shfl_sync(0xffffffffu, upto, m) - nsplit) * a.nkv;
     kvh = at / nsplit;
     split = at % nsplit;
     t0 = nt * split / nsplit;
@@ -799,20 +801,21 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
   const float* sn = a.sin + (int64_t)rp * a.rot;
   const int* bt = a.block_table + (int64_t)m * a.ldbt;
   // half h of this run: the K (even) or V (odd) tile of its tile h / 2.  One thread asks for a bf16 tile (16 cp.async a thread, or a
-  // bulk copy a row, took longer than the products), int8 rows are converted on the way.
+  // bulk copy a row, took longer than the products); int8 rows arrive in registers and convert_half puts them into the ring.
+  uint2 raw[Q8 ? 16 : 1];
+  float rsc = 0.f;
   auto load_half = [&](int h) {
     if (h >= 2 * cnt) return;
     const int64_t slot0 = (int64_t)bt[t0 + (h >> 1) * step] * kBlock;
     const int at = h % 3;
     bf16* dst = ring + at * TILE;
-    if (a.kscale) {
+    if (Q8) {
       const int8_t* pool = reinterpret_cast<const int8_t*>((h & 1) ? a.vpool : a.kpool);
       const float* scale = (h & 1) ? a.vscale : a.kscale;
-      for (int idx = tid; idx < 64 * CPR; idx += 128) {
-        const int r = idx / CPR, c = idx % CPR;
-        const int64_t row = (slot0 + r) * a.nkv + kvh;
-        *reinterpret_cast<uint4*>(dst + piece(r, c)) = q8x8_to_bf16x8(*reinterpret_cast<const uint2*>(pool + row * HD + c * 8), scale[row]);
-      }
+      const int64_t row = (slot0 + warp) * a.nkv + kvh, next = 4 * (int64_t)a.nkv;       // warp w: rows w, w + 4, ..
+#pragma unroll
+      for (int j = 0; j < 16; ++j) raw[j] = *reinterpret_cast<const uint2*>(pool + (row + j * next) * HD + lane * 8);
+      rsc = lane < 16 ? scale[row + lane * next] : 0.f;
     } else if (tid == 0) {
       sm100::mbar_expect_tx(&full[at], TILE * 2);
 #pragma unroll
@@ -820,9 +823,16 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
         sm100::tma_load_2d(dst + c * 64 * 64, (h & 1) ? &tmV : &tmK, &full[at], kvh * HD + c * 64, (int)slot0);
     }
   };
-  auto arrived = [&](int h) { return a.kscale || sm100::mbar_wait(&full[h % 3], (h / 3) & 1); };
+  auto convert_half = [&](int h) {
+    if (!Q8 || h >= 2 * cnt) return;
+    bf16* dst = ring + (h % 3) * TILE;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      *reinterpret_cast<uint4*>(dst + piece(warp + 4 * j, lane)) = q8x8_to_bf16x8(raw[Q8 ? j : 0], __shfl_sync(0xffffffffu, rsc, j));
+  };
+  auto arrived = [&](int h) { return Q8 || sm100::mbar_wait(&full[h % 3], (h / 3) & 1); };
   load_half(0);
-  load_half(1);
+  if (!Q8) load_half(1);
   // ---- prologue: q heads -> Qs (bf16), this token's K / V -> pool and shared copies ---------------
   for (int idx = tid; idx < 16 * CPR; idx += 128)
     *reinterpret_cast<uint4*>(Qs + (idx / CPR) * LD + (idx % CPR) * 8) = make_uint4(0, 0, 0, 0);
@@ -843,7 +853,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 #pragma unroll
         for (int e = 0; e < EPL; ++e) x[e] = __bfloat162float(src[e]);
         norm_rope_lane<HD>(x, a.kg, cs, sn, a.rot, a.eps, lane);
-        if (a.kscale) {            // the shared copy holds the dequantised row, what later steps will read
+        if (Q8) {                  // the shared copy holds the dequantised row, what later steps will read
           const float sc = quant_row_q8<EPL>(x, reinterpret_cast<int8_t*>(a.kpool) + (slot * a.nkv + kvh) * HD, lane);
           if (lane == 0) a.kscale[slot * a.nkv + kvh] = sc;
 #pragma unroll
@@ -855,7 +865,7 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
         }
       } else {
         const bf16* src = prow + (int64_t)a.nh * 2 * HD + (int64_t)(a.nkv + kvh) * HD + lane * EPL;
-        if (a.vscale) {
+        if (Q8) {
 #pragma unroll
           for (int e = 0; e < EPL; ++e) x[e] = __bfloat162float(src[e]);
           const float sc = quant_row_q8<EPL>(x, reinterpret_cast<int8_t*>(a.vpool) + (slot * a.nkv + kvh) * HD, lane);
@@ -882,18 +892,25 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
     __syncthreads();
   };
   __syncthreads();                                // the query tile is complete
-  uint32_t qf[HD / 16][4];
+  uint32_t qf[Q8 ? 1 : HD / 16][4];               // Q8: the registers hold the next tile instead
+  auto load_q = [&](int kk) {
+    uint32_t* q = qf[Q8 ? 0 : kk];
+    ldsm_x4(q[0], q[1], q[2], q[3], Qs + (lane & 15) * LD + kk * 16 + (lane >> 4) * 8);
+  };
 #pragma unroll
-  for (int kk = 0; kk < HD / 16; ++kk)
-    ldsm_x4(qf[kk][0], qf[kk][1], qf[kk][2], qf[kk][3], Qs + (lane & 15) * LD + kk * 16 + (lane >> 4) * 8);
+  for (int kk = 0; !Q8 && kk < HD / 16; ++kk) load_q(kk);
   bool ok = true;
+  if (Q8) {
+    convert_half(0);
+    load_half(1);
+  }
   for (int i = 0; i < cnt; ++i) {
     const int kt = t0 + i * step;
     bf16* Ks = ring + (2 * i % 3) * TILE;
     bf16* Vs = ring + ((2 * i + 1) % 3) * TILE;
     if (!(ok = arrived(2 * i))) break;
     __syncthreads();                              // K is here; the V tile before it is consumed
-    load_half(2 * i + 2);
+    if (!Q8) load_half(2 * i + 2);
     if (kt == ntiles - 1) patch(Ks, kcur);
     // ---- S = Q K^T for this warp's 16 keys; SHARED: two chains -----------------------------------
     float sc[2][4], s2[2][4];
@@ -902,9 +919,10 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 #pragma unroll
     for (int kk = 0; kk < HD / 16; ++kk) {
       uint32_t b0, b1, b2, b3;
+      if (Q8) load_q(kk);
       ldsm_x4(b0, b1, b2, b3, Ks + piece(warp * 16 + (lane & 7) + ((lane >> 4) << 3), kk * 2 + ((lane >> 3) & 1)));
-      mma_bf16(SHARED && (kk & 1) ? s2[0] : sc[0], qf[kk], b0, b1);
-      mma_bf16(SHARED && (kk & 1) ? s2[1] : sc[1], qf[kk], b2, b3);
+      mma_bf16(SHARED && (kk & 1) ? s2[0] : sc[0], qf[Q8 ? 0 : kk], b0, b1);
+      mma_bf16(SHARED && (kk & 1) ? s2[1] : sc[1], qf[Q8 ? 0 : kk], b2, b3);
     }
 #pragma unroll
     for (int n = 0; SHARED && n < 2; ++n) { sc[n][0] += s2[n][0]; sc[n][1] += s2[n][1]; }
@@ -935,8 +953,12 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
 #pragma unroll
     for (int n = 0; n < HD / 8; ++n) { o[n][0] *= corr; o[n][1] *= corr; }
     if (!(ok = arrived(2 * i + 1))) break;
+    if (Q8) {                                     // into the stage of the K tile before this one, consumed when this one was published
+      convert_half(2 * i + 1);
+      load_half(2 * i + 2);
+    }
     __syncthreads();                              // V is here, K is consumed
-    load_half(2 * i + 3);
+    if (!Q8) load_half(2 * i + 3);
     if (kt == ntiles - 1) patch(Vs, vcur);
     // ---- O += P V for the same 16 keys -------------------------------------------------------------
 #pragma unroll
@@ -948,6 +970,10 @@ attn_decode_batch_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_c
       mma_bf16(c1, pf, b2, b3);
       o[2 * np][0] = c0[0]; o[2 * np][1] = c0[1];
       o[2 * np + 1][0] = c1[0]; o[2 * np + 1][1] = c1[1];
+    }
+    if (Q8) {
+      convert_half(2 * i + 2);
+      load_half(2 * i + 3);
     }
   }
   // ---- merge the four warps, normalise, gate, store -----------------------------------------------------
@@ -1162,7 +1188,8 @@ CB_EXPORT int cb_attn_decode(const void* proj, int64_t ldp, const void* qg, cons
       if (rc) return rc;
     }
     const bool shared = M <= kSharedRows && nsplit > 1 && 2 * nkv * M <= kSharedCtas;
-    auto kern = shared ? attn_decode_batch_kernel<HD, true> : attn_decode_batch_kernel<HD, false>;
+    auto kern = kscale ? (shared ? attn_decode_batch_kernel<HD, true, true> : attn_decode_batch_kernel<HD, false, true>)
+                       : (shared ? attn_decode_batch_kernel<HD, true, false> : attn_decode_batch_kernel<HD, false, false>);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     return (int)cb_launch(kern, shared ? dim3(kSharedCtas) : dim3((unsigned)nkv, (unsigned)M, (unsigned)nsplit), dim3(128), smem,

@@ -1250,3 +1250,47 @@ def test_decode_attention_of_wide_batches_takes_a_row_by_itself(M, nkv):
                       out, nh=nh, nkv=nkv, hd=hd, rot=rot, nsplit=ns, eps=1e-6)
         outs.append(out[:M // 2])
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("M,nkv,nsplit", [(8, 4, 64), (9, 4, 1), (16, 2, 4), (70, 1, 9)])
+def test_decode_attention_of_int8_pages(M, nkv, nsplit):
+    """The batch kernel on int8 pages (rows of one token, of a tile and one more, several tiles a split and none, padded rows) against the
+    kernel that takes a row at a time: the pages and scales it writes are the same bytes; scores and sums in fp32, keys and values
+    rounded to bf16 (2^-9) in both, P in one of them.  A second run gives the same bits."""
+    k = K()
+    rep, hd, rot = 4, 256, 64
+    nh = nkv * rep
+    g = torch.Generator().manual_seed(M)
+    pos = torch.randint(0, 900, (M,), generator=g, dtype=torch.int32)
+    pos[0], pos[1], pos[2], pos[3], pos[M // 2], pos[M - 1] = 0, 3001, 64, 127, -1, 63
+    pages = [(int(p) + 64) // 64 for p in pos.clamp(min=0)]
+    order, bt, at = torch.randperm(sum(pages), generator=g), torch.zeros(M, max(pages), dtype=torch.int32), 0
+    for m, p in enumerate(pages):
+        bt[m, :p] = order[at:at + p]
+        at += p
+    rows = sum(pages) * 64
+    q8 = [torch.randint(-127, 128, (rows, nkv, hd), generator=g, dtype=torch.int8).to(DEV) for _ in range(2)]
+    sc = [(torch.rand(rows, nkv, generator=g) * 0.02 + 0.005).to(DEV) for _ in range(2)]
+    proj = torch.randn(M, nh * 2 * hd + 2 * nkv * hd, generator=g).bfloat16().to(DEV)
+    gain = torch.ones(hd, device=DEV)
+    cos, sin = (t.to(DEV) for t in O.rope_tables(rot, 1e6, 3100))
+    pos, bt = pos.to(DEV), bt.to(DEV)
+
+    def run(ctas, ns):
+        pools, scales, out = [t.clone() for t in q8], [t.clone() for t in sc], torch.zeros(M, nh * hd, dtype=torch.bfloat16, device=DEV)
+        part_o, part_ml = torch.empty(M, nh, ns, hd, device=DEV), torch.empty(M, nh, ns, 2, device=DEV)
+        tickets = torch.zeros(M, nkv, dtype=torch.int32, device=DEV)
+        k._lib.call_nostream("set_attn_batch_ctas", ctas)
+        try:
+            for _ in range(2):
+                before = out.clone()
+                k.attn_decode(proj, gain, gain, cos, sin, pos, pos.clamp(min=0), bt, *pools, part_o, part_ml, tickets, out, nh=nh, nkv=nkv,
+                              hd=hd, rot=rot, nsplit=ns, eps=1e-6, kscale=scales[0], vscale=scales[1])
+        finally:
+            k._lib.call_nostream("set_attn_batch_ctas", 32)
+        assert not bool(tickets.any()) and torch.equal(before, out)
+        return out, pools, scales
+
+    (want, wp, ws), (got, gp, gs) = run(0, 8), run(1, nsplit)
+    assert all(torch.equal(x, y) for x, y in zip(wp + ws, gp + gs))
+    close(got, want, 1e-2)
