@@ -358,6 +358,39 @@ def test_wide_decode_bucket_matches_single_rows(name):
 
 
 @torch.no_grad()
+@pytest.mark.parametrize("name", ["tiny", "tiny-moe"])
+def test_partly_filled_wide_buckets_of_int4_weights(name, monkeypatch):
+    """Nine sequences in the 16-row bucket give the logits that they give with three more beside them, bit for bit: in eager and captured
+    steps, with the bf16 expansions of the projections kept and made anew for every product.  Alone (int4 codes, int8 activations;
+    router near-ties may flip) they agree to the quantisation."""
+    from coffin_b200.models.qwen35 import moe
+    from coffin_b200.models.qwen35.model import Qwen35Model
+    cfg = preset(name)
+    sd = random_state_dict(cfg, 0)
+    seqs = [_tokens(cfg, 30 + 7 * r, seed=80 + r) for r in range(12)]
+    tables = [list(range(1 + 4 * r, 5 + 4 * r)) for r in range(12)]
+    toks, pos = [int(s[-1]) for s in seqs], [len(s) - 1 for s in seqs]
+    seen = []
+    for budget in (moe.PREFILL_CACHE_BYTES, 0):
+        monkeypatch.setattr(moe, "PREFILL_CACHE_BYTES", budget)
+        model = Qwen35Model(cfg, sd, max_seq=256, num_slots=12, quant="w4a8")
+        for r, s in enumerate(seqs):
+            model.zero_state(r)
+            model.prefill(s[:-1].cuda(), 0, r, torch.tensor(tables[r], dtype=torch.int32, device="cuda"), want_logits=False)
+        snaps = [model.snapshot_state(r) for r in range(12)]
+        for n, graph in ((9, False), (12, False), (9, True), (12, True), (9, True)):
+            model.set_rows(16, toks[:n], pos[:n], list(range(n)), tables[:n])
+            seen.append(model.decode(16, graph=graph)[1][:9].clone())
+            for r in range(n):
+                model.restore_state(r, snaps[r])
+        for r in (0, 8):
+            model.set_rows(1, [toks[r]], [pos[r]], [r], [tables[r]])
+            assert _rel(model.decode(1, graph=False)[1][0], seen[-1][r].cpu()) < (8e-2 if name == "tiny" else 0.25)
+            model.restore_state(r, snaps[r])
+    assert all(torch.equal(x, seen[0]) for x in seen[1:])
+
+
+@torch.no_grad()
 def test_grouped_prefill_equals_separate_prefills():
     """Three chunks (one of them a continuation at a non-zero position) stacked into one forward give
     the logits, KV and delta-net states of three separate prefills."""
@@ -386,8 +419,8 @@ def test_grouped_prefill_equals_separate_prefills():
 @pytest.mark.parametrize("rows", [1, 3, 12, 40])
 def test_int8_kv_pool_matches_the_int8_kv_oracle(rows):
     """``kv_dtype="int8"``: K/V rows are quantised per (token, kv head) when appended (prefill prep, decode
-    append) and dequantised on load by every attention kernel - prefill flash, single-row decode, the
-    tensor-core batch kernel (40 rows x 2 kv heads) and the wide bucket.  Against the fp32 oracle that
+    append) and dequantised on load by the attention kernels of heads of 64 - prefill flash, decode a row at a
+    time, up to 40 rows x 2 kv heads - and in the wide bucket.  Against the fp32 oracle that
     quantises its KV the same way; and the pool really is int8 with one scale per (token, head)."""
     from coffin_b200.models.qwen35.model import Qwen35Model
     cfg = preset("tiny")
