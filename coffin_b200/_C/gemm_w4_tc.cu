@@ -197,7 +197,7 @@ gemm_w4_grouped_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
     }
   } else if (warp >= 6 && warp < 6 + NDQ) {
     // ------------------------------- dequant ----------------------------------------------------------
-    // Two groups of four warps take alternate k-blocks, so a group has two k-block times for one tile and
+    // Two groups of eight warps take alternate k-blocks, so a group has two k-block times for one tile and
     // the expansion of k-block n+1 overlaps that of n.  Thread tg of a group owns weight row tg.
     const int grp = (warp - 6) / (NDQ / 2), tg = threadIdx.x - 6 * 32 - grp * (NDQ * 16);
     uint32_t it = 0;

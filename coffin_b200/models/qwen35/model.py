@@ -396,8 +396,8 @@ class Qwen35Model:
         """Row-parallel projection + all-reduce.  With a peer-memory region the all-reduce is a
         reduce-scatter + all-gather over NVLink: for a prefill chunk the tcgen05 GEMM epilogue leaves its
         partial rows in this rank's peer-visible buffer and publishes a sequence number; for the few
-        rows of a decode bucket the K-split GEMM (one wave of CTAs, which a 128-row tile per CTA would
-        not fill) writes the partial rows and a small kernel copies them there.  A reduce/gather kernel
+        rows of a decode bucket the product of few rows (K split over a cluster where the tiles do not fill the
+        machine) writes the partial rows and a small kernel copies them there.  A reduce/gather kernel
         on every rank then pulls the rows it owns from all ranks, adds them and stores the sums to every rank.  Without the region the partial result is all-reduced by NCCL."""
         if self.tp is not None and self.tp.pf_rows:
             if A.shape[0] <= K.ROWS:
@@ -861,7 +861,7 @@ class Qwen35Model:
                               nh=c.num_attention_heads, nkv=c.num_key_value_heads, hd=c.head_dim,
                               rot=c.rotary_dim, nsplit=b["nsplit"], eps=self.eps, **self._kvs(j))
             if tpw and self.tp.pf_rows:
-                # K-split GEMM, then the one-shot all-reduce whose second kernel also adds the residual and
+                # the product, then the one-shot all-reduce whose second kernel also adds the residual and
                 # applies the post-attention norm
                 self._gemm(act, lw.w_out, out=b["part"])
                 gq = aq if (lw.moe is None and isinstance(lw.w_gu, QW)) else None

@@ -132,7 +132,7 @@ def test_gemv_fused_norm_swiglu(M, H, I):
                                        # CTA pairs (256-row tiles, 256 / 320 columns), edge tiles in both directions
                                        (300, 520, 1032, 1256), (300, 520, 1032, 1320), (257, 264, 72, 1320), (300, 520, 1032, 1288), (2048, 2560, 512, 1288),
                                        (1000, 1536, 512, 1256), (2048, 2560, 4096, 1320), (2100, 1288, 2560, 1256),
-                                       # at most 128 rows: K split over CTAs, partial tiles reduced by the last slice
+                                       # at most 128 rows: weights as the M operand, K in slices over a cluster
                                        (64, 2560, 4096, 0), (16, 12352, 2560, 0), (128, 520, 9216, 0), (5, 264, 520, 0)])
 def test_gemm_tcgen05(M, N, Kd, bn):
     k = K()
@@ -732,8 +732,8 @@ def _intact(buf, rows, cols):
 
 @pytest.mark.parametrize("M,N,Kd", [(1, 2560, 9216), (8, 2560, 4096), (4, 1000, 520), (40, 2560, 4096), (64, 520, 1024)])
 def test_projections_stay_in_bounds_and_repeat_bit_exact(M, N, Kd):
-    """Kernels that split K over CTAs and finish through arrival tickets (the tensor-core GEMV for
-    narrow outputs, the split-K tcgen05 GEMM for decode buckets): outputs written into a canary-padded
+    """Kernels that split K over CTAs (the tensor-core GEMV for narrow outputs, which finishes through arrival
+    tickets; the tcgen05 product of few rows, which adds its slices over a cluster): outputs written into a canary-padded
     buffer leave the canaries alone, and a second run of the same launch gives the same bits (partial
     sums are added in slice order, never in arrival order)."""
     k = K()
