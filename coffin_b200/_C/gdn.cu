@@ -851,8 +851,8 @@ __device__ __forceinline__ void chunk_decay(float g0, float g1, float be0, float
 // the triangular system itself is still solved from TF32 products in fp32.
 // Bound by latencies, not by memory (two CTAs of 16 dependent phases an SM): at 2048 tokens, 16 key and 32 value heads 141 us with
 // the value rows fetched where they are used, the inverse column by column through shared memory and one value head a CTA; 95 us
-// with the rows requested ahead, the diagonal blocks inverted in registers and ldmatrix fragments; 87 us with the value heads of a
-// key head in one CTA.
+// with the rows requested ahead, the diagonal blocks inverted in registers and ldmatrix fragments; 91 us with the value heads of a
+// key head in one CTA and the factors beta and e^c taken as the last products load their fragments.
 template <int DK, int DV, bool BF = false, bool FUSE = false>
 __global__ void __launch_bounds__(256, 2) gdn_chunk_prepare_tc_kernel(const GdnChunkArgs a) {
   using Lay = PrepTcLayout<DK, DV>;
