@@ -740,7 +740,7 @@ class Qwen35Model:
                 K.gdn_decode(proj, lw.conv_w, lw.A_log, lw.dt_bias, lw.norm_w, self.ring[j], self.state[j],
                              b["slots"], b["positions"], act, nk=c.linear_num_key_heads,
                              nv=c.linear_num_value_heads, dk=c.linear_key_head_dim, dv=c.linear_value_head_dim,
-                             eps=self.eps, settled=K.capturing())
+                             eps=self.eps, settled=self._own_graph)
             else:
                 j = self.full_ids[li]
                 act = b["act_full"]
@@ -852,7 +852,7 @@ class Qwen35Model:
                 K.gdn_decode(proj, lw.conv_w, lw.A_log, lw.dt_bias, lw.norm_w, self.ring[j], self.state[j],
                              b["slots"], b["positions"], act, nk=c.linear_num_key_heads,
                              nv=c.linear_num_value_heads, dk=c.linear_key_head_dim, dv=c.linear_value_head_dim,
-                             eps=self.eps, settled=K.capturing())
+                             eps=self.eps, settled=self._own_graph)
             else:
                 j = self.full_ids[li]
                 act = b["act_full"]
@@ -970,6 +970,7 @@ class Qwen35Model:
             raise ValueError(f"state slot {slot} outside 0..{self.num_slots - 1}")
 
     _advance = False
+    _own_graph = False        # the step goes into a graph by itself: a replay starts when everything enqueued before it has completed
 
     def _gkey(self, M: int, advance: bool):
         return (M, self.lane, bool(advance), bool(self.full_logits) if self.tp_world > 1 else True, bool(self.use_mega))
@@ -997,8 +998,12 @@ class Qwen35Model:
         if self.graph_pool is None:
             self.graph_pool = torch.cuda.graph_pool_handle()
         l0 = K.LAUNCHES
-        with K.capture_graph(g, pool=self.graph_pool):
-            self._decode_body(M)
+        self._own_graph = True
+        try:
+            with K.capture_graph(g, pool=self.graph_pool):
+                self._decode_body(M)
+        finally:
+            self._own_graph = False
         self._step_launches[M] = K.LAUNCHES - l0
         self._graphs[gkey] = g
         self._advance = False

@@ -552,6 +552,8 @@ class Qwen4ExpModel:
         return gv + torch.nn.functional.silu(conv)
 
     # ------------------------------------------------------------------ mixers
+    _own_graph = False        # the step goes into a graph by itself: a replay starts when everything enqueued before it has completed
+
     def _gdn(self, L, li: int, ws: dict, T: int, mixed, out, *, slot=None, pos0=None, slots=None, positions=None,
              verify: bool = False):
         """``verify``: the ``T`` rows are consecutive tokens of one sequence scored without touching its
@@ -568,7 +570,7 @@ class Qwen4ExpModel:
                          ws["one_pos"], act, ntok=T, record=ws["record"][j], write_state=False, **kw)
         elif slots is not None:
             K.gdn_decode(proj, L.conv_w, L.A_log, L.dt_bias, L.norm_w, self.ring[j], self.state[j], slots, positions, act,
-                         settled=K.capturing(), **kw)
+                         settled=self._own_graph, **kw)
         else:
             K.gdn_prefill(proj, L.conv_w, L.A_log, L.dt_bias, L.norm_w, self.ring[j, slot], self.state[j, slot],
                           ws["gdn"], act, pos0=pos0, **kw)
@@ -817,8 +819,12 @@ class Qwen4ExpModel:
             g = torch.cuda.CUDAGraph()
             if self.graph_pool is None:
                 self.graph_pool = torch.cuda.graph_pool_handle()
-            with K.capture_graph(g, pool=self.graph_pool):
-                self._decode_body(n, M, True, host=False)
+            self._own_graph = True
+            try:
+                with K.capture_graph(g, pool=self.graph_pool):
+                    self._decode_body(n, M, True, host=False)
+            finally:
+                self._own_graph = False
             self._graphs[key] = g
             for s_, sn in zip(st["slots"], snaps):      # the capture itself does not run the kernels; states are as staged
                 self.restore_state(s_, sn)

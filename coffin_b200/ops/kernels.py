@@ -50,11 +50,6 @@ def capture_graph(graph: "torch.cuda.CUDAGraph", pool=None):
             gc.enable()
 
 
-def capturing() -> bool:
-    """Whether the current launches go into a graph: a replay starts when everything enqueued before it has completed."""
-    return torch.cuda.is_current_stream_capturing()
-
-
 def _count(n: int = 1) -> None:
     global LAUNCHES
     LAUNCHES += n
@@ -446,6 +441,7 @@ def w4_dequant(Wq: torch.Tensor, wscale: torch.Tensor, out: torch.Tensor | None 
 def settle() -> None:
     """What was enqueued before is complete when anything enqueued after this starts (launches of this library may overlap)."""
     call("settle")
+    _count()
 
 
 def moe_dispatch(idx: torch.Tensor, n_experts: int, tile: int = 128) -> dict:

@@ -1158,7 +1158,7 @@ def test_moe_gemv_w4a8_by_expert(E, N, Kd, swiglu, slots, monkeypatch):
 @pytest.mark.parametrize("E,T,kind", [(256, 33, "padded"), (256, 64, "wanted"), (600, 64, "padded"), (2, 128, "wanted"), (7, 9, "one")])
 def test_moe_gemv_w4a8_by_expert_of_uneven_routing(E, T, kind, monkeypatch):
     """Passes of eight slots of one expert in CTAs of their own: the rows behind the last sequence all alike, experts that every row wants
-    (9, 64 and 65 slots), all slots on one expert, one after it; every slot's result that of the slot-wise kernel."""
+    (9, 64 and 65 slots), all slots on one expert, one after it; every slot's result that of the slot-wise kernel, twice the same bits."""
     k = K()
     from coffin_b200.weights.quant import W4A8Weight
     g = torch.Generator().manual_seed(E + T)
@@ -1181,6 +1181,7 @@ def test_moe_gemv_w4a8_by_expert_of_uneven_routing(E, T, kind, monkeypatch):
     monkeypatch.setattr(k, "W4_GROUP_SHARE", 0)
     k.moe_gemv_w4(wq, sc, x, got, slots, rows)
     close(got, want, 2 ** -7)
+    assert torch.equal(k.moe_gemv_w4(wq, sc, x, torch.full_like(got, 3.0), slots, rows), got)
 
 
 @pytest.mark.parametrize("M,nkv,nsplit", [(8, 4, 64), (9, 4, 1), (16, 2, 2), (70, 1, 9)])
@@ -1227,7 +1228,7 @@ def test_decode_attention_of_rows_of_any_length(M, nkv, nsplit):
 @pytest.mark.parametrize("M,nkv", [(16, 4), (33, 2), (64, 4), (130, 1)])
 def test_decode_attention_of_wide_batches_takes_a_row_by_itself(M, nkv):
     """From nine rows on a row's output is the same bits whatever the lengths of the others, with one split a row and several, splits
-    without a tile, and the row's token in the last one."""
+    without a tile, and the row's token in the last one; a second run repeats them."""
     k = K()
     rep, hd, rot = 4, 256, 64
     nh, ns = nkv * rep, k.decode_splits(nkv, M)
@@ -1246,8 +1247,12 @@ def test_decode_attention_of_wide_batches_takes_a_row_by_itself(M, nkv):
     for pos in (one, two):
         pos, pools, out = pos.to(DEV), (kp.clone(), vp.clone()), torch.zeros(M, nh * hd, dtype=torch.bfloat16, device=DEV)
         part_o, part_ml = torch.empty(M, nh, ns, hd, device=DEV), torch.empty(M, nh, ns, 2, device=DEV)
-        k.attn_decode(proj, gain, gain, cos, sin, pos, pos, bt, *pools, part_o, part_ml, torch.zeros(M, nkv, dtype=torch.int32, device=DEV),
-                      out, nh=nh, nkv=nkv, hd=hd, rot=rot, nsplit=ns, eps=1e-6)
+        tickets = torch.zeros(M, nkv, dtype=torch.int32, device=DEV)
+        for _ in range(2):
+            before = out.clone()
+            k.attn_decode(proj, gain, gain, cos, sin, pos, pos, bt, *pools, part_o, part_ml, tickets, out, nh=nh, nkv=nkv, hd=hd, rot=rot,
+                          nsplit=ns, eps=1e-6)
+        assert torch.equal(out, before)
         outs.append(out[:M // 2])
     assert torch.equal(*outs)
 

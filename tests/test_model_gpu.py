@@ -391,6 +391,43 @@ def test_partly_filled_wide_buckets_of_int4_weights(name, monkeypatch):
 
 
 @torch.no_grad()
+def test_steps_captured_together_by_a_caller():
+    """Two uncaptured steps that a caller puts into one graph (the second starts from states that the first writes) give what two
+    captured steps give one after the other."""
+    from coffin_b200.models.qwen35.model import Qwen35Model
+    from coffin_b200.ops import kernels as K
+    cfg = preset("tiny")
+    model = Qwen35Model(cfg, random_state_dict(cfg, 0), max_seq=256, num_slots=2)
+    seqs = [_tokens(cfg, 40 + r, seed=60 + r) for r in range(2)]
+    tables = [[1, 2], [3, 4]]
+    for r, s in enumerate(seqs):
+        model.zero_state(r)
+        model.prefill(s[:-1].cuda(), 0, r, torch.tensor(tables[r], dtype=torch.int32, device="cuda"), want_logits=False)
+    snaps = [model.snapshot_state(r) for r in range(2)]
+
+    def stage():
+        for r in range(2):
+            model.restore_state(r, snaps[r])
+        model.set_rows(2, [int(s[-1]) for s in seqs], [len(s) - 1 for s in seqs], [0, 1], tables)
+
+    stage()
+    for _ in range(2):
+        want = model.decode(2, advance=True)[1].clone()
+    stage()
+    for _ in range(2):
+        model.decode(2, graph=False, advance=True)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with K.capture_graph(g, pool=model.graph_pool):
+        for _ in range(2):
+            got = model.decode(2, graph=False, advance=True)[1]
+    for _ in range(3):
+        stage()
+        g.replay()
+        assert torch.equal(got, want)
+
+
+@torch.no_grad()
 def test_grouped_prefill_equals_separate_prefills():
     """Three chunks (one of them a continuation at a non-zero position) stacked into one forward give
     the logits, KV and delta-net states of three separate prefills."""
