@@ -841,7 +841,7 @@ def attn_decode(proj, qg, kg, cos, sin, positions, rope_pos, block_table, kpool,
     """``tickets``: zero-initialised int32 ``[M, nkv]`` arrival counters (re-armed by the kernel)."""
     M = positions.numel()
     call("attn_decode", proj, proj.stride(0), qg, kg, cos, sin, positions, rope_pos, block_table,
-         block_table.stride(0), kpool, vpool, kpool.shape[0], part_o, part_ml, tickets, out, out.stride(0), M, nh, nkv, hd, rot,
+         block_table.stride(0), kpool, vpool, kpool.numel() // (nkv * hd), part_o, part_ml, tickets, out, out.stride(0), M, nh, nkv, hd, rot,
          nsplit, float(eps), kscale, vscale, status_word(proj.device))
     _count()
     return out

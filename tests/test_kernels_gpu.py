@@ -1248,8 +1248,10 @@ def test_decode_attention_of_wide_batches_takes_a_row_by_itself(M, nkv):
         pos, pools, out = pos.to(DEV), (kp.clone(), vp.clone()), torch.zeros(M, nh * hd, dtype=torch.bfloat16, device=DEV)
         part_o, part_ml = torch.empty(M, nh, ns, hd, device=DEV), torch.empty(M, nh, ns, 2, device=DEV)
         tickets = torch.zeros(M, nkv, dtype=torch.int32, device=DEV)
-        for _ in range(2):
+        for turn in range(2):
             before = out.clone()
+            if turn:                                 # pools may come as blocks of rows
+                pools = [t.view(-1, 64, nkv, hd) for t in pools]
             k.attn_decode(proj, gain, gain, cos, sin, pos, pos, bt, *pools, part_o, part_ml, tickets, out, nh=nh, nkv=nkv, hd=hd, rot=rot,
                           nsplit=ns, eps=1e-6)
         assert torch.equal(out, before)
