@@ -1041,7 +1041,6 @@ def test_gdn_decode_of_many_rows(nk, nv, M):
     """More (row, head) pairs than two CTAs an SM hold: the streaming kernel against the per-pair one on eight rows at a time.  The
     norm's sum is taken in another order (fp32, one bf16 rounding) and the compiler contracts other multiplies and adds: a few fp32
     roundings (2^-24 each) of sums of 128 terms, 1e-5 of the scale.  Padded rows stay untouched."""
-
     k = K()
     dk, n = 128, M + 2
     proj, conv_w, A_log, dt_bias, norm_w, conv_dim = _gdn_inputs(M, nk, nv, dk, dk, 91)
